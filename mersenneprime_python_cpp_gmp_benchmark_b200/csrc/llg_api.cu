@@ -28,7 +28,7 @@
 
 namespace {
 
-// padded layout of the NTT quarter tables (same as gl::qpad8 in llg_ntt.cuh)
+// padded layout of the NTT twiddle tables (same as gl::qpad8 in llg_ntt.cuh)
 constexpr uint32_t gl_qpad8(uint32_t r) { return r + (r >> 4); }
 constexpr uint32_t gl_qpad8_len(uint32_t qm) { return qm + (qm >> 4) + 1; }
 
@@ -68,7 +68,7 @@ constexpr int kSmallLogMax = 13;  // N = 8192
 struct DeviceTables {
     std::map<uint32_t, double2*> qtw;      // quarter-wave twiddles of the M-point FFT, by M
     std::map<uint32_t, double2*> qtw_s;    // the same in the spread layout (qpad_s), by M
-    uint64_t* nqtw[kSmallLogMax + 1] = {}; // NTT: padded quarter table of the N-point transform
+    uint64_t* nqtw[kSmallLogMax + 1] = {}; // NTT: padded twiddle table of the N-point transform
     NttConst nk[kSmallLogMax + 1] = {};
 };
 
@@ -99,9 +99,10 @@ bool ntt_constants(int log_n, uint64_t& omega, NttConst& K) {
         pw = hmul(pw, r192);
     }
     if (s == 192) return false;
-    K.root2 = hpow(om, s);
-    K.inv_root2 = hinv(K.root2);
-    K.invN = hinv(N % kGQ);
+    const uint64_t root2 = hpow(om, s), R = 0xFFFFFFFFull;  // R = 2^64 mod q (Montgomery form)
+    K.root2 = hmul(root2, R);
+    K.inv_root2 = hmul(hinv(root2), R);
+    K.invN = hmul(hinv(N % kGQ), hmul(R, R));
     return true;
 }
 std::map<int, DeviceTables> g_tables;  // per device ordinal
@@ -143,9 +144,9 @@ int get_ntt(int dev, int log_n, const uint64_t** qtw, NttConst* K) {
         uint64_t omega;
         NttConst k;
         if (!ntt_constants(log_n, omega, k)) return fail(LLG_E_UNSUPPORTED, "no N-th root of 2 for N=2^%d", log_n);
-        const uint32_t QL = (1u << log_n) / 2;  // half table
+        const uint32_t QL = 1u << log_n;
         std::vector<uint64_t> h(gl_qpad8_len(QL), 0ull);
-        uint64_t w = 1;
+        uint64_t w = 0xFFFFFFFFull;  // 1 in Montgomery form
         for (uint32_t r = 0; r < QL; ++r) {
             h[gl_qpad8(r)] = w;
             w = hmul(w, omega);

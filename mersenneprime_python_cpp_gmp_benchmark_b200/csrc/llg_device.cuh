@@ -246,12 +246,4 @@ __device__ __forceinline__ double dsplit_e(double v, int e, double& c) {
 // An integer-valued double with |x| < 2^31 as int32 (the low word of x + 1.5 * 2^52).
 __device__ __forceinline__ int d2i_exact(double x) { return __double2loint(__dadd_rn(x, 6755399441055744.0)); }
 
-// One balanced-digit step: v = x + carry_in; returns the digit in [-2^(b-1), 2^(b-1)) and sets
-// carry = floor((v + 2^(b-1)) / 2^b)  (lucaslehmer.cpp:299-303).
-__device__ __forceinline__ long long balance(long long v, int b, long long& carry) {
-    const long long c = (v + (1LL << (b - 1))) >> b;
-    carry = c;
-    return v - (c << b);
-}
-
 }  // namespace llg

@@ -63,13 +63,15 @@ cudaError_t launch_small_fp64_mixed(uint32_t n, const SmallJob* jobs, int njobs,
 // p < 256: exact multi-limb word arithmetic, one thread per exponent (4 limbs out per exponent).
 cudaError_t launch_word(const SmallJob* jobs, int njobs, uint64_t* res, cudaStream_t st);
 
-// Goldilocks constants of one NTT length N: an N-th root of 2, its inverse, N^-1 (mod q).
+// Goldilocks constants of one NTT length N (mod q): an N-th root of 2 and its inverse in Montgomery
+// form (x 2^64), and 2^128 / N (1 / N in Montgomery form, times the 2^64 that the pointwise
+// Montgomery square takes out).
 struct NttConst {
     uint64_t root2, inv_root2, invN;
 };
 
-// Exact NTT whole-test kernel, N = 2^log_n with 5 <= log_n <= 13 (qtw: padded half table of the
-// N-point transform, gl::qpad8 layout).
+// Exact NTT whole-test kernel, N = 2^log_n with 6 <= log_n <= 13 (qtw: padded twiddle table of the
+// N-point transform, gl::qpad8 layout, Montgomery form).
 cudaError_t launch_small_ntt(int log_n, const SmallJob* jobs, int njobs, const uint64_t* qtw, NttConst K,
                              int64_t* digits, SmallResult* results, cudaStream_t st);
 
@@ -121,7 +123,6 @@ struct LargeCtl {
     unsigned int timeout;            // set when a bounded wait gave up (the result is then invalid)
     unsigned long long err_max;      // bits of the max round-off over the run (double, >= 0)
     unsigned long long err_since;    // same, since the host last cleared it
-    unsigned int halo_read;          // NTT: epoch + 1 once block 0 has read the wrap-around rows
 };
 
 enum { LARGE_INIT = 0, LARGE_ITER = 1, LARGE_FINAL = 2 };
@@ -187,8 +188,9 @@ cudaError_t launch_large_col(int log_r, const LargeArgs& a, cudaStream_t st);
 
 struct NttLargeArgs {
     uint64_t* V;              // state: element (row a, column slot pos) at pos * R + a
-    const uint64_t* qtwC;     // padded half table of the C-point row NTT (gl::qpad8)
-    const uint64_t* qtwR;     // padded half table of the R-point column NTT
+    // every constant in Montgomery form (llg_ntt.cuh)
+    const uint64_t* qtwC;     // padded twiddle table of the C-point row NTT (gl::qpad8)
+    const uint64_t* qtwR;     // padded twiddle table of the R-point column NTT
     const uint64_t* tw1;      // w_N^x, x < 2^tw_shift
     const uint64_t* tw2;      // w_N^(y 2^tw_shift)
     const int* pos_of_c;      // column slot of row-NTT frequency c
@@ -196,14 +198,14 @@ struct NttLargeArgs {
     const uint64_t* iwA;      // [R] w^-sA(a)
     const int* sA;            // [R] (-a p) mod N
     const uint64_t* wB;       // [C] w^sB(b)
-    const uint64_t* iwB;      // [C] w^-sB(b) / N
+    const uint64_t* iwB;      // [C] w^-sB(b) / N, times the square's 2^64
     const int* sB;            // [C] (-R b p) mod N
-    long long* c1;            // [nblocks][C] hop-1 carry-outs of each block's last row
-    int* c2;                  // [nblocks][C] hop-2 carry-outs
-    int* c3;                  // [nblocks][C] hop-3 carry-outs
-    long long* halo;          // block 0's wrap-around carries: C int64 + 2 * C int32
+    long long* c1;            // [nblocks + 1][C] hop-1 carry-outs of a tile's last row: slot 0 the
+                              // wrap-around job's (row R-1, one column on), k + 1 tile k's
+    int* c2;                  // [nblocks + 1][C] hop-2 carry-outs
+    int* c3;                  // [nblocks + 1][C] hop-3 carry-outs
     LargeCtl* ctl;
-    unsigned int* flags;      // [nblocks] epoch + 1 once block k published its carries
+    unsigned int* flags;      // [nblocks + 1] epoch + 1 once the job of that slot published its carries
     int* digits;              // N int32, natural order (INIT input; dump / FINAL output)
     int dump;
     int tw_shift;

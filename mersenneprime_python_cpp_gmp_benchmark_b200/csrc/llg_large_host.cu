@@ -426,24 +426,14 @@ uint64_t qpow(uint64_t a, uint64_t e) {
     return r;
 }
 
-int ntt_pos_of_freq(int log_l, int k) {  // SmallGeom<log_l> (16 values per thread) digit reversal
-    const int L = 1 << log_l, P = (log_l + 3) / 4;
-    const int RLAST = (log_l % 4 == 0) ? 16 : (1 << (log_l % 4));
-    const int klast = k / (L / RLAST);
-    int low = k % (L / RLAST), rest = 0;
-    for (int q = 0; q < P - 1; ++q) {
-        rest = (rest << 4) | (low & 15);
-        low >>= 4;
-    }
-    return rest * RLAST + klast;
-}
+uint64_t to_mont(uint64_t x) { return qmul(x, 0xFFFFFFFFull); }  // x 2^64 mod q
 
-std::vector<uint64_t> ntt_half(int log_l) {  // w_L^r at gl::qpad8(r), r < L/2
-    const uint32_t L = 1u << log_l, QL = L / 2;
-    std::vector<uint64_t> t(QL + (QL >> 4) + 1, 0ull);
+std::vector<uint64_t> ntt_table(int log_l) {  // w_L^r at gl::qpad8(r), r < L, Montgomery form
+    const uint32_t L = 1u << log_l;
+    std::vector<uint64_t> t(L + (L >> 4) + 1, 0ull);
     const uint64_t w = qpow(7, (kQ - 1) / L);
-    uint64_t x = 1;
-    for (uint32_t r = 0; r < QL; ++r) {
+    uint64_t x = to_mont(1);
+    for (uint32_t r = 0; r < L; ++r) {
         t[r + (r >> 4)] = x;
         x = qmul(x, w);
     }
@@ -508,35 +498,35 @@ cudaError_t NttLargeTest::init(uint64_t p_, int log_n) {
     };
     NttLargeArgs& A = args;
     std::memset(&A, 0, sizeof A);
-    std::vector<uint64_t> qc = ntt_half(logC), qr = ntt_half(logR);
+    std::vector<uint64_t> qc = ntt_table(logC), qr = ntt_table(logR);
     std::vector<uint64_t> t1(1ull << s), t2(N >> s);
     {
-        uint64_t x = 1;
+        uint64_t x = to_mont(1);
         for (size_t i = 0; i < t1.size(); ++i) {
             t1[i] = x;
             x = qmul(x, omega);
         }
         const uint64_t st = qpow(omega, 1ull << s);
-        x = 1;
+        x = to_mont(1);
         for (size_t i = 0; i < t2.size(); ++i) {
             t2[i] = x;
             x = qmul(x, st);
         }
     }
     std::vector<int> pc(C), hsA(R), hsB(C);
-    for (int c = 0; c < C; ++c) pc[c] = ntt_pos_of_freq(logC, c);
+    for (int c = 0; c < C; ++c) pc[c] = host_pos_of_freq(logC, 3, c);  // the kernels' radix-8 passes
     std::vector<uint64_t> hwA(R), hiwA(R), hwB(C), hiwB(C);
     for (int a = 0; a < R; ++a) {
         const uint64_t sj = (N - (uint64_t)(((unsigned __int128)a * p) % N)) % N;
         hsA[a] = (int)sj;
-        hwA[a] = qpow(root2, sj);
-        hiwA[a] = qpow(iroot2, sj);
+        hwA[a] = to_mont(qpow(root2, sj));
+        hiwA[a] = to_mont(qpow(iroot2, sj));
     }
     for (int b = 0; b < C; ++b) {
         const uint64_t sj = (N - (uint64_t)(((unsigned __int128)R * b * p) % N)) % N;
         hsB[b] = (int)sj;
-        hwB[b] = qpow(root2, sj);
-        hiwB[b] = qmul(qpow(iroot2, sj), invN);
+        hwB[b] = to_mont(qpow(root2, sj));
+        hiwB[b] = to_mont(to_mont(qmul(qpow(iroot2, sj), invN)));
     }
     const uint64_t *cqc, *cqr, *ct1, *ct2, *cwA, *ciwA, *cwB, *ciwB;
     const int *cpc, *csA, *csB;
@@ -544,15 +534,15 @@ cudaError_t NttLargeTest::init(uint64_t p_, int log_n) {
         (e = up(pc, &cpc)) || (e = up(hwA, &cwA)) || (e = up(hiwA, &ciwA)) || (e = up(hsA, &csA)) ||
         (e = up(hwB, &cwB)) || (e = up(hiwB, &ciwB)) || (e = up(hsB, &csB)))
         return e;
-    void *dV, *dc1, *dc2, *dc3, *dh, *dctl, *dd, *dfl;
-    if ((e = alloc(N * sizeof(uint64_t), &dV)) || (e = alloc((size_t)nblocks * C * sizeof(long long), &dc1)) ||
-        (e = alloc((size_t)nblocks * C * sizeof(int), &dc2)) || (e = alloc((size_t)nblocks * C * sizeof(int), &dc3)) ||
-        (e = alloc((size_t)C * (sizeof(long long) + 2 * sizeof(int)), &dh)) ||
+    void *dV, *dc1, *dc2, *dc3, *dctl, *dd, *dfl;
+    if ((e = alloc(N * sizeof(uint64_t), &dV)) || (e = alloc((size_t)(nblocks + 1) * C * sizeof(long long), &dc1)) ||
+        (e = alloc((size_t)(nblocks + 1) * C * sizeof(int), &dc2)) ||
+        (e = alloc((size_t)(nblocks + 1) * C * sizeof(int), &dc3)) ||
         (e = alloc(sizeof(LargeCtl), &dctl)) || (e = alloc(N * sizeof(int), &dd)) ||
-        (e = alloc((size_t)nblocks * sizeof(unsigned), &dfl)))
+        (e = alloc((size_t)(nblocks + 1) * sizeof(unsigned), &dfl)))
         return e;
     if ((e = cudaMemset(dctl, 0, sizeof(LargeCtl)))) return e;
-    if ((e = cudaMemset(dfl, 0, (size_t)nblocks * sizeof(unsigned)))) return e;
+    if ((e = cudaMemset(dfl, 0, (size_t)(nblocks + 1) * sizeof(unsigned)))) return e;
     ctl = static_cast<LargeCtl*>(dctl);
     digits = static_cast<int*>(dd);
     A.V = static_cast<uint64_t*>(dV);
@@ -570,7 +560,6 @@ cudaError_t NttLargeTest::init(uint64_t p_, int log_n) {
     A.c1 = static_cast<long long*>(dc1);
     A.c2 = static_cast<int*>(dc2);
     A.c3 = static_cast<int*>(dc3);
-    A.halo = static_cast<long long*>(dh);
     A.ctl = ctl;
     A.flags = static_cast<unsigned*>(dfl);
     A.digits = digits;
@@ -593,7 +582,7 @@ cudaError_t NttLargeTest::start_seed(cudaStream_t st) {
 cudaError_t NttLargeTest::start_device(cudaStream_t st) {
     cudaError_t e;
     if ((e = cudaMemsetAsync(ctl, 0, sizeof(LargeCtl), st))) return e;
-    if ((e = cudaMemsetAsync(args.flags, 0, (size_t)nblocks * sizeof(unsigned), st))) return e;
+    if ((e = cudaMemsetAsync(args.flags, 0, (size_t)(nblocks + 1) * sizeof(unsigned), st))) return e;
     if ((e = launch_ntt_row(logC, LARGE_INIT, args, st))) return e;
     if ((e = launch_ntt_col(logR, args, st))) return e;
     done = 1;
@@ -635,8 +624,7 @@ cudaError_t NttLargeTest::step(uint64_t k, cudaStream_t st) {
 cudaError_t NttLargeTest::final_pass(cudaStream_t st) {
     cudaError_t e;
     if ((e = launch_ntt_row(logC, LARGE_FINAL, args, st))) return e;
-    if ((e = cudaMemsetAsync(&ctl->halo_read, 0, sizeof(unsigned), st))) return e;
-    return cudaMemsetAsync(args.flags, 0, (size_t)nblocks * sizeof(unsigned), st);
+    return cudaMemsetAsync(args.flags, 0, (size_t)(nblocks + 1) * sizeof(unsigned), st);
 }
 
 cudaError_t NttLargeTest::finish(cudaStream_t st, std::vector<int>& out) {

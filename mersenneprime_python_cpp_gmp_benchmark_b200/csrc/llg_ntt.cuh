@@ -2,13 +2,20 @@
 // the number-theoretic transforms (exact IBDWT; the reference's CUDA engine, cuda/ll_ntt.cu:38-61
 // and 100-127, does the same field with radix-2 stages and a 128-bit-free u64 multiply).
 //
-//   * products: the 128-bit product is built from four 32 x 32-bit multiply-adds (mad.lo / mad.hi
-//     with carry chains) and reduced with 2^64 == 2^32 - 1 and 2^96 == -1 (mod q);
-//   * 2 has order 192, so every root of unity of order dividing 64 is a power of two: with the
-//     primitive N-th roots w_N = 7^((q-1)/N) that the reference uses (cuda/ll_ntt.cu:187),
-//     w_16 = 2^156, w_8 = 2^120, w_4 = 2^48, w_2 = 2^96 = -1. The twiddles inside a radix-16
-//     butterfly are therefore shifts and a reduction, not products;
-//   * values are kept canonical in [0, q).
+// The integer ALU bounds these kernels (a 32-bit add, shift or select takes 2 cycles of a warp
+// scheduler's ALU, multiply-adds issue beside them), so every primitive is written for the fewest
+// 32-bit ALU instructions:
+//   * products are Montgomery products a b 2^-64 mod q (mul). With q = 2^64 - 2^32 + 1 the
+//     reduction needs no multiplication: for X = a b = xh 2^64 + r1 2^32 + r0 and
+//     t + e 2^32 = r0 + r1, X 2^-64 == xh + r1 - (t 2^32 + e (2^32 - 1)), one 64-bit difference with
+//     one correction. Every constant (twiddles, weights) is stored as c 2^64 mod q ("Montgomery
+//     form"), so mul(value, constant) is the plain product and the values themselves stay plain.
+//     29 cycles a warp product per scheduler, against 41 with the 128-bit reduction it replaces;
+//   * a sum is a difference with the negative (add), canonical without a compare;
+//   * 2 has order 192, so w_8 = 7^((q-1)/8) = 2^120 and w_4 = 2^48: the twiddles inside a radix-8
+//     butterfly are shifts with their own short reductions (rot24, rot48, rot72). A radix-8
+//     butterfly takes 41 cycles a value, against 63 before.
+// "any" below means any 64-bit value standing for itself mod q; canonical means < q.
 #pragma once
 
 #include <cstdint>
@@ -17,136 +24,108 @@ namespace llg {
 namespace gl {
 
 constexpr uint64_t Q = 0xFFFFFFFF00000001ull;
-constexpr uint64_t EPS = 0xFFFFFFFFull;  // 2^64 mod q
+constexpr uint64_t ONE = 0xFFFFFFFFull;           // 2^64 mod q: 1 in Montgomery form
+constexpr uint64_t HALF = 0x8000000000000000ull;  // 2^63: 1/2 in Montgomery form
 
-// a + b for canonical a, b: the 65-bit sum with its carry c, and s + EPS with its carry; the
-// result is s + EPS when either carried (a carry means a + b - 2^64 + EPS = a + b - q; a carry of
-// s + EPS alone means s >= q), else s. 32-bit add-with-carry chains.
-__device__ __forceinline__ uint64_t add(uint64_t a, uint64_t b) {
-    uint64_t r;
-    asm("{\n\t.reg .u32 a0, a1, b0, b1, s0, s1, t0, t1, c, z;\n\t.reg .pred p;\n\t"
-        "mov.u32 z, 0;\n\t"
-        "mov.b64 {a0, a1}, %1;\n\t"
-        "mov.b64 {b0, b1}, %2;\n\t"
-        "add.cc.u32 s0, a0, b0;\n\t"
-        "addc.cc.u32 s1, a1, b1;\n\t"
-        "addc.u32 c, z, z;\n\t"
-        "add.cc.u32 t0, s0, 0xFFFFFFFF;\n\t"
-        "addc.cc.u32 t1, s1, z;\n\t"
-        "addc.u32 c, c, z;\n\t"
-        "setp.ne.u32 p, c, 0;\n\t"
-        "selp.b32 s0, t0, s0, p;\n\t"
-        "selp.b32 s1, t1, s1, p;\n\t"
-        "mov.b64 %0, {s0, s1};\n\t}"
-        : "=l"(r)
-        : "l"(a), "l"(b));
-    return r;
-}
-
-// a - b for canonical a, b: on a borrow, a - b + 2^64 - EPS = a - b + q
+// a - b for any a and b <= q: on a borrow, a - b + 2^64 - (2^32 - 1) = a - b + q. The result is
+// canonical when a is.
 __device__ __forceinline__ uint64_t sub(uint64_t a, uint64_t b) {
     uint64_t r;
-    asm("{\n\t.reg .u32 a0, a1, b0, b1, d0, d1, br, z;\n\t"
-        "mov.u32 z, 0;\n\t"
+    asm("{\n\t.reg .u32 a0, a1, b0, b1, m;\n\t"
         "mov.b64 {a0, a1}, %1;\n\t"
         "mov.b64 {b0, b1}, %2;\n\t"
-        "sub.cc.u32 d0, a0, b0;\n\t"
-        "subc.cc.u32 d1, a1, b1;\n\t"
-        "subc.u32 br, z, z;\n\t"      // 0, or 0xFFFFFFFF = EPS after a borrow
-        "sub.cc.u32 d0, d0, br;\n\t"
-        "subc.u32 d1, d1, z;\n\t"
-        "mov.b64 %0, {d0, d1};\n\t}"
+        "sub.cc.u32 a0, a0, b0;\n\t"
+        "subc.cc.u32 a1, a1, b1;\n\t"
+        "subc.u32 m, 0, 0;\n\t"  // 0, or 0xFFFFFFFF = 2^64 - q after a borrow
+        "sub.cc.u32 a0, a0, m;\n\t"
+        "subc.u32 a1, a1, 0;\n\t"
+        "mov.b64 %0, {a0, a1};\n\t}"
         : "=l"(r)
         : "l"(a), "l"(b));
     return r;
 }
 
-__device__ __forceinline__ uint64_t neg(uint64_t a) { return a ? Q - a : 0ull; }
+// a + b for any a and canonical b: a - (q - b); canonical when a is.
+__device__ __forceinline__ uint64_t add(uint64_t a, uint64_t b) { return sub(a, Q - b); }
 
-// (hi * 2^64 + lo) mod q with hi = h1 * 2^32 + h0:  lo - h1 + h0 * (2^32 - 1), canonical.
-// t = lo - h1 (minus EPS on a borrow: no second borrow since h1 < 2^32), u = h0 2^32 - h0,
-// r = t + u with the same carry / canonical step as add (r + EPS when t + u or r + EPS carries).
-__device__ __forceinline__ uint64_t reduce128(uint64_t lo, uint64_t hi) {
+// The canonical form of any a.
+__device__ __forceinline__ uint64_t canon(uint64_t a) { return sub(a, Q); }
+
+// Montgomery product a b 2^-64 mod q; canonical when a or b is (then xh <= q - 1, so xh + r1 does
+// not overflow), any otherwise excluded: one operand must be canonical.
+__device__ __forceinline__ uint64_t mul(uint64_t a, uint64_t b) {
+    const uint64_t lo = a * b, hi = __umul64hi(a, b);
     uint64_t r;
-    asm("{\n\t.reg .u32 l0, l1, h0, h1, t0, t1, u0, u1, r0, r1, s0, s1, br, c, z;\n\t.reg .pred p;\n\t"
-        "mov.u32 z, 0;\n\t"
-        "mov.b64 {l0, l1}, %1;\n\t"
-        "mov.b64 {h0, h1}, %2;\n\t"
-        "sub.cc.u32 t0, l0, h1;\n\t"
-        "subc.cc.u32 t1, l1, z;\n\t"
-        "subc.u32 br, z, z;\n\t"
-        "sub.cc.u32 t0, t0, br;\n\t"
-        "subc.u32 t1, t1, z;\n\t"
-        "sub.cc.u32 u0, z, h0;\n\t"
-        "subc.u32 u1, h0, z;\n\t"
-        "add.cc.u32 r0, t0, u0;\n\t"
-        "addc.cc.u32 r1, t1, u1;\n\t"
-        "addc.u32 c, z, z;\n\t"
-        "add.cc.u32 s0, r0, 0xFFFFFFFF;\n\t"
-        "addc.cc.u32 s1, r1, z;\n\t"
-        "addc.u32 c, c, z;\n\t"
-        "setp.ne.u32 p, c, 0;\n\t"
-        "selp.b32 r0, s0, r0, p;\n\t"
-        "selp.b32 r1, s1, r1, p;\n\t"
-        "mov.b64 %0, {r0, r1};\n\t}"
+    asm("{\n\t.reg .u32 r0, r1, r2, r3, t, m, e;\n\t"
+        "mov.b64 {r0, r1}, %1;\n\t"
+        "mov.b64 {r2, r3}, %2;\n\t"
+        "add.cc.u32 t, r1, r0;\n\t"
+        "addc.u32 e, 0, 0;\n\t"
+        "neg.s32 e, e;\n\t"
+        "add.cc.u32 r2, r2, r1;\n\t"
+        "addc.u32 r3, r3, 0;\n\t"
+        "sub.cc.u32 r2, r2, e;\n\t"
+        "subc.cc.u32 r3, r3, t;\n\t"
+        "subc.u32 m, 0, 0;\n\t"
+        "sub.cc.u32 r2, r2, m;\n\t"
+        "subc.u32 r3, r3, 0;\n\t"
+        "mov.b64 %0, {r2, r3};\n\t}"
         : "=l"(r)
         : "l"(lo), "l"(hi));
     return r;
 }
 
-// a * b mod q, the 128-bit product from 32-bit multiply-adds
-__device__ __forceinline__ uint64_t mul(uint64_t a, uint64_t b) {
-    const uint32_t a0 = (uint32_t)a, a1 = (uint32_t)(a >> 32);
-    const uint32_t b0 = (uint32_t)b, b1 = (uint32_t)(b >> 32);
-    uint32_t r0, r1, r2, r3;
-    asm("mul.lo.u32 %0, %4, %6;\n\t"
-        "mul.hi.u32 %1, %4, %6;\n\t"
-        "mad.lo.cc.u32 %1, %4, %7, %1;\n\t"
-        "madc.hi.u32 %2, %4, %7, 0;\n\t"
-        "mad.lo.cc.u32 %1, %5, %6, %1;\n\t"
-        "madc.hi.cc.u32 %2, %5, %6, %2;\n\t"
-        "madc.hi.u32 %3, %5, %7, 0;\n\t"
-        "mad.lo.cc.u32 %2, %5, %7, %2;\n\t"
-        "addc.u32 %3, %3, 0;"
-        : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3)
-        : "r"(a0), "r"(a1), "r"(b0), "r"(b1));
-    const uint64_t lo = ((uint64_t)r1 << 32) | r0;
-    const uint64_t hi = ((uint64_t)r3 << 32) | r2;
-    return reduce128(lo, hi);
+// x 2^24, canonical for any x: x 2^24 = lo + h 2^64 with h < 2^24, and -h 2^64 == q - h (2^32 - 1)
+// = (~h) 2^32 + h + 1 takes two instructions.
+__device__ __forceinline__ uint64_t rot24(uint64_t x) {
+    const uint32_t x0 = (uint32_t)x, x1 = (uint32_t)(x >> 32), h = x1 >> 8;
+    const uint64_t lo = ((uint64_t)__funnelshift_l(x0, x1, 24) << 32) | (x0 << 24);
+    return sub(lo, ((uint64_t)(~h) << 32) | (h + 1u));
 }
 
-// x * 2^S mod q for a compile-time shift S (any integer; 2^192 == 1, 2^96 == -1)
-template <int S>
-__device__ __forceinline__ uint64_t mul2k(uint64_t x) {
-    constexpr int s = ((S % 192) + 192) % 192;
-    if constexpr (s == 0) {
-        return x;
-    } else if constexpr (s >= 96) {
-        return neg(mul2k<s - 96>(x));
-    } else if constexpr (s >= 64) {
-        return mul2k<s - 32>(mul2k<32>(x));
-    } else {
-        return reduce128(x << s, x >> (64 - s));
-    }
+// x 2^48, canonical for any x: 2^48 == -2^16 2^-64, the negated Montgomery reduction of x 2^16.
+__device__ __forceinline__ uint64_t rot48(uint64_t x) {
+    const uint32_t x0 = (uint32_t)x, x1 = (uint32_t)(x >> 32);
+    uint64_t r;
+    asm("{\n\t.reg .u32 t, e, m, y0, y1;\n\t"
+        "add.cc.u32 t, %2, %1;\n\t"
+        "addc.u32 e, 0, 0;\n\t"
+        "neg.s32 e, e;\n\t"
+        "add.cc.u32 y0, %3, %2;\n\t"
+        "addc.u32 y1, 0, 0;\n\t"
+        "sub.cc.u32 e, e, y0;\n\t"
+        "subc.cc.u32 t, t, y1;\n\t"
+        "subc.u32 m, 0, 0;\n\t"
+        "sub.cc.u32 e, e, m;\n\t"
+        "subc.u32 t, t, 0;\n\t"
+        "mov.b64 %0, {e, t};\n\t}"
+        : "=l"(r)
+        : "r"(x0 << 16), "r"(__funnelshift_l(x0, x1, 16)), "r"(x1 >> 16));
+    return r;
 }
 
-// x * w^e for the primitive R-th root w_R = 2^(156 * 16 / R) (R | 16), conjugate (w^-e) if INV
-template <int R, int E, bool INV>
-__device__ __forceinline__ uint64_t rotr(uint64_t x) {
-    constexpr int step = 156 * (16 / R);
-    constexpr int e = ((E % R) + R) % R;
-    return mul2k<(INV ? -step * e : step * e)>(x);
+// x 2^72, canonical for any x: 2^72 == -2^40 2^-64, the same with x 2^40 (its low word is zero).
+__device__ __forceinline__ uint64_t rot72(uint64_t x) {
+    const uint32_t x0 = (uint32_t)x, x1 = (uint32_t)(x >> 32);
+    uint64_t r;
+    asm("{\n\t.reg .u32 t, y0, y1, m;\n\t"
+        "add.cc.u32 y0, %2, %1;\n\t"
+        "addc.u32 y1, %3, 0;\n\t"
+        "sub.cc.u32 y0, 0, y0;\n\t"
+        "subc.cc.u32 t, %1, y1;\n\t"
+        "subc.u32 m, 0, 0;\n\t"
+        "sub.cc.u32 y0, y0, m;\n\t"
+        "subc.u32 t, t, 0;\n\t"
+        "mov.b64 %0, {y0, t};\n\t}"
+        : "=l"(r)
+        : "r"(x0 << 8), "r"(__funnelshift_l(x0, x1, 8)), "r"(x1 >> 24));
+    return r;
 }
 
-// In-register DFT of R points over GF(q), natural order in and out:
-//   X_k = sum_n x_n w_R^{+-nk}   (w_R for the forward transform, w_R^-1 for INV; unscaled).
+// In-register DFT of R points over GF(q), natural order, canonical in and out:
+//   X_k = sum_n x_n w_R^{+-nk}   (w_R = 7^((q-1)/R) forward, its inverse for INV; unscaled).
 template <int R, bool INV>
 struct NDft;
-
-template <bool INV>
-struct NDft<1, INV> {
-    __device__ __forceinline__ static void run(uint64_t*) {}
-};
 
 template <bool INV>
 struct NDft<2, INV> {
@@ -162,7 +141,8 @@ struct NDft<4, INV> {
     __device__ __forceinline__ static void run(uint64_t* v) {
         const uint64_t a0 = add(v[0], v[2]), a1 = sub(v[0], v[2]);
         const uint64_t b0 = add(v[1], v[3]);
-        const uint64_t b1 = rotr<4, 1, INV>(sub(v[1], v[3]));
+        // w_4 = 2^48, w_4^-1 = -2^48
+        const uint64_t b1 = rot48(INV ? sub(v[3], v[1]) : sub(v[1], v[3]));
         v[0] = add(a0, b0);
         v[2] = sub(a0, b0);
         v[1] = add(a1, b1);
@@ -170,63 +150,41 @@ struct NDft<4, INV> {
     }
 };
 
-// R = R1 * R2, decimation in frequency on the register array (as the FP64 DftSplit)
-template <int R1, int R2, bool INV>
-struct NDftSplit {
-    static constexpr int R = R1 * R2;
-    template <int N2, int K1>
-    __device__ __forceinline__ static void twiddle_all(uint64_t (&a)[R1][R2]) {
-        if constexpr (N2 < R2) {
-            if constexpr (K1 < R1) {
-                a[K1][N2] = rotr<R, N2 * K1, INV>(a[K1][N2]);
-                twiddle_all<N2, K1 + 1>(a);
-            } else {
-                twiddle_all<N2 + 1, 0>(a);
-            }
-        }
-    }
-    __device__ __forceinline__ static void run(uint64_t* v) {
-        uint64_t a[R1][R2];
-#pragma unroll
-        for (int n2 = 0; n2 < R2; ++n2) {
-            uint64_t col[R1];
-#pragma unroll
-            for (int n1 = 0; n1 < R1; ++n1) col[n1] = v[n1 * R2 + n2];
-            NDft<R1, INV>::run(col);
-#pragma unroll
-            for (int k1 = 0; k1 < R1; ++k1) a[k1][n2] = col[k1];
-        }
-        twiddle_all<0, 0>(a);
-#pragma unroll
-        for (int k1 = 0; k1 < R1; ++k1) {
-            NDft<R2, INV>::run(a[k1]);
-#pragma unroll
-            for (int k2 = 0; k2 < R2; ++k2) v[k1 + R1 * k2] = a[k1][k2];
-        }
-    }
-};
-
 template <bool INV>
 struct NDft<8, INV> {
-    __device__ __forceinline__ static void run(uint64_t* v) { NDftSplit<2, 4, INV>::run(v); }
-};
-template <bool INV>
-struct NDft<16, INV> {
-    __device__ __forceinline__ static void run(uint64_t* v) { NDftSplit<4, 4, INV>::run(v); }
+    __device__ __forceinline__ static void run(uint64_t* v) {
+        uint64_t s[4], d[4];
+#pragma unroll
+        for (int n = 0; n < 4; ++n) s[n] = add(v[n], v[n + 4]);
+        d[0] = sub(v[0], v[4]);
+        if constexpr (!INV) {  // w_8 = -2^24, w_8^2 = 2^48, w_8^3 = -2^72
+            d[1] = rot24(sub(v[5], v[1]));
+            d[2] = rot48(sub(v[2], v[6]));
+            d[3] = rot72(sub(v[7], v[3]));
+        } else {  // w_8^-1 = 2^72, w_8^-2 = -2^48, w_8^-3 = 2^24
+            d[1] = rot72(sub(v[1], v[5]));
+            d[2] = rot48(sub(v[6], v[2]));
+            d[3] = rot24(sub(v[3], v[7]));
+        }
+        NDft<4, INV>::run(s);
+        NDft<4, INV>::run(d);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            v[2 * k] = s[k];
+            v[2 * k + 1] = d[k];
+        }
+    }
 };
 
-// Half table of the L-point transform, stored padded (entry r at qpad8(r) = r + r/16: strided
-// pass indices spread over the 8-byte banks): t[qpad8(r)] = w_L^r, r < L/2. w_L^x for x < L is
-// t[x] or, past L/2, -t[x - L/2] (w_L^(L/2) = -1): a read and a negation, no further product.
+// Table of the L-point transform: w_L^r in Montgomery form at slot qpad8(r) = r + r/16, r < L
+// (strided pass indices spread over the 8-byte banks).
 __host__ __device__ constexpr uint32_t qpad8(uint32_t r) { return r + (r >> 4); }
-__host__ __device__ constexpr uint32_t qpad8_len(uint32_t qm) { return qm + (qm >> 4) + 1; }
+__host__ __device__ constexpr uint32_t qpad8_len(uint32_t n) { return n + (n >> 4) + 1; }
 
 template <int LOG_L>
 __device__ __forceinline__ uint64_t twiddle(const uint64_t* __restrict__ t, uint32_t x, bool inv) {
-    constexpr uint32_t L = 1u << LOG_L, HL = L / 2;
-    if (inv) x = (L - x) & (L - 1);  // w^-x = w^(L - x)
-    const uint64_t w = t[qpad8(x & (HL - 1))];
-    return (x & HL) ? neg(w) : w;
+    constexpr uint32_t L = 1u << LOG_L;
+    return t[qpad8(inv ? (L - x) & (L - 1) : x)];  // w^-x = w^(L - x)
 }
 
 }  // namespace gl
@@ -235,11 +193,25 @@ __device__ __forceinline__ uint64_t twiddle(const uint64_t* __restrict__ t, uint
 #include "llg_fft.cuh"
 
 namespace llg {
+
+// Barrier of a block of one warp (or part of one).
+struct WarpSync {
+    unsigned mask;
+    __device__ __forceinline__ void operator()() const { __syncwarp(mask); }
+};
+
 namespace gl {
 
+// log2 of the values per thread of the NTT kernels: radix-8 passes. Against the radix-16 passes
+// they replace, a pass costs as much per transformed bit, but its code is a third as long (the
+// unrolled radix-16 kernels waited for instruction fetch 4 to 5.5 cycles per issued instruction)
+// and twice the threads share the work.
+constexpr int kLogE = 3;
+
 // Radix pass S of the L-point NTT on the register array (same geometry, positions and exchange
-// pattern as the FP64 passes of llg_fft.cuh; 8-byte field elements in the exchange buffer).
-template <class G, int S, bool INV, bool SYNC_BEFORE_STORE, class SYNC>
+// pattern as the FP64 passes of llg_fft.cuh; 8-byte field elements in the exchange buffer; ES and
+// PADLOG as there). Values are canonical before and after.
+template <class G, int S, bool INV, bool SYNC_BEFORE_STORE, class SYNC, int ES = 1, int PADLOG = 4>
 __device__ __forceinline__ void radix_pass(uint64_t (&v)[G::E], uint64_t* __restrict__ buf,
                                            const uint64_t* __restrict__ qtw, int t, const SYNC& sync) {
     constexpr int R = G::radix(S);
@@ -256,26 +228,22 @@ __device__ __forceinline__ void radix_pass(uint64_t (&v)[G::E], uint64_t* __rest
         uint64_t* vv = v + h * R;
         if constexpr (LOAD) {
 #pragma unroll
-            for (int n1 = 0; n1 < R; ++n1) vv[n1] = buf[phys(base + n1 * ST)];
+            for (int n1 = 0; n1 < R; ++n1) vv[n1] = buf[physp<PADLOG>(base + n1 * ST) * ES];
         }
-        if constexpr (!INV) {
-            NDft<R, false>::run(vv);
-            if constexpr (ST > 1) {
+        if constexpr (INV && ST > 1) {
 #pragma unroll
-                for (int k1 = 1; k1 < R; ++k1)
-                    vv[k1] = mul(vv[k1], twiddle<G::LOG_M_>(qtw, (uint32_t)(n2 * k1) << (G::LE * S), false));
-            }
-        } else {
-            if constexpr (ST > 1) {
+            for (int k1 = 1; k1 < R; ++k1)
+                vv[k1] = mul(vv[k1], twiddle<G::LOG_M_>(qtw, (uint32_t)(n2 * k1) << (G::LE * S), true));
+        }
+        NDft<R, INV>::run(vv);
+        if constexpr (!INV && ST > 1) {
 #pragma unroll
-                for (int k1 = 1; k1 < R; ++k1)
-                    vv[k1] = mul(vv[k1], twiddle<G::LOG_M_>(qtw, (uint32_t)(n2 * k1) << (G::LE * S), true));
-            }
-            NDft<R, true>::run(vv);
+            for (int k1 = 1; k1 < R; ++k1)
+                vv[k1] = mul(vv[k1], twiddle<G::LOG_M_>(qtw, (uint32_t)(n2 * k1) << (G::LE * S), false));
         }
         if constexpr (STORE && !SYNC_BEFORE_STORE) {
 #pragma unroll
-            for (int k1 = 0; k1 < R; ++k1) buf[phys(base + k1 * ST)] = vv[k1];
+            for (int k1 = 0; k1 < R; ++k1) buf[physp<PADLOG>(base + k1 * ST) * ES] = vv[k1];
         }
     }
     if constexpr (STORE && SYNC_BEFORE_STORE) {
@@ -286,33 +254,36 @@ __device__ __forceinline__ void radix_pass(uint64_t (&v)[G::E], uint64_t* __rest
             const int g = beta / ST, n2 = beta % ST;
             const int base = g * L + n2;
 #pragma unroll
-            for (int k1 = 0; k1 < R; ++k1) buf[phys(base + k1 * ST)] = v[h * R + k1];
+            for (int k1 = 0; k1 < R; ++k1) buf[physp<PADLOG>(base + k1 * ST) * ES] = v[h * R + k1];
         }
     }
 }
 
-template <class G, int S, class SYNC = CtaSync>
+// Forward passes S .. P-1 (pass S loads from buf unless S == 0).
+template <class G, int S, class SYNC = CtaSync, int ES = 1, int PADLOG = 4>
 __device__ __forceinline__ void forward_from(uint64_t (&v)[G::E], uint64_t* buf, const uint64_t* qtw,
                                              int t, const SYNC& sync = SYNC()) {
     if constexpr (S < G::P) {
-        radix_pass<G, S, false, false>(v, buf, qtw, t, sync);
+        radix_pass<G, S, false, false, SYNC, ES, PADLOG>(v, buf, qtw, t, sync);
         if constexpr (S < G::P - 1) sync();
-        forward_from<G, S + 1, SYNC>(v, buf, qtw, t, sync);
+        forward_from<G, S + 1, SYNC, ES, PADLOG>(v, buf, qtw, t, sync);
     }
 }
 
-template <class G, int S, bool FIRST_SYNC = true, class SYNC = CtaSync>
+// Inverse passes S down to 0, starting from registers.
+template <class G, int S, bool FIRST_SYNC = true, class SYNC = CtaSync, int ES = 1, int PADLOG = 4>
 __device__ __forceinline__ void inverse_from(uint64_t (&v)[G::E], uint64_t* buf, const uint64_t* qtw,
                                              int t, const SYNC& sync = SYNC()) {
     if constexpr (S >= 0) {
-        radix_pass<G, S, true, FIRST_SYNC && S == G::P - 1>(v, buf, qtw, t, sync);
+        radix_pass<G, S, true, FIRST_SYNC && S == G::P - 1, SYNC, ES, PADLOG>(v, buf, qtw, t, sync);
         if constexpr (S > 0) sync();
-        inverse_from<G, S - 1, false, SYNC>(v, buf, qtw, t, sync);
+        inverse_from<G, S - 1, false, SYNC, ES, PADLOG>(v, buf, qtw, t, sync);
     }
 }
 
+// b^e for b in Montgomery form (the power too).
 __device__ __forceinline__ uint64_t pow(uint64_t b, uint64_t e) {
-    uint64_t r = 1;
+    uint64_t r = ONE;
     while (e) {
         if (e & 1) r = mul(r, b);
         b = mul(b, b);
@@ -321,12 +292,25 @@ __device__ __forceinline__ uint64_t pow(uint64_t b, uint64_t e) {
     return r;
 }
 
-// signed value of a canonical field element that holds an integer of magnitude < q/2
+// signed value of a canonical field element that holds an integer of magnitude below 2^62 (the
+// exactness bound of the lengths): z >= 2^63 stands for z - q = z - 2^64 + 2^32 - 1
 __device__ __forceinline__ long long lift(uint64_t z) {
-    return (z > (Q >> 1)) ? -(long long)(Q - z) : (long long)z;
+    return (long long)(z + (uint64_t)(uint32_t)((int32_t)(uint32_t)(z >> 32) >> 31));
 }
-__device__ __forceinline__ uint64_t from_int(long long x) {
-    return (x < 0) ? Q - (uint64_t)(-x) : (uint64_t)x;
+// a digit as a canonical element
+__device__ __forceinline__ uint64_t from_int(int x) {
+    return (uint64_t)(long long)x - (uint64_t)(uint32_t)(x >> 31);
+}
+
+// One balanced-digit step at b bits: v = x + c 2^b with x in [-2^(b-1), 2^(b-1)), the carry
+// c = floor((v + 2^(b-1)) / 2^b) (lucaslehmer.cpp:299-303).
+__device__ __forceinline__ int balance64(long long v, int b, long long& c) {
+    c = (v + (1LL << (b - 1))) >> b;
+    return (int)((uint32_t)v - ((uint32_t)c << b));
+}
+__device__ __forceinline__ int balance32(int v, int b, int& c) {
+    c = (v + (1 << (b - 1))) >> b;
+    return v - (c << b);
 }
 
 }  // namespace gl

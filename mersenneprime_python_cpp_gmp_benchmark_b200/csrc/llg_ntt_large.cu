@@ -1,19 +1,32 @@
 // Two-pass exact IBDWT over GF(2^64 - 2^32 + 1) for N = 2^14 .. 2^23, the residue resident in HBM
 // as N field elements (8N bytes, the same footprint as the FP64 engine's N/2 complex values).
 //
-// Same four-step structure and carry scheme as the FP64 two-pass engine (llg_large.cu), with one
+// Same four-step structure and tile layout as the FP64 two-pass engine (llg_large.cu), with one
 // digit per element instead of two (no real-FFT packing, so the column pass needs no partner
 // column: one block per column, pointwise square):
-//   row pass (kNttRowG consecutive rows a, all C columns):  inverse C-point NTT, unweight (and
-//       1/N), signed lift, carry, "- 2", weight, forward C-point NTT;
+//   row pass (a tile of kNttRowG consecutive rows a, all C columns):  inverse C-point NTT, unweight
+//       (and 1/N), signed lift, carry, "- 2", weight, forward C-point NTT;
 //   column pass (one column c):  twiddle w_N^{ac}, forward R-point NTT, square, inverse, w_N^{-ac}.
+// A row tile interleaves its rows across the lanes of every warp (thread t: row t % G, NTT thread
+// t / G): loads and stores go straight between memory and registers, and the carries between the
+// rows of a tile are lane shuffles.
 // Carry: digit j = a + R b, so the chain runs down the rows of each column. Each row's carry-out
 // is taken from zero (independent of its carry-in); the carry-in is absorbed with two
 // renormalisations (hops 2, 3) whose own carries move one row further down, and the last, tiny
-// remainder is added without renormalising (hop 4). A block's last row therefore publishes three
-// carries, all computable without the previous block (a block has >= 3 rows); block k+1 reads them
-// after a bounded wait on block k's flag (tickets in launch order keep block k resident). Block 0
-// recomputes rows R-3 .. R-1 for the wrap-around carry into row 0 (2^p == 1).
+// remainder is added without renormalising (hop 4). A tile's last row therefore publishes three
+// carries, all computable without the previous tile (a tile has >= 3 rows); tile k+1 reads them
+// after a bounded wait on tile k's flag (tickets in launch order keep tile k resident). The
+// wrap-around carry into row 0 (2^p == 1) comes from row R-1: the first ticket is a separate job
+// that runs the last tile's rows through the inverse NTT and the hops and publishes their
+// carries, one column on, in the slot tile 0 reads; the last tile waits (bounded) for that job
+// before overwriting those rows.
+//
+// Both passes are bound by the integer ALU (the arithmetic of llg_ntt.cuh). Measured, us a squaring
+// replayed from graphs, against radix-16 passes of one row per warp group with the 128-bit
+// reduction: N = 2^16 55.5 -> 18.5, 2^18 67.3 -> 39.1, 2^21 176.8 -> 107.0, 2^23 654 -> 436. At 2^21 the
+// row pass issues 37.2 M warp instructions (47.3 M before) at 57% of the ALU's rate (39%), the
+// column pass 31.1 M at 67% (58%); neither waits for instruction fetch any more (5.5 cycles per
+// issued instruction before).
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -29,7 +42,6 @@ namespace llg {
 namespace {
 
 constexpr int kNttRowG = 4;
-constexpr unsigned long long kNttSpinLimit = 1ull << 22;
 
 __device__ __forceinline__ uint64_t twiddle_N(const NttLargeArgs& A, uint32_t x) {
     return gl::mul(__ldg(A.tw1 + (x & ((1u << A.tw_shift) - 1u))), __ldg(A.tw2 + (x >> A.tw_shift)));
@@ -37,272 +49,213 @@ __device__ __forceinline__ uint64_t twiddle_N(const NttLargeArgs& A, uint32_t x)
 
 }  // namespace
 
+template <int LOG_C>
+using NttRowG = SmallG<LOG_C, gl::kLogE>;
+template <int LOG_R>
+using NttColG = SmallG<LOG_R, gl::kLogE>;
+
+// exchange-buffer slots of a tile: its rows of C + C/8 padded slots
+template <int LOG_C>
+__host__ __device__ constexpr int ntt_row_slots() { return kNttRowG * ((1 << LOG_C) + ((1 << LOG_C) >> gl::kLogE)); }
+
 template <int LOG_C, int MODE>
-__global__ void __launch_bounds__(kNttRowG * (1 << LOG_C) / 16, 2) ntt_row(const NttLargeArgs A) {
-    using GC = SmallG<LOG_C>;
-    constexpr int C = GC::M, TR = GC::T, E = GC::E, G = kNttRowG, T = G * TR;
-    constexpr int RS = GC::PAD + 1;  // odd row stride (8-byte slots): the G rows of a slot hit G banks
-    constexpr int QL = (int)gl::qpad8_len(C / 2);
+__global__ void __launch_bounds__(kNttRowG * NttRowG<LOG_C>::T, 1024 / (kNttRowG * NttRowG<LOG_C>::T) > 8 ? 8 : 1024 / (kNttRowG * NttRowG<LOG_C>::T))
+    ntt_row(const NttLargeArgs A) {
+    using GC = NttRowG<LOG_C>;
+    constexpr int C = GC::M, TR = GC::T, E = GC::E, G = kNttRowG, T = G * TR, PL = gl::kLogE;
+    constexpr int QL = (int)gl::qpad8_len(C);
+    constexpr unsigned FULL = 0xffffffffu;
+    static_assert(T % 32 == 0 && 32 % G == 0 && G >= 4 && C % T == 0, "whole warps of whole row groups");
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    uint64_t* bufs = reinterpret_cast<uint64_t*>(smem_raw);   // G exchange buffers
-    uint64_t* qtw = bufs + G * RS;                             // padded half table
-    int* carr2 = reinterpret_cast<int*>(qtw + QL + (QL & 1));  // G x C hop-2 carry-outs
-    int* carr3 = carr2 + G * C;                                // G x C hop-3 carry-outs
-    long long* carr1 = reinterpret_cast<long long*>(bufs);     // G x C hop-1 carry-outs (reuses bufs)
-    __shared__ int s_blk;
+    uint64_t* xbuf = reinterpret_cast<uint64_t*>(smem_raw);  // exchange: slot physp(x) * G + row
+    uint64_t* qtw = xbuf + ntt_row_slots<LOG_C>();            // padded twiddle table
+    uint64_t* swB = qtw + QL;                                 // C column weights
+    uint64_t* siwB = swB + C;                                 // C inverse column weights
+    int* ssB = reinterpret_cast<int*>(siwB + C);              // C column weight exponents
+    __shared__ int s_job;
     __shared__ unsigned s_epoch;
 
-    const int t = threadIdx.x, rg = t / TR, tr = t % TR;
-    uint64_t* buf = bufs + rg * RS;
+    const int t = threadIdx.x, ra = t % G, tr = t / G;
+    uint64_t* buf = xbuf + ra;
     const int N = 1 << A.logN, R = A.R;
-    using RowSync = typename std::conditional<(TR >= 32), NamedSync, CtaSync>::type;
-    RowSync gsync;
-    if constexpr (TR >= 32) gsync = NamedSync{1u + (unsigned)rg, (unsigned)TR};
+    const CtaSync sync;
 
+    // the next pass may launch once every block of this one has started; constant tables first,
+    // nothing the previous pass writes before the wait
+    pdl_launch_dependents();
+    for (int k = t; k < QL; k += T) cp_async<8>(qtw + k, A.qtwC + k);
+    for (int k = t; k < C; k += T) {
+        cp_async<8>(swB + k, A.wB + k);
+        if (MODE != LARGE_INIT) cp_async<8>(siwB + k, A.iwB + k);
+        cp_async<4>(ssB + k, A.sB + k);
+    }
+    pdl_wait_previous();
     if (t == 0) {
         const unsigned ep = *reinterpret_cast<volatile unsigned*>(&A.ctl->epoch);
         s_epoch = ep;
         if (MODE == LARGE_INIT) {
-            s_blk = blockIdx.x;
+            s_job = blockIdx.x;
         } else {
-            const int b = (int)atomicAdd(&A.ctl->ticket[ep & 1], 1u);
-            if (b == A.nblocks - 1) {
+            // tickets in launch order: ticket 0 is the wrap-around job, ticket k tile k - 1
+            const int tk = (int)atomicAdd(&A.ctl->ticket[ep & 1], 1u);
+            if (tk == A.nblocks) {
                 // every block of this launch holds its ticket: both counters can be reset
                 A.ctl->ticket[(ep + 1) & 1] = 0u;
                 A.ctl->ticket[ep & 1] = 0u;
             }
-            s_blk = b;
+            s_job = tk - 1;
         }
     }
-    for (int k = t; k < QL; k += T) qtw[k] = A.qtwC[k];
     __syncthreads();
-    const int blk = s_blk;
+    const int job = s_job;  // -1: the wrap-around job (rows R-G .. R-1), else the tile
     const unsigned ep = s_epoch;
-    const int a0 = blk * G;
-    const int a = a0 + rg;
+    const bool wrap_job = job < 0;
+    const int a = (wrap_job ? R - G : job * G) + ra;  // this thread's row
     const int sA = __ldg(A.sA + a);
 
     uint64_t v[E];
-    long long x[E];
-
-    // unweight (with 1/N), lift, hop 1 of row `row` from the inverse transform in v
-    auto hop1 = [&](int row, long long* c1out) {
-        const int sa = __ldg(A.sA + row);
-        const uint64_t iwa = __ldg(A.iwA + row);
+    int x[E];
+    uint32_t big = 0u, wrap = 0u;  // bit i: the digit has q + 1 bits; sA + sB >= N
+    auto kinds = [&]() {
 #pragma unroll
         for (int i = 0; i < E; ++i) {
-            const int b = tr + TR * i;
-            const int sb = __ldg(A.sB + b);
-            const bool o = sa + sb >= N;
-            const int s = o ? sa + sb - N : sa + sb;
-            uint64_t z = gl::mul(v[i], gl::mul(iwa, __ldg(A.iwB + b)));
-            if (o) z = gl::add(z, z);  // w^-(s_j) = w^-sA w^-sB w^N, w^N = 2
-            long long c;
-            x[i] = balance(gl::lift(z), A.q + (s < A.rem), c);
-            c1out[i] = c;
+            const int sb = ssB[tr + TR * i];
+            const bool o = sA + sb >= N;
+            const int s = o ? sA + sb - N : sA + sb;
+            big |= (uint32_t)(s < A.rem) << i;
+            wrap |= (uint32_t)o << i;
         }
     };
-    auto bits_of = [&](int row, int b) {
-        const int sa = __ldg(A.sA + row), sb = __ldg(A.sB + b);
-        const int s = (sa + sb >= N) ? sa + sb - N : sa + sb;
-        return A.q + (s < A.rem);
-    };
+    auto bits = [&](int i) { return A.q + (int)((big >> i) & 1u); };
 
     if constexpr (MODE == LARGE_INIT) {
 #pragma unroll
-        for (int i = 0; i < E; ++i) {
-            const int b = tr + TR * i;
-            x[i] = A.digits[(size_t)a + (size_t)R * b];
-        }
+        for (int i = 0; i < E; ++i) x[i] = A.digits[(size_t)a + (size_t)R * (tr + TR * i)];
+        cp_async_wait_all();
+        __syncthreads();  // the tables are in shared memory
+        kinds();
     } else {
-        // ---- block 0: wrap-around carries from rows R-3 .. R-1 (into row 0, column b + 1), the
-        //      three rows transformed side by side (row group 3 repeats row R-1) ----
-        if (blk == 0) {
-            long long* hin1 = A.halo;  // c1 of row R-1, shifted to the column it feeds
-            int* hin2 = reinterpret_cast<int*>(A.halo + C);
-            int* hin3 = hin2 + C;
-            const int ah = R - 3 + (rg < 3 ? rg : 2);
-#pragma unroll
-            for (int j = 0; j < E; ++j) v[j] = A.V[(size_t)(tr * E + j) * R + ah];
-            gl::inverse_from<GC, GC::P - 1, false>(v, buf, qtw, tr, gsync);
-            __syncthreads();  // the exchange buffers become the hop-1 carry array
-            if (t == 0) {
-                // rows R-3 .. R-1 are read: the last block may overwrite them
-                __threadfence();
-                *reinterpret_cast<volatile unsigned*>(&A.ctl->halo_read) = ep + 1u;
-            }
-            long long c1[E];
-            hop1(ah, c1);
-#pragma unroll
-            for (int i = 0; i < E; ++i) carr1[rg * C + tr + TR * i] = c1[i];
-            __syncthreads();
-            if (rg == 1) {  // row R-2: hop 2 with row R-3's carry
-#pragma unroll
-                for (int i = 0; i < E; ++i) {
-                    const int b = tr + TR * i;
-                    long long c;
-                    balance(x[i] + carr1[b], bits_of(ah, b), c);
-                    carr2[b] = (int)c;
-                }
-            }
-            __syncthreads();
-            if (rg == 2) {  // row R-1: hops 2 and 3
-#pragma unroll
-                for (int i = 0; i < E; ++i) {
-                    const int b = tr + TR * i;
-                    const int nb = bits_of(ah, b);
-                    long long c;
-                    const long long y = balance(x[i] + carr1[C + b], nb, c);
-                    const long long c2 = c;
-                    balance(y + carr2[b], nb, c);
-                    const int to = (b + 1) & (C - 1);
-                    hin1[to] = c1[i];
-                    hin2[to] = (int)c2;
-                    hin3[to] = (int)c;
-                }
-            }
-            __syncthreads();
-        }
-
-        // ---- load the block's rows (coalesced: kNttRowG contiguous elements per column slot) ----
         {
-            uint64_t tmp[G * C / T];
+            const uint64_t* lp = A.V + (size_t)(tr * E) * R + a;
 #pragma unroll
-            for (int r = 0; r < G * C / T; ++r) {
-                const int qq = t + T * r, pos = qq / G, ra = qq % G;
-                tmp[r] = A.V[(size_t)pos * R + a0 + ra];
-            }
-#pragma unroll
-            for (int r = 0; r < G * C / T; ++r) {
-                const int qq = t + T * r, pos = qq / G, ra = qq % G;
-                bufs[ra * RS + phys(pos)] = tmp[r];
-            }
+            for (int j = 0; j < E; ++j) v[j] = __ldcg(lp + (size_t)j * R);
         }
-        __syncthreads();
-#pragma unroll
-        for (int j = 0; j < E; ++j) v[j] = buf[phys(tr * E + j)];
-        gl::inverse_from<GC, GC::P - 1, false>(v, buf, qtw, tr, gsync);
-        __syncthreads();  // the exchange buffers become the hop-1 carry array
+        cp_async_wait_all();
+        __syncthreads();  // the tables are in shared memory
+        gl::inverse_from<GC, GC::P - 1, false, CtaSync, G, PL>(v, buf, qtw, tr, sync);
+        kinds();
 
-        // hop 1, every row
-        {
-            long long c1[E];
-            hop1(a, c1);
-#pragma unroll
-            for (int i = 0; i < E; ++i) {
-                const int b = tr + TR * i;
-                carr1[rg * C + b] = c1[i];
-                if (rg == G - 1) A.c1[(size_t)blk * C + b] = c1[i];
-            }
-        }
-        __syncthreads();
-        // hop 2, rows fed from inside the block
-        if (rg >= 1) {
-#pragma unroll
-            for (int i = 0; i < E; ++i) {
-                const int b = tr + TR * i;
-                long long c;
-                x[i] = balance(x[i] + carr1[(rg - 1) * C + b], bits_of(a, b), c);
-                carr2[rg * C + b] = (int)c;
-                if (rg == G - 1) A.c2[(size_t)blk * C + b] = (int)c;
-            }
-        }
-        __syncthreads();
-        // hop 3, rows whose hop-2 input is already known
-        if (rg >= 2) {
-#pragma unroll
-            for (int i = 0; i < E; ++i) {
-                const int b = tr + TR * i;
-                long long c;
-                x[i] = balance(x[i] + carr2[(rg - 1) * C + b], bits_of(a, b), c);
-                carr3[rg * C + b] = (int)c;
-                if (rg == G - 1) A.c3[(size_t)blk * C + b] = (int)c;
-            }
-        }
-        __threadfence();  // carry-out stores ordered before the flag
-        __syncthreads();
-        if (t == 0) {
-            __threadfence();
-            *reinterpret_cast<volatile unsigned*>(&A.flags[blk]) = ep + 1u;
-            if (blk > 0) wait_flag(&A.flags[blk - 1], ep + 1u, A.ctl, kNttSpinLimit);
-        }
-        __syncthreads();
-        const long long* hin1 = A.halo;
-        const int* hin2 = reinterpret_cast<const int*>(A.halo + C);
-        const int* hin3 = hin2 + C;
-        // hop 2 of the block's first row (previous block, or the wrap, and the "- 2" at digit 0)
-        if (rg == 0) {
-#pragma unroll
-            for (int i = 0; i < E; ++i) {
-                const int b = tr + TR * i;
-                long long cin = (blk > 0) ? __ldcg(A.c1 + (size_t)(blk - 1) * C + b) : hin1[b];
-                if (a == 0 && b == 0) cin -= 2;
-                long long c;
-                x[i] = balance(x[i] + cin, bits_of(a, b), c);
-                carr2[b] = (int)c;
-            }
-        }
-        __syncthreads();
-        // hop 3 of the first two rows
-        if (rg <= 1) {
-#pragma unroll
-            for (int i = 0; i < E; ++i) {
-                const int b = tr + TR * i;
-                const int cin = (rg == 1) ? carr2[b] : (blk > 0) ? __ldcg(A.c2 + (size_t)(blk - 1) * C + b) : hin2[b];
-                long long c;
-                x[i] = balance(x[i] + cin, bits_of(a, b), c);
-                carr3[rg * C + b] = (int)c;
-            }
-        }
-        __syncthreads();
-        // hop 4: the remainder of the row above, not renormalised
+        // ---- unweight, lift, hop 1 of every row; hops 2 to 4 of the rows whose carry-in comes from
+        //      inside the tile. Row G-1 publishes its three carry-outs (the wrap job: one column on).
+        const int slot = job + 1;
+        const uint64_t ia = __ldg(A.iwA + a), ia2 = gl::add(ia, ia);
+        int c3r[E];  // hop-3 carry-outs (row 1's, which row 2 needs, are formed after the wait)
 #pragma unroll
         for (int i = 0; i < E; ++i) {
             const int b = tr + TR * i;
-            const int cin = (rg > 0) ? carr3[(rg - 1) * C + b] : (blk > 0) ? __ldcg(A.c3 + (size_t)(blk - 1) * C + b) : hin3[b];
-            x[i] += cin;
+            const int nb = bits(i);
+            // w^-s = w^-sA w^-sB, times w^N = 2 past N
+            const uint64_t z = gl::mul(v[i], gl::mul((wrap >> i) & 1u ? ia2 : ia, siwB[b]));
+            long long c1, c;
+            int y = gl::balance64(gl::lift(z), nb, c1);
+            c = c1;
+            const long long in1 = __shfl_up_sync(FULL, c1, 1, G);
+            int c2 = 0, c3 = 0;
+            if (ra > 0) {
+                y = gl::balance64((long long)y + in1, nb, c);
+                c2 = (int)c;
+            }
+            const int in2 = __shfl_up_sync(FULL, c2, 1, G);
+            if (ra > 1) y = gl::balance32(y + in2, nb, c3);
+            const int in3 = __shfl_up_sync(FULL, c3, 1, G);
+            if (ra > 2) y += in3;
+            if (ra == G - 1) {
+                const size_t o = (size_t)slot * C + (wrap_job ? ((b + 1) & (C - 1)) : b);
+                A.c1[o] = c1;
+                A.c2[o] = c2;
+                A.c3[o] = c3;
+            }
+            x[i] = y;
+        }
+        if (ra == G - 1) __threadfence();  // each publisher orders its carry stores before the flag
+        __syncthreads();
+        if (t == 0) *reinterpret_cast<volatile unsigned*>(&A.flags[slot]) = ep + 1u;
+        if (wrap_job) return;
+        // ---- the tile's first row: hops 2 to 4 from the previous tile's last row (or the wrap). The
+        //      row passes through the exchange buffer, so that every thread takes C / T of its
+        //      columns rather than one lane in G all of them. ----
+        int* row0 = reinterpret_cast<int*>(xbuf);  // C digits of row 0
+        int* h2 = row0 + C;                        // its hop-2 and hop-3 carry-outs
+        int* h3 = h2 + C;
+        if (ra == 0) {
+#pragma unroll
+            for (int i = 0; i < E; ++i) row0[tr + TR * i] = x[i];
+        }
+        if (t == 0) wait_flag(&A.flags[job], ep + 1u, A.ctl, kSpinLimit);
+        __syncthreads();
+        {
+            const int s0 = __ldg(A.sA + job * G);
+            const size_t o = (size_t)job * C;
+#pragma unroll
+            for (int k = 0; k < C / T; ++k) {
+                const int b = t + T * k;
+                const int sb = ssB[b];
+                const int s = (s0 + sb >= N) ? s0 + sb - N : s0 + sb;
+                const int nb = A.q + (s < A.rem);
+                long long cin = __ldcg(A.c1 + o + b), c;
+                if (job == 0 && b == 0) cin -= 2;  // the "- 2" of s^2 - 2 (digit 0)
+                int y = gl::balance64((long long)row0[b] + cin, nb, c), c3;
+                h2[b] = (int)c;
+                y = gl::balance32(y + __ldcg(A.c2 + o + b), nb, c3);
+                h3[b] = c3;
+                row0[b] = y + __ldcg(A.c3 + o + b);
+            }
+        }
+        __syncthreads();
+        // row 1: hops 3 and 4 from row 0; row 2: hop 4 from row 1
+#pragma unroll
+        for (int i = 0; i < E; ++i) {
+            const int b = tr + TR * i;
+            c3r[i] = 0;
+            if (ra == 0) x[i] = row0[b];
+            else if (ra == 1) x[i] = gl::balance32(x[i] + h2[b], bits(i), c3r[i]) + h3[b];
+            const int in3 = __shfl_up_sync(FULL, c3r[i], 1, G);
+            if (ra == 2) x[i] += in3;
         }
         if (MODE == LARGE_FINAL || A.dump) {
 #pragma unroll
-            for (int i = 0; i < E; ++i) {
-                const int b = tr + TR * i;
-                A.digits[(size_t)a + (size_t)R * b] = (int)x[i];
-            }
+            for (int i = 0; i < E; ++i) A.digits[(size_t)a + (size_t)R * (tr + TR * i)] = x[i];
         }
         if constexpr (MODE == LARGE_FINAL) return;
-        __syncthreads();  // carry reads done before the exchange buffers are reused
     }
 
     // ---- weight, forward row NTT, store ----
-    const uint64_t wa = __ldg(A.wA + a);
+    const uint64_t wa = __ldg(A.wA + a), wah = gl::mul(wa, gl::HALF);
 #pragma unroll
-    for (int i = 0; i < E; ++i) {
-        const int b = tr + TR * i;
-        const bool o = sA + __ldg(A.sB + b) >= N;
-        uint64_t w = gl::mul(wa, __ldg(A.wB + b));
-        if (o) w = gl::mul2k<191>(w);  // / 2
-        v[i] = gl::mul(gl::from_int(x[i]), w);
+    for (int i = 0; i < E; ++i)
+        v[i] = gl::mul(gl::from_int(x[i]), gl::mul((wrap >> i) & 1u ? wah : wa, swB[tr + TR * i]));
+    // the first forward pass stores after a barrier: the first row's carries may still be read from
+    // the exchange buffer
+    gl::radix_pass<GC, 0, false, true, CtaSync, G, PL>(v, buf, qtw, tr, sync);
+    static_assert(GC::P > 1, "at least two row passes");
+    sync();
+    gl::forward_from<GC, 1, CtaSync, G, PL>(v, buf, qtw, tr, sync);
+    if (MODE == LARGE_ITER && job == A.nblocks - 1) {
+        // rows R-G .. R-1 are the wrap job's input: wait (bounded) until it has read them
+        if (t == 0) wait_flag(&A.flags[0], ep + 1u, A.ctl, kSpinLimit);
+        __syncthreads();
     }
-    gl::forward_from<GC, 0>(v, buf, qtw, tr, gsync);
+    uint64_t* vp = A.V + (size_t)(tr * E) * R + a;
 #pragma unroll
-    for (int j = 0; j < E; ++j) buf[phys(tr * E + j)] = v[j];
-    if (MODE == LARGE_ITER && blk == A.nblocks - 1 && t == 0) {
-        // rows R-3 .. R-1 are block 0's wrap-around input: wait (bounded) until it has read them
-        wait_flag(&A.ctl->halo_read, ep + 1u, A.ctl, kNttSpinLimit);
-    }
-    __syncthreads();
-#pragma unroll
-    for (int r = 0; r < G * C / T; ++r) {
-        const int qq = t + T * r, pos = qq / G, ra = qq % G;
-        A.V[(size_t)pos * R + a0 + ra] = bufs[ra * RS + phys(pos)];
-    }
+    for (int j = 0; j < E; ++j) __stcg(vp + (size_t)j * R, v[j]);
 }
 
 template <int LOG_R>
-__global__ void __launch_bounds__((1 << LOG_R) / 16, (LOG_R >= 13 ? 2 : 3)) ntt_col(const NttLargeArgs A) {
-    using GR = SmallG<LOG_R>;
+__global__ void __launch_bounds__(NttColG<LOG_R>::T, 1024 / NttColG<LOG_R>::T > 16 ? 16 : 1024 / NttColG<LOG_R>::T)
+    ntt_col(const NttLargeArgs A) {
+    using GR = NttColG<LOG_R>;
     constexpr int R = GR::M, TC = GR::T, E = GR::E;
-    constexpr int QL = (int)gl::qpad8_len(R / 2);
+    constexpr int QL = (int)gl::qpad8_len(R);
     extern __shared__ __align__(16) unsigned char smem_raw[];
     uint64_t* buf = reinterpret_cast<uint64_t*>(smem_raw);
     uint64_t* qtw = buf + GR::PAD;
@@ -310,7 +263,8 @@ __global__ void __launch_bounds__((1 << LOG_R) / 16, (LOG_R >= 13 ? 2 : 3)) ntt_
     const int tc = threadIdx.x;
     const int c = blockIdx.x;
     const int N = 1 << A.logN;
-    for (int k = tc; k < QL; k += TC) qtw[k] = A.qtwR[k];
+    pdl_launch_dependents();  // as in ntt_row
+    for (int k = tc; k < QL; k += TC) cp_async<8>(qtw + k, A.qtwR + k);
     // four-step twiddle w_N^{a c}, a = tc + TC i: w_N^{c tc} * w_N^{c TC i}
     for (int i = tc; i < E; i += TC) {
         const uint32_t xi = (uint32_t)(((uint64_t)c * TC * i) & (uint64_t)(N - 1));
@@ -319,15 +273,15 @@ __global__ void __launch_bounds__((1 << LOG_R) / 16, (LOG_R >= 13 ? 2 : 3)) ntt_
     }
     const uint32_t xq = (uint32_t)(((uint64_t)c * tc) & (uint64_t)(N - 1));
     uint64_t* col = A.V + (size_t)__ldg(A.pos_of_c + c) * R;
+    const uint64_t q = twiddle_N(A, xq);
+    pdl_wait_previous();
     uint64_t v[E];
 #pragma unroll
     for (int i = 0; i < E; ++i) v[i] = col[tc + TC * i];
+    cp_async_wait_all();
     __syncthreads();
-    {
-        const uint64_t q = twiddle_N(A, xq);
 #pragma unroll
-        for (int i = 0; i < E; ++i) v[i] = gl::mul(v[i], gl::mul(q, ptab[i]));
-    }
+    for (int i = 0; i < E; ++i) v[i] = gl::mul(v[i], gl::mul(q, ptab[i]));
     gl::forward_from<GR, 0>(v, buf, qtw, tc);
 #pragma unroll
     for (int j = 0; j < E; ++j) v[j] = gl::mul(v[j], v[j]);
@@ -342,15 +296,31 @@ __global__ void __launch_bounds__((1 << LOG_R) / 16, (LOG_R >= 13 ? 2 : 3)) ntt_
 
 template <int LOG_C>
 static size_t ntt_row_smem() {
-    using GC = SmallGeom<LOG_C>;
-    const size_t ql = gl::qpad8_len(GC::M / 2);
-    return sizeof(uint64_t) * (kNttRowG * (GC::PAD + 1) + ql + (ql & 1)) + 2 * sizeof(int) * kNttRowG * GC::M;
+    constexpr int C = 1 << LOG_C;
+    return sizeof(uint64_t) * (ntt_row_slots<LOG_C>() + gl::qpad8_len(C) + 2 * C) + sizeof(int) * C;
 }
 
 template <int LOG_R>
 static size_t ntt_col_smem() {
-    using GR = SmallGeom<LOG_R>;
-    return sizeof(uint64_t) * (GR::PAD + gl::qpad8_len(GR::M / 2) + 2 * GR::E);
+    using GR = NttColG<LOG_R>;
+    return sizeof(uint64_t) * (GR::PAD + gl::qpad8_len(GR::M) + 2 * GR::E);
+}
+
+// Programmatic stream serialisation, as the FP64 passes at power-of-two lengths.
+template <class... KArgs>
+static cudaError_t launch_pdl(void (*kernel)(KArgs...), int grid, int block, size_t smem, cudaStream_t st,
+                              const NttLargeArgs& a) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3((unsigned)block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, a);
 }
 
 template <int LOG_C, int MODE>
@@ -359,16 +329,16 @@ static cudaError_t ntt_row_attr() {
                                 (int)ntt_row_smem<LOG_C>());
 }
 
+// INIT: one block per tile. ITER / FINAL: one block more, for the wrap-around job.
 template <int LOG_C, int MODE>
 static cudaError_t ntt_row_t(const NttLargeArgs& a, cudaStream_t st) {
-    ntt_row<LOG_C, MODE><<<a.nblocks, kNttRowG * (1 << LOG_C) / 16, ntt_row_smem<LOG_C>(), st>>>(a);
-    return cudaGetLastError();
+    return launch_pdl(ntt_row<LOG_C, MODE>, a.nblocks + (MODE == LARGE_INIT ? 0 : 1), kNttRowG * NttRowG<LOG_C>::T,
+                      ntt_row_smem<LOG_C>(), st, a);
 }
 
 template <int LOG_R>
 static cudaError_t ntt_col_t(const NttLargeArgs& a, cudaStream_t st) {
-    ntt_col<LOG_R><<<a.C, (1 << LOG_R) / 16, ntt_col_smem<LOG_R>(), st>>>(a);
-    return cudaGetLastError();
+    return launch_pdl(ntt_col<LOG_R>, a.C, NttColG<LOG_R>::T, ntt_col_smem<LOG_R>(), st, a);
 }
 
 template <int LOG_R>
