@@ -68,6 +68,7 @@ constexpr int kSmallLogMax = 13;  // N = 8192
 struct DeviceTables {
     std::map<uint32_t, double2*> qtw;      // quarter-wave twiddles of the M-point FFT, by M
     std::map<uint32_t, double2*> qtw_s;    // the same in the spread layout (qpad_s), by M
+    std::map<uint32_t, double2*> qtw_p;    // twiddles in pass order (pass_twiddle_table), by 64 log2 M + log2 E
     uint64_t* nqtw[kSmallLogMax + 1] = {}; // NTT: padded twiddle table of the N-point transform
     NttConst nk[kSmallLogMax + 1] = {};
 };
@@ -129,6 +130,19 @@ int get_qtw(int dev, uint32_t m, const double2** out, bool spread = false) {
     if (!d) {
         // padded layout (qpad), or the spread one (qpad_s)
         std::vector<double2> h = spread ? spread_quarter_table(m) : padded_quarter_table(m);
+        CK(cudaMalloc(&d, h.size() * sizeof(double2)));
+        CK(cudaMemcpy(d, h.data(), h.size() * sizeof(double2), cudaMemcpyHostToDevice));
+        count_h2d(h.size() * sizeof(double2));
+    }
+    *out = d;
+    return LLG_OK;
+}
+
+int get_pass_table(int dev, int log_m, int log_e, const double2** out) {
+    std::lock_guard<std::mutex> lk(g_mx);
+    double2*& d = g_tables[dev].qtw_p[64u * (uint32_t)log_m + (uint32_t)log_e];
+    if (!d) {
+        std::vector<double2> h = pass_twiddle_table(log_m, log_e);
         CK(cudaMalloc(&d, h.size() * sizeof(double2)));
         CK(cudaMemcpy(d, h.data(), h.size() * sizeof(double2), cudaMemcpyHostToDevice));
         count_h2d(h.size() * sizeof(double2));
@@ -404,10 +418,11 @@ int launch_group(llg_batch* b, Group& g, cudaStream_t caller) {
                             (SmallResult*)g.d_results, g.st));
     } else if (is_small_pow2_length(g.n)) {
         const double2* qtw = nullptr;
-        int rc = get_qtw(b->dev, g.n / 2, &qtw, small_fp64_spread_table(ilog2_exact(g.n)));
+        const int ln = ilog2_exact(g.n), le = small_fp64_log_e(ln, cnt);
+        int rc = small_fp64_pass_table(le) ? get_pass_table(b->dev, ln - 1, le, &qtw) : get_qtw(b->dev, g.n / 2, &qtw, true);
         if (rc) return rc;
         float* elog = (cnt == 1) ? b->d_errlog : nullptr;
-        CK(launch_small_fp64(ilog2_exact(g.n), (const SmallJob*)g.d_jobs, cnt, qtw, (int64_t*)g.d_digits,
+        CK(launch_small_fp64(ln, le, (const SmallJob*)g.d_jobs, cnt, qtw, (int64_t*)g.d_digits,
                              (SmallResult*)g.d_results, elog, g_abort_err.load(), g.st));
     } else {
         int r0 = 0, ll = 0;

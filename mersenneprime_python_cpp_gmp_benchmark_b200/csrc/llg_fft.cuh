@@ -17,8 +17,11 @@ namespace llg {
 
 // Twiddle table of a geometry: e^{-2 pi i r / M} at slot qpad(r) for r < M/4 (TW_QUARTER: the
 // other quadrants by rotation), r < M/2 (TW_HALF: the other half by negation), or r < M (TW_FULL:
-// one table read, no fold); TW_QUARTER_S: the quarter table at slot qpad_s(r).
-enum { TW_QUARTER = 0, TW_HALF = 1, TW_FULL = 2, TW_QUARTER_S = 3 };
+// one table read, no fold); TW_QUARTER_S: the quarter table at slot qpad_s(r); TW_PASS: the twiddles
+// of every radix pass in the order the pass reads them, entry (k1 - 1) ST + n2 of pass S holds
+// w^(n2 k1 E^S) (pass_offset(S) on): consecutive lanes read consecutive slots, and nothing is folded
+// or multiplied up from other entries. About M entries, where the quarter table has M / 4.
+enum { TW_QUARTER = 0, TW_HALF = 1, TW_FULL = 2, TW_QUARTER_S = 3, TW_PASS = 4 };
 
 // L = 2^LOG_M points, E = 2^LOG_E values per thread (radix-E passes, the last one RLAST).
 template <int LOG_M, int LOG_E = 4>
@@ -35,6 +38,12 @@ struct SmallGeom {
     static __host__ __device__ constexpr int radix(int s) { return s == P - 1 ? RLAST : E; }
     static __host__ __device__ constexpr int len(int s) { return M >> (LOG_E * s); }
     static __host__ __device__ constexpr int stride(int s) { return len(s) / radix(s); }
+    // TW_PASS: slot of pass s's first twiddle (passes of stride 1 have none)
+    static __host__ __device__ constexpr int pass_offset(int s) {
+        int o = 0;
+        for (int i = 0; i < s; ++i) o += (radix(i) - 1) * stride(i);
+        return o;
+    }
 };
 
 __device__ __forceinline__ int phys(int x) { return x + (x >> 4); }
@@ -90,6 +99,12 @@ __device__ __forceinline__ int pos_of_freq(int k) {
 struct CtaSync {
     __device__ __forceinline__ void operator()() const { __syncthreads(); }
 };
+// A block of one warp (or part of one).
+struct WarpSync {
+    unsigned mask;
+    __device__ __forceinline__ void operator()() const { __syncwarp(mask); }
+};
+
 struct NamedSync {
     unsigned id, nthreads;  // id 1..15; nthreads a multiple of 32
     __device__ __forceinline__ void operator()() const {
@@ -143,6 +158,20 @@ __device__ __forceinline__ void apply_twiddles(double2* vv, const double2* __res
     }
 }
 
+// The twiddles of radix pass S on one butterfly: vv[k1] *= w_L^{n2 k1}, L = M / E^S.
+template <class G, int S, bool INV>
+__device__ __forceinline__ void pass_twiddles(double2* vv, const double2* __restrict__ qtw, int n2) {
+    constexpr int R = G::radix(S), ST = G::stride(S);
+    if constexpr (G::TWM == TW_PASS) {
+        const double2* w = qtw + G::pass_offset(S) + n2;
+#pragma unroll
+        for (int k1 = 1; k1 < R; ++k1)
+            vv[k1] = INV ? cmulc(vv[k1], w[(k1 - 1) * ST]) : cmul(vv[k1], w[(k1 - 1) * ST]);
+    } else {
+        apply_twiddles<G, R, INV>(vv, qtw, (uint32_t)n2 << (G::LE * S));
+    }
+}
+
 // Forward (INV=false) or inverse radix pass S on the register array v (E values).
 // Forward: load (S > 0), DFT, twiddle w_L^{n2 k1}, store (S < P-1).
 // Inverse: load (S < P-1), conj twiddle, inverse DFT, store (S > 0).
@@ -181,9 +210,9 @@ __device__ __forceinline__ void radix_pass(double2 (&v)[G::E], double2* __restri
         }
         if constexpr (!INV) {
             Dft<R, false>::run(vv);
-            if constexpr (ST > 1) apply_twiddles<G, R, false>(vv, qtw, (uint32_t)n2 << (G::LE * S));
+            if constexpr (ST > 1) pass_twiddles<G, S, false>(vv, qtw, n2);
         } else {
-            if constexpr (ST > 1) apply_twiddles<G, R, true>(vv, qtw, (uint32_t)n2 << (G::LE * S));
+            if constexpr (ST > 1) pass_twiddles<G, S, true>(vv, qtw, n2);
             Dft<R, true>::run(vv);
         }
         if constexpr (STORE && !SYNC_BEFORE_STORE) {
@@ -247,6 +276,7 @@ struct SmallG : SmallGeom<LOG_M_T, LOG_E> {
 template <class G>
 __host__ __device__ constexpr uint32_t twiddle_table_len() {
     if (G::TWM == TW_QUARTER_S) return qpad_s_len((uint32_t)G::M >> 2);
+    if (G::TWM == TW_PASS) return (uint32_t)G::pass_offset(G::P - 1);
     return qpad_len((uint32_t)G::M >> (G::TWM == TW_FULL ? 0 : G::TWM == TW_HALF ? 1 : 2));
 }
 

@@ -26,6 +26,8 @@ std::vector<double2> padded_quarter_table(uint64_t L);
 double2 padded_quarter_slot(uint64_t L, uint64_t i);
 // The same quarter-wave table in the spread layout (entry r at qpad_s(r)).
 std::vector<double2> spread_quarter_table(uint64_t L);
+// The twiddles of an L-point FFT of 2^log_e values a thread, pass by pass (TW_PASS).
+std::vector<double2> pass_twiddle_table(int log_l, int log_e);
 
 struct LargeTest {
     uint64_t p = 0, N = 0, M = 0;

@@ -27,6 +27,12 @@ struct PerDeviceOnce {
     }
 };
 
+// Shared-memory carve-out of the whole-test kernels: all of it. The blocks of a launch are resident
+// for the whole test, so a carve-out that holds fewer of them than the registers would leaves tests
+// waiting for a full test's time; the default carve-out did so in some launches (1184 tests at
+// N = 512, eight an SM: 11.4 us a squaring by default, 6.4 with all of it).
+constexpr int kWholeTestCarveout = 100;
+
 enum : uint32_t {
     LLG_ST_OK = 0,
     LLG_ST_ROUNDOFF = 1,  // a round-off distance exceeded the abort threshold
@@ -45,11 +51,13 @@ struct SmallResult {
     uint32_t pad;
 };
 
-// Whether the whole-test FP64 kernel of length 2^log_n reads its twiddle table in the spread
-// layout (spread_quarter_table) rather than the padded one (padded_quarter_table).
-bool small_fp64_spread_table(int log_n);
-// FP64 whole-test kernel, N = 2^log_n with 5 <= log_n <= 13. digits: njobs * N int64 (may be null).
-cudaError_t launch_small_fp64(int log_n, const SmallJob* jobs, int njobs, const double2* qtw,
+// FP64 whole-test kernel, N = 2^log_n with 5 <= log_n <= 13, in the form with 2^log_e values a
+// thread that small_fp64_log_e gives for this many tests; qtw: the table of M = N / 2 points, in the
+// form's own pass order (pass_twiddle_table) or the spread quarter table (spread_quarter_table).
+// digits: njobs * N int64 (may be null).
+int small_fp64_log_e(int log_n, int njobs);
+bool small_fp64_pass_table(int log_e);
+cudaError_t launch_small_fp64(int log_n, int log_e, const SmallJob* jobs, int njobs, const double2* qtw,
                               int64_t* digits, SmallResult* results, float* errlog,
                               double abort_err, cudaStream_t st);
 

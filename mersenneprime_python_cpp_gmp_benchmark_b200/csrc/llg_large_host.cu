@@ -70,6 +70,23 @@ std::vector<double2> spread_quarter_table(uint64_t L) {
     return t;
 }
 
+std::vector<double2> pass_twiddle_table(int log_l, int log_e) {
+    const uint64_t L = 1ull << log_l, E = 1ull << log_e;
+    std::vector<double2> t;
+    const long double two_pi = 6.283185307179586476925286766559005768L;
+    // pass s: groups of len values in R strides of st; w_len^(n2 k1) = w_L^(n2 k1 L / len)
+    for (uint64_t len = L; len > E || (len > 1 && len == L); len /= E) {
+        const uint64_t st = len / E;
+        if (st <= 1) break;
+        for (uint64_t k1 = 1; k1 < E; ++k1)
+            for (uint64_t n2 = 0; n2 < st; ++n2) {
+                const long double ang = two_pi * (long double)((n2 * k1 * (L / len)) % L) / (long double)L;
+                t.push_back(make_double2((double)cosl(ang), -(double)sinl(ang)));
+            }
+    }
+    return t;
+}
+
 std::vector<double2> padded_quarter_table(uint64_t L) {
     const uint64_t n = qpad_len((uint32_t)(L / 4));
     std::vector<double2> t(n);

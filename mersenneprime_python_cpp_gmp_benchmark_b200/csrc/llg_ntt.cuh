@@ -193,13 +193,6 @@ __device__ __forceinline__ uint64_t twiddle(const uint64_t* __restrict__ t, uint
 #include "llg_fft.cuh"
 
 namespace llg {
-
-// Barrier of a block of one warp (or part of one).
-struct WarpSync {
-    unsigned mask;
-    __device__ __forceinline__ void operator()() const { __syncwarp(mask); }
-};
-
 namespace gl {
 
 // log2 of the values per thread of the NTT kernels: radix-8 passes. Against the radix-16 passes

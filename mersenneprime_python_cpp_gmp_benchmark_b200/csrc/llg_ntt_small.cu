@@ -201,6 +201,8 @@ static cudaError_t launch_small_ntt_t(const SmallJob* jobs, int njobs, const uin
     static PerDeviceOnce configured;
     if (!configured.done()) {
         cudaError_t e = cudaFuncSetAttribute(ll_small_ntt<LOG_N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(ll_small_ntt<LOG_N>, cudaFuncAttributePreferredSharedMemoryCarveout, kWholeTestCarveout);
         if (e != cudaSuccess) return e;
         configured.mark();
     }

@@ -7,8 +7,8 @@
 // single-block GPU loop of cuda/ll_ntt.cu:91-163, with a different transform:
 //
 //   * the N real weighted digits are packed as M = N/2 complex values u_m = y_2m + i y_2m+1 and
-//     transformed by an M-point complex FFT (radix-16 passes, radix-8 for M = 512, in-register
-//     DFTs, one shared-memory exchange per pass, no bit reversal);
+//     transformed by an M-point complex FFT (passes of radix 2 to 16 by the values a thread holds,
+//     in-register DFTs, one shared-memory exchange per pass, no bit reversal);
 //   * the real-FFT split and the pointwise square are one step on the pair (k, M-k):
 //       U'_k = [(3A - B)(A + B) - w^k (A - B)^2] / 4,  A = U_k, B = conj(U_{M-k}), w = e^{-2 pi i/M}
 //     which equals DFT_M(z_even + i z_odd) for the cyclic square z = y * y;
@@ -25,7 +25,9 @@
 // it at the next larger N.
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstdint>
+#include <type_traits>
 
 #include "llg_device.cuh"
 #include "llg_fft.cuh"
@@ -33,31 +35,69 @@
 
 namespace llg {
 
-// log2 of the complex values per thread for M = 2^log_m: 8 (radix-8 passes, twice the warps)
-// for M = 2^9, where that takes no more passes than 16 (8 x 8 x 8 against 16 x 16 x 2); 16 else
-__host__ __device__ constexpr int small_log_e(int log_m) { return log_m == 9 ? 3 : 4; }
-// twiddle-table layout: spread (qpad_s) from M = 2^10 up, where the radix-16 passes' strided
-// reads and the real-FFT split's digit-reversed reads conflict most in the qpad layout
-__host__ __device__ constexpr int small_tw_layout(int log_m) { return log_m >= 10 ? TW_QUARTER_S : TW_QUARTER; }
-template <int LOG_M>
-using SmallGeo = SmallG<LOG_M, small_log_e(LOG_M), small_tw_layout(LOG_M), true>;
+// twiddle-table layout: every pass's own twiddles (TW_PASS) where they fit beside the exchange
+// buffers of the resident blocks, i.e. below 16 values a thread; else (M = 2^12) the spread quarter
+// table with factored twiddles
+__host__ __device__ constexpr int small_tw_layout(int le) { return le >= 4 ? TW_QUARTER_S : TW_PASS; }
+// log2 of the complex values per thread. Fewer values spread a test over more warps (its squarings
+// are a serial chain, and a test alone on its SM otherwise runs at one or two warps' issue rate); more
+// values take fewer passes and exchanges. Measured, us a squaring (the choice first), against 16
+// values everywhere but N = 1024 (8 there) before:
+//   one test      N = 32 .57 (2 values), .65 (4); 64 .67, .77; 128 .77 (4), .88 (2); 256 1.07 (4),
+//                 1.54 (8); 512 1.31 (4), 1.67 (8); 1024 2.05 (8), 2.04 (4); 2048 2.81 (8), 3.38 (4);
+//                 4096 4.83 (8), 6.2 (16); 8192 8.6 (16), 9.2 (8)
+//        before   2.9, 4.6, 4.7, 4.9, 5.1, 3.3, 5.7, 6.2, 8.6
+//   1184 tests    N = 32 2.5 (4 values); 64 2.1; 128 2.7; 256 2.9 (8); 512 6.4 (8); 1024 14.9 (8);
+//                 2048 25.7 (8); 592 tests: 4096 17.0 (16), 17.4 (8)
+//        before   15.8, 11.2, 7.4, 10.1, 9.4, 16.9, 34.6, 17.0
+// Above one test per SM (small_fp64_log_e) the batch form runs.
+__host__ __device__ constexpr int small_log_e_alone(int log_m) {
+    return log_m <= 5 ? 1 : log_m <= 8 ? 2 : log_m <= 11 ? 3 : 4;
+}
+__host__ __device__ constexpr int small_log_e_batch(int log_m) { return log_m <= 6 ? 2 : log_m <= 10 ? 3 : 4; }
+// M = 2^LOG_M complex points, 2^LE complex values per thread
+template <int LOG_M, int LE>
+using SmallGeo = SmallG<LOG_M, LE, small_tw_layout(LE), true>;
 
-bool small_fp64_spread_table(int log_n) { return small_tw_layout(log_n - 1) == TW_QUARTER_S; }
-// blocks per SM the kernel is built for: 128 registers a thread at 16 values, ~85 at 8
-__host__ __device__ constexpr int small_min_blocks(int t, int le) {
-    return t < 32 ? 16 : (le >= 4 ? 512 : 768) / t > 16 ? 16 : (le >= 4 ? 512 : 768) / t;
+// blocks per SM the kernel is built for: 128 registers a thread (80 at 8 values a thread spilled,
+// and cost 10 to 20% at N = 1024 and 2048)
+__host__ __device__ constexpr int small_min_blocks(int t) { return t < 32 ? 16 : 512 / t > 16 ? 16 : 512 / t; }
+
+// Real-FFT split twiddle e^{-2 pi i k / M} from the TW_PASS table, whose first M / E entries are the
+// powers below M / E (k1 = 1 of the first pass): k folds to r <= M/8 (E = 8) or r < M/4, by the
+// quadrant (bits 13, 14: times (-i)^quad) and, past an eighth, by swapping cosine and sine
+// (bit 15). r = M/8 itself is w^{2 (M/16)}, entry M/16 of k1 = 2.
+template <int M, int E>
+__device__ __forceinline__ unsigned short split_code(int k) {
+    const int quad = k / (M / 4);
+    int r = k % (M / 4), swap = 0;
+    if (E == 8 && r > M / 8) {
+        r = M / 4 - r;
+        swap = 1;
+    }
+    if (E == 8 && r == M / 8) r = M / 8 + M / 16;
+    return (unsigned short)(r | (quad << 13) | (swap << 15));
+}
+__device__ __forceinline__ double2 split_twiddle(const double2* __restrict__ tw, unsigned code) {
+    const double2 w = tw[code & 0x1fffu];
+    const bool swap = (code & 0x8000u) != 0, odd = (code & 0x2000u) != 0;
+    // e^{-i(pi/2 - a)} = sin a - i cos a: (x, y) -> (-y, -x); times (-i): (x, y) -> (y, -x)
+    const double2 a = swap ? make_double2(-w.y, -w.x) : w;
+    const double2 b = odd ? make_double2(a.y, -a.x) : a;
+    return (code & 0x4000u) ? make_double2(-b.x, -b.y) : b;
 }
 
-template <int LOG_M>
-__global__ void __launch_bounds__(SmallGeo<LOG_M>::T, small_min_blocks(SmallGeo<LOG_M>::T, small_log_e(LOG_M)))
+template <int LOG_M, int LE>
+__global__ void __launch_bounds__(SmallGeo<LOG_M, LE>::T, small_min_blocks(SmallGeo<LOG_M, LE>::T))
     ll_small_fp64(const SmallJob* __restrict__ jobs, const double2* __restrict__ qtw_g,
                   int64_t* __restrict__ digits_out, SmallResult* __restrict__ results,
                   float* __restrict__ errlog, double abort_err) {
-    using G = SmallGeo<LOG_M>;
-    constexpr int M = G::M, N = G::N, E = G::E, T = G::T, W = G::W;
+    using G = SmallGeo<LOG_M, LE>;
+    constexpr int M = G::M, N = G::N, E = G::E, T = G::T, W = G::W, PL = LE;
+    constexpr int PAD = M + M / E;  // exchange slots: one of padding per E
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    double2* buf = reinterpret_cast<double2*>(smem_raw);          // exchange buffer, PAD slots
-    double2* qtw = buf + G::PAD;                                   // padded quarter-wave table
+    double2* buf = reinterpret_cast<double2*>(smem_raw);          // exchange buffer
+    double2* qtw = buf + PAD;                                   // padded quarter-wave table
     constexpr int QL = (int)twiddle_table_len<G>();
     double* wB = reinterpret_cast<double*>(qtw + QL);
     double* iwB = wB + E;
@@ -67,9 +107,11 @@ __global__ void __launch_bounds__(SmallGeo<LOG_M>::T, small_min_blocks(SmallGeo<
     // slot of the partner U_{M-k} of this thread's position t E + j, [j][t]: fixed for the whole
     // test, read in the real-FFT split instead of two digit reversals a value
     unsigned short* pslot = reinterpret_cast<unsigned short*>(serr + 2);  // E * T
+    // TW_PASS: the split's twiddle w^freq_rev of the NB positions, [h][t]: table slot and rotation
+    constexpr int NBK = E / G::RLAST;
+    unsigned short* kslot = pslot + E * T;  // NBK * T
 
     const int t = threadIdx.x;  // blockDim.x == T (a partial warp when T < 32)
-    constexpr bool active = true;
     unsigned long long t_start = 0;
     if (t == 0) asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t_start));
     const SmallJob job = jobs[blockIdx.x];
@@ -91,14 +133,18 @@ __global__ void __launch_bounds__(SmallGeo<LOG_M>::T, small_min_blocks(SmallGeo<
 #pragma unroll
     for (int j = 0; j < E; ++j) {
         const int kp = (M - freq_of_pos<G>(t * E + j)) & (M - 1);
-        pslot[j * T + t] = (unsigned short)phys(pos_of_freq<G>(kp));
+        pslot[j * T + t] = (unsigned short)physp<PL>(pos_of_freq<G>(kp));
+    }
+    if constexpr (G::TWM == TW_PASS) {
+#pragma unroll
+        for (int h = 0; h < NBK; ++h) kslot[h * T + t] = split_code<M, E>(freq_rev<G>(t * NBK + h));
     }
     __syncthreads();
 
     // per-thread weight halves for the even (e=0) and odd (e=1) digit of each u_m
     int sA0 = 0, sA1 = 0;
     double wA0 = 1, wA1 = 1, iwA0 = 1, iwA1 = 1;
-    if (active) {
+    {
         sA0 = (int)((uint64_t)(N - (int)(((uint64_t)(2 * t) * p) & (uint64_t)(N - 1))) & (uint64_t)(N - 1));
         sA1 = (int)((uint64_t)(N - (int)(((uint64_t)(2 * t + 1) * p) & (uint64_t)(N - 1))) & (uint64_t)(N - 1));
         wA0 = exp2((double)sA0 / (double)N);
@@ -137,30 +183,30 @@ __global__ void __launch_bounds__(SmallGeo<LOG_M>::T, small_min_blocks(SmallGeo<
     if (t == 0) v[0].x = 4.0;
 
     const int lane = t & 31, warp = t >> 5;
-    const int lastlane = (warp == W - 1) ? ((T - 1) & 31) : 31;
-    const unsigned wmask = (T >= 32) ? 0xffffffffu : ((1u << T) - 1u);
+    constexpr unsigned wmask = (T >= 32) ? 0xffffffffu : ((1u << (T & 31)) - 1u);
+    using Sync = typename std::conditional<(T > 32), CtaSync, WarpSync>::type;
+    Sync sync;
+    if constexpr (T <= 32) sync.mask = wmask;
     double maxerr = 0.0;
     uint64_t it = 0;
     uint32_t status = LLG_ST_OK;
     int x0s[E], x1s[E];
 
     for (;;) {
-        forward_from<G, 0>(v, buf, qtw, t);
+        forward_from<G, 0, Sync, 1, PL>(v, buf, qtw, t, sync);
         // pair (k, M-k): real-FFT split + square, result scaled by 4 (folded into iwB)
-        if (active) {
 #pragma unroll
-            for (int j = 0; j < E; ++j) {
-                const int x = phys(t * E + j);
-                buf[x] = v[j];
-            }
-        }
-        __syncthreads();
-        if (active) {
+        for (int j = 0; j < E; ++j) buf[physp<PL>(t * E + j)] = v[j];
+        sync();
+        {
             // w^k of position t E + j: one table value per j / RLAST, times w_RLAST^(j % RLAST)
             constexpr int RL = G::RLAST, NB = E / RL;
             double2 wk[NB];
 #pragma unroll
-            for (int h = 0; h < NB; ++h) wk[h] = twiddle_g<G>(qtw, (uint32_t)freq_rev<G>(t * NB + h), false);
+            for (int h = 0; h < NB; ++h) {
+                if constexpr (G::TWM == TW_PASS) wk[h] = split_twiddle(qtw, kslot[h * T + t]);
+                else wk[h] = twiddle_g<G>(qtw, (uint32_t)freq_rev<G>(t * NB + h), false);
+            }
 #pragma unroll
             for (int j = 0; j < E; ++j) {
                 const int x = pslot[j * T + t];
@@ -170,15 +216,48 @@ __global__ void __launch_bounds__(SmallGeo<LOG_M>::T, small_min_blocks(SmallGeo<
                 const double2 d2 = make_double2((d.x - d.y) * (d.x + d.y), 2.0 * d.x * d.y);
                 v[j] = csub(cmul(a3, s), cmul(wk[j / RL], rot_k<RL, false>(d2, j % RL)));
             }
-            // the first inverse pass stores only after a barrier (partners may still be reading)
-            inverse_from<G, G::P - 1>(v, buf, qtw, t);
         }
+        // the first inverse pass stores only after a barrier (partners may still be reading)
+        inverse_from<G, G::P - 1, true, Sync, 1, PL>(v, buf, qtw, t, sync);
 
         // unweight, round, error, local carry (even -> odd digit); the carry-out of column i goes
         // to thread t+1 (lane shuffle) or, at a warp boundary, through cbuf after the barrier
         double lerr = 0.0;
+        int bad;
         refresh_kinds();
-        if (active) {
+        if constexpr (W == 1) {
+            // one warp: the last thread's carry-outs go to thread 0 one column on, by shuffle too
+            double x0[E], x1[E], c[E];
+#pragma unroll
+            for (int i = 0; i < E; ++i) {
+                const uint32_t kd = kind(i);
+                const double iw = iwB[i];
+                const double a = v[i].x * (iwA0 * iw) * ((kd & 4u) ? 2.0 : 1.0);
+                const double b = v[i].y * (iwA1 * iw) * ((kd & 8u) ? 2.0 : 1.0);
+                long long la, lb;
+                const double ra = round_shift(a, la), rb = round_shift(b, lb);
+                lerr = fmax(lerr, fmax(fabs(a - ra), fabs(b - rb)));
+                double cy;
+                x0[i] = dsplit_e(ra, q + (int)(kd & 1u), cy);
+                x1[i] = dsplit_e(rb + cy, q + (int)((kd >> 1) & 1u), c[i]);
+                c[i] = __shfl_sync(wmask, c[i], (t + T - 1) & (T - 1));
+            }
+            const double wrap = c[E - 1];
+#pragma unroll
+            for (int i = E - 1; i > 0; --i) c[i] = t == 0 ? c[i - 1] : c[i];
+            c[0] = t == 0 ? wrap - 2.0 : c[0];  // the "- 2" of s^2 - 2
+#pragma unroll
+            for (int i = 0; i < E; ++i) {
+                double cy;
+                x0s[i] = d2i_exact(dsplit_e(x0[i] + c[i], q + (int)(kind(i) & 1u), cy));
+                x1s[i] = d2i_exact(x1[i] + cy);
+            }
+            if (errlog) {
+                atomicMax(&serr[it & 1], (unsigned long long)__double_as_longlong(lerr));
+                __syncwarp(wmask);
+            }
+            bad = __any_sync(wmask, lerr > abort_err);
+        } else {
 #pragma unroll
             for (int i = 0; i < E; ++i) {
                 const uint32_t kd = kind(i);
@@ -193,8 +272,8 @@ __global__ void __launch_bounds__(SmallGeo<LOG_M>::T, small_min_blocks(SmallGeo<
                 double x0 = dsplit_e(ra, b0, c);
                 const double x1 = dsplit_e(rb + c, b1, c);
                 const double cout = c;
-                if (lane == lastlane) cbuf[warp * E + i] = cout;
-                const double cin = __shfl_up_sync(wmask, cout, 1);
+                if (lane == 31) cbuf[warp * E + i] = cout;
+                const double cin = __shfl_up_sync(0xffffffffu, cout, 1);
                 if (lane != 0) {
                     x0 = dsplit_e(x0 + cin, b0, c);
                     x1s[i] = d2i_exact(x1 + c);
@@ -203,16 +282,16 @@ __global__ void __launch_bounds__(SmallGeo<LOG_M>::T, small_min_blocks(SmallGeo<
                 }
                 x0s[i] = d2i_exact(x0);
             }
+            if (errlog) atomicMax(&serr[it & 1], (unsigned long long)__double_as_longlong(lerr));
+            bad = __syncthreads_or(lerr > abort_err);
         }
         maxerr = fmax(maxerr, lerr);
-        if (errlog) atomicMax(&serr[it & 1], (unsigned long long)__double_as_longlong(lerr));
-        const int bad = __syncthreads_or(lerr > abort_err);
         if (errlog && t == 0) {
             errlog[it] = (float)__longlong_as_double((long long)serr[it & 1]);
             serr[(it + 1) & 1] = 0ull;
         }
         refresh_kinds();
-        if (active && lane == 0) {
+        if (W > 1 && lane == 0) {
 #pragma unroll
             for (int i = 0; i < E; ++i) {
                 double cin = (warp > 0) ? cbuf[(warp - 1) * E + i]
@@ -230,18 +309,16 @@ __global__ void __launch_bounds__(SmallGeo<LOG_M>::T, small_min_blocks(SmallGeo<
         }
         if (it >= iters) break;
         refresh_kinds();
-        if (active) {
 #pragma unroll
-            for (int i = 0; i < E; ++i) {
-                const uint32_t kd = kind(i);
-                const double w = wB[i];
-                v[i].x = i2d_shift(x0s[i]) * (wA0 * w) * ((kd & 4u) ? 0.5 : 1.0);
-                v[i].y = i2d_shift(x1s[i]) * (wA1 * w) * ((kd & 8u) ? 0.5 : 1.0);
-            }
+        for (int i = 0; i < E; ++i) {
+            const uint32_t kd = kind(i);
+            const double w = wB[i];
+            v[i].x = i2d_shift(x0s[i]) * (wA0 * w) * ((kd & 4u) ? 0.5 : 1.0);
+            v[i].y = i2d_shift(x1s[i]) * (wA1 * w) * ((kd & 8u) ? 0.5 : 1.0);
         }
     }
 
-    if (active && digits_out) {
+    if (digits_out) {
         int64_t* out = digits_out + (size_t)blockIdx.x * N;
 #pragma unroll
         for (int i = 0; i < E; ++i) {
@@ -365,47 +442,80 @@ cudaError_t launch_word(const SmallJob* jobs, int njobs, uint64_t* res, cudaStre
     return cudaGetLastError();
 }
 
-template <int LOG_M>
+// SM count of the current device (148 when it cannot be asked).
+static int device_sms() {
+    static std::atomic<int> sms[64];
+    const int d = PerDeviceOnce::current();
+    if (d < 0) return 148;
+    int n = sms[d].load();
+    if (n == 0) {
+        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, d) != cudaSuccess || n <= 0) n = 148;
+        sms[d].store(n);
+    }
+    return n;
+}
+
+template <int LOG_M, int LE>
 static size_t small_smem_bytes() {
-    using G = SmallGeo<LOG_M>;
-    size_t b = sizeof(double2) * G::PAD;
+    using G = SmallGeo<LOG_M, LE>;
+    size_t b = sizeof(double2) * (G::M + G::M / G::E);
     b += sizeof(double2) * twiddle_table_len<G>();
     b += 2 * sizeof(double) * G::E + sizeof(int) * (G::E + (G::E & 1 ? 1 : 0) + 2);
     b += sizeof(double) * G::W * G::E + 2 * sizeof(unsigned long long);
     b += sizeof(unsigned short) * G::E * G::T;  // partner slots of the real-FFT split
+    if (G::TWM == TW_PASS) b += sizeof(unsigned short) * (G::E / G::RLAST) * G::T;  // its twiddles
     return b;
 }
 
-template <int LOG_M>
-static cudaError_t launch_small_t(const SmallJob* jobs, int njobs, const double2* qtw,
-                                  int64_t* digits, SmallResult* results, float* errlog,
-                                  double abort_err, cudaStream_t st) {
-    using G = SmallGeo<LOG_M>;
-    const size_t smem = small_smem_bytes<LOG_M>();
+template <int LOG_M, int LE>
+static cudaError_t launch_small_le(const SmallJob* jobs, int njobs, const double2* qtw,
+                                   int64_t* digits, SmallResult* results, float* errlog,
+                                   double abort_err, cudaStream_t st) {
+    using G = SmallGeo<LOG_M, LE>;
+    const size_t smem = small_smem_bytes<LOG_M, LE>();
     static PerDeviceOnce configured;
     if (!configured.done()) {
-        cudaError_t e = cudaFuncSetAttribute(ll_small_fp64<LOG_M>,
+        cudaError_t e = cudaFuncSetAttribute(ll_small_fp64<LOG_M, LE>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(ll_small_fp64<LOG_M, LE>, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                     kWholeTestCarveout);
         if (e != cudaSuccess) return e;
         configured.mark();
     }
-    ll_small_fp64<LOG_M><<<njobs, G::T, smem, st>>>(jobs, qtw, digits, results, errlog, abort_err);
+    ll_small_fp64<LOG_M, LE><<<njobs, G::T, smem, st>>>(jobs, qtw, digits, results, errlog, abort_err);
     return cudaGetLastError();
 }
 
-cudaError_t launch_small_fp64(int log_n, const SmallJob* jobs, int njobs, const double2* qtw,
+int small_fp64_log_e(int log_n, int njobs) {
+    return njobs <= device_sms() ? small_log_e_alone(log_n - 1) : small_log_e_batch(log_n - 1);
+}
+bool small_fp64_pass_table(int log_e) { return small_tw_layout(log_e) == TW_PASS; }
+
+template <int LOG_M>
+static cudaError_t launch_small_t(int log_e, const SmallJob* jobs, int njobs, const double2* qtw,
+                                  int64_t* digits, SmallResult* results, float* errlog,
+                                  double abort_err, cudaStream_t st) {
+    if (log_e == small_log_e_alone(LOG_M))
+        return launch_small_le<LOG_M, small_log_e_alone(LOG_M)>(jobs, njobs, qtw, digits, results, errlog, abort_err, st);
+    if (log_e == small_log_e_batch(LOG_M))
+        return launch_small_le<LOG_M, small_log_e_batch(LOG_M)>(jobs, njobs, qtw, digits, results, errlog, abort_err, st);
+    return cudaErrorInvalidValue;
+}
+
+cudaError_t launch_small_fp64(int log_n, int log_e, const SmallJob* jobs, int njobs, const double2* qtw,
                               int64_t* digits, SmallResult* results, float* errlog,
                               double abort_err, cudaStream_t st) {
     switch (log_n - 1) {
-        case 4: return launch_small_t<4>(jobs, njobs, qtw, digits, results, errlog, abort_err, st);
-        case 5: return launch_small_t<5>(jobs, njobs, qtw, digits, results, errlog, abort_err, st);
-        case 6: return launch_small_t<6>(jobs, njobs, qtw, digits, results, errlog, abort_err, st);
-        case 7: return launch_small_t<7>(jobs, njobs, qtw, digits, results, errlog, abort_err, st);
-        case 8: return launch_small_t<8>(jobs, njobs, qtw, digits, results, errlog, abort_err, st);
-        case 9: return launch_small_t<9>(jobs, njobs, qtw, digits, results, errlog, abort_err, st);
-        case 10: return launch_small_t<10>(jobs, njobs, qtw, digits, results, errlog, abort_err, st);
-        case 11: return launch_small_t<11>(jobs, njobs, qtw, digits, results, errlog, abort_err, st);
-        case 12: return launch_small_t<12>(jobs, njobs, qtw, digits, results, errlog, abort_err, st);
+        case 4: return launch_small_t<4>(log_e, jobs, njobs, qtw, digits, results, errlog, abort_err, st);
+        case 5: return launch_small_t<5>(log_e, jobs, njobs, qtw, digits, results, errlog, abort_err, st);
+        case 6: return launch_small_t<6>(log_e, jobs, njobs, qtw, digits, results, errlog, abort_err, st);
+        case 7: return launch_small_t<7>(log_e, jobs, njobs, qtw, digits, results, errlog, abort_err, st);
+        case 8: return launch_small_t<8>(log_e, jobs, njobs, qtw, digits, results, errlog, abort_err, st);
+        case 9: return launch_small_t<9>(log_e, jobs, njobs, qtw, digits, results, errlog, abort_err, st);
+        case 10: return launch_small_t<10>(log_e, jobs, njobs, qtw, digits, results, errlog, abort_err, st);
+        case 11: return launch_small_t<11>(log_e, jobs, njobs, qtw, digits, results, errlog, abort_err, st);
+        case 12: return launch_small_t<12>(log_e, jobs, njobs, qtw, digits, results, errlog, abort_err, st);
         default: return cudaErrorInvalidValue;
     }
 }
