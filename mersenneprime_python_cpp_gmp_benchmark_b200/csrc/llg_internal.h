@@ -27,6 +27,19 @@ struct PerDeviceOnce {
     }
 };
 
+// SM count of the current device (148 when it cannot be asked).
+inline int device_sms() {
+    static std::atomic<int> sms[64];
+    const int d = PerDeviceOnce::current();
+    if (d < 0) return 148;
+    int n = sms[d].load();
+    if (n == 0) {
+        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, d) != cudaSuccess || n <= 0) n = 148;
+        sms[d].store(n);
+    }
+    return n;
+}
+
 // Shared-memory carve-out of the whole-test kernels: all of it. The blocks of a launch are resident
 // for the whole test, so a carve-out that holds fewer of them than the registers would leaves tests
 // waiting for a full test's time; the default carve-out did so in some launches (1184 tests at
@@ -115,19 +128,18 @@ constexpr bool large_rows_supported(int log_c, int g) {
 __host__ __device__
 #endif
 constexpr int large_rows_per_block(int log_c) { return log_c >= 11 ? 2 : 4; }
-constexpr int kLargeLogE = 4;         // log2 of the complex values per thread in the column pass
 constexpr unsigned long long kSpinLimit = 1ull << 22;  // x ~64 ns sleeps: ~0.3 s, then give up + flag
 // log2 of the complex values per thread in the row pass of g rows of 2^log_c complex: 8 values
-// (radix-8 passes, 64 registers a thread, two or more blocks per SM) for rows of up to 2^9, 16
-// (radix-16 passes, 128 registers) for longer rows
+// (radix-8 passes, two or more blocks per SM) for rows of up to 2^9, 16 (radix-16 passes) for longer
 #ifdef __CUDACC__
 __host__ __device__
 #endif
 constexpr int large_row_log_e(int log_c, int g) { return (void)g, log_c <= 9 ? 3 : 4; }
 
 struct LargeCtl {
+    unsigned long long tickets;      // FP64 row-pass tickets taken since the start
     unsigned int epoch;              // squarings whose column pass has finished; +1 per column pass
-    unsigned int ticket[2];          // row-pass block tickets, alternating by epoch parity
+    unsigned int ticket[2];          // NTT row-pass block tickets, alternating by epoch parity
     unsigned int timeout;            // set when a bounded wait gave up (the result is then invalid)
     unsigned long long err_max;      // bits of the max round-off over the run (double, >= 0)
     unsigned long long err_since;    // same, since the host last cleared it
@@ -153,6 +165,14 @@ __device__ __forceinline__ void wait_flag(unsigned int* f, unsigned int target, 
 }
 #endif
 
+// One column's carry-outs of a row tile's last row, published and read as one 16-byte access: the
+// tag says whose they are, so a reader needs no separate flag (and the writer no fence).
+struct __align__(16) LargeCarry {
+    double c1;      // hop-1 carry-out (an integer)
+    int c2;         // hop-2 carry-out (an integer of a few units)
+    unsigned tag;   // epoch + 1 of the squaring they belong to
+};
+
 struct LargeArgs {
     double2* V;               // state: element (row a, column slot pos) at pos * R + a
     const double2* qtwC;      // full padded twiddle table of the C-point row FFT
@@ -168,16 +188,16 @@ struct LargeArgs {
     const double* wB;         // [C] 2^(sB/N)
     const double* iwB;        // [C] 2^(-sB/N) / (4M)
     const int* sB;            // [C] (-2Rb p) mod N
-    double* carry;            // [nblocks + 1][C] hop-1 carry-outs of a tile's last row (integers):
-                              // slot 0 the wrap-around job's (row R-1, one column on), k + 1 tile k's
-    double* carry2;           // [nblocks + 1][C] hop-2 carry-outs (integers of a few units)
+    LargeCarry* carry;        // [nblocks + 1][C] carry-outs of a tile's last row: slot 0 the
+                              // wrap-around job's (row R-1, one column on), k + 1 tile k's
     LargeCtl* ctl;
-    unsigned int* flags;      // [nblocks + 1] epoch + 1 once the job of that slot published its carries
+    unsigned int* wrap_read;  // epoch + 1 once the wrap-around job has read its rows
     unsigned long long spin_limit;  // bound of every wait on a flag (x ~64 ns sleeps)
     int* digits;              // N int32, natural order (INIT input; dump / FINAL output)
     float* errlog;            // per-epoch max round-off ring (may be null)
     int errlog_len;
     int dump;                 // ITER: also write the digits
+    int pdl_late;             // where the passes let the next one launch: at their end, or at their start
     int tw_shift;
     int C, R, nblocks;
     int q, rem;               // p / N, p % N

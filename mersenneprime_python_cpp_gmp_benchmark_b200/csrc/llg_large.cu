@@ -32,9 +32,9 @@
 // digit and split again (hop 2), and the small remainder of that split goes into the next row's
 // first digit (hop 3). That keeps every digit within a few units of balanced and makes carry-outs
 // independent of carry-ins. Inside a tile the carries pass between lanes; between tiles, tile k
-// publishes its last row's hop-1 and hop-2 carry-outs and a flag, and tile k+1 reads them after a
-// bounded wait. Tiles take tickets in launch order, so the tile waited on is always resident or
-// finished. The wrap-around carry into row 0 (2^p == 1) comes from row R-1: the first ticket is a
+// publishes its last row's hop-1 and hop-2 carry-outs with a tag, 16 bytes a column, and tile k+1
+// reads them, waiting (bounded) for the tag. Tiles
+// take tickets in launch order, so the tile waited on is always resident or finished. The wrap-around carry into row 0 (2^p == 1) comes from row R-1: the first ticket is a
 // separate job that runs the last tile's rows through the inverse FFT and hops 1-2 and publishes
 // their carry-outs (one column on) in the slot tile 0 reads; the last tile waits (bounded) for
 // that job before overwriting those rows.
@@ -64,9 +64,11 @@ __device__ __forceinline__ double2 twiddle_M(const LargeArgs& A, uint32_t x, boo
 __host__ __device__ constexpr int large_row_threads(int log_c, int g) {
     return g * (1 << log_c) / (1 << large_row_log_e(log_c, g));
 }
-// blocks per SM the row kernel is built for: 128 registers a thread at 16 values, 64 at 8
-__host__ __device__ constexpr int large_row_min_blocks(int log_c, int g) {
-    const int b = (large_row_log_e(log_c, g) >= 4 ? 512 : 1024) / large_row_threads(log_c, g);
+// blocks per SM the row kernel is built for: 128 registers a thread (64 at 8 values a thread spilled
+// 200 to 350 bytes: N = 2^20 34 against 19 us a squaring). dense: a fifth block of the 128-thread
+// tiles at 102 registers, for tile counts that then fit one wave (launch_large_row).
+__host__ __device__ constexpr int large_row_min_blocks(int log_c, int g, bool dense = false) {
+    const int b = (dense ? 640 : 512) / large_row_threads(log_c, g);
     return b > 16 ? 16 : (b < 1 ? 1 : b);
 }
 // exchange-buffer slots of a tile: G rows of C + C/E padded slots
@@ -74,8 +76,38 @@ __host__ __device__ constexpr int large_row_slots(int log_c, int g) {
     return g * ((1 << log_c) + ((1 << log_c) >> large_row_log_e(log_c, g)));
 }
 
-template <int LOG_C, int G, int MODE>
-__global__ void __launch_bounds__(large_row_threads(LOG_C, G), large_row_min_blocks(LOG_C, G))
+// Carry slots move as single 16-byte relaxed accesses at device scope.
+__device__ __forceinline__ void st_carry(LargeCarry* p, double c1, int c2, unsigned tag) {
+    const unsigned long long lo = (unsigned long long)__double_as_longlong(c1);
+    const unsigned long long hi = ((unsigned long long)tag << 32) | (unsigned)c2;
+    asm volatile("{\n\t.reg .b128 v;\n\tmov.b128 v, {%1, %2};\n\tst.relaxed.gpu.global.b128 [%0], v;\n\t}" ::"l"(p), "l"(lo), "l"(hi) : "memory");
+}
+__device__ __forceinline__ LargeCarry ld_carry(const LargeCarry* p) {
+    unsigned long long lo, hi;
+    asm volatile("{\n\t.reg .b128 v;\n\tld.relaxed.gpu.global.b128 v, [%2];\n\tmov.b128 {%0, %1}, v;\n\t}" : "=l"(lo), "=l"(hi) : "l"(p) : "memory");
+    LargeCarry r;
+    r.c1 = __longlong_as_double((long long)lo);
+    r.c2 = (int)(unsigned)hi;
+    r.tag = (unsigned)(hi >> 32);
+    return r;
+}
+// Bounded wait until the slot holds the carries tagged `tag`. On giving up (or once another wait
+// has) the run's result is reported invalid by ctl->timeout, so a kernel never spins forever.
+__device__ __noinline__ LargeCarry wait_carry(const LargeCarry* p, unsigned tag, LargeCtl* ctl, unsigned long long limit) {
+    LargeCarry c = ld_carry(p);
+    for (unsigned long long spins = 0; c.tag != tag; ++spins) {
+        if (spins > limit || ((spins & 255) == 255 && *reinterpret_cast<volatile unsigned*>(&ctl->timeout))) {
+            atomicExch(&ctl->timeout, 1u);
+            break;
+        }
+        __nanosleep(spins < 16 ? 20 : 64);
+        c = ld_carry(p);
+    }
+    return c;
+}
+
+template <int LOG_C, int G, int MODE, bool DENSE>
+__global__ void __launch_bounds__(large_row_threads(LOG_C, G), large_row_min_blocks(LOG_C, G, DENSE))
     large_row(const LargeArgs A) {
     constexpr int LE = large_row_log_e(LOG_C, G);
     using GC = SmallG<LOG_C, LE, TW_FULL, true>;  // full twiddle table, factored twiddles
@@ -98,37 +130,40 @@ __global__ void __launch_bounds__(large_row_threads(LOG_C, G), large_row_min_blo
     const int N = A.N, R = A.R;
     const CtaSync sync;
 
-    // The next pass may launch once every block of this one has started (its blocks then take
-    // the SMs this pass's last wave leaves idle). This pass's own constant tables are requested
-    // (asynchronous copies, completed before the barrier that follows the tile loads) before it
-    // waits for the previous pass to complete; nothing it reads from the state, the control block
-    // or the carry slots is touched before that wait.
-    pdl_launch_dependents();
+    // The pass's constant tables are requested (asynchronous copies, completed before the barrier that
+    // follows the tile loads) and its ticket is taken before it waits for the previous pass to
+    // complete; nothing it reads from the state or the carry slots is touched before that wait.
     for (int k = t; k < QL; k += T) cp_async<16>(qtw + k, A.qtwC + k);
     for (int k = t; k < C; k += T) {
         cp_async<8>(swB + k, A.wB + k);
         if (MODE != LARGE_INIT) cp_async<8>(siwB + k, A.iwB + k);
         cp_async<4>(ssB + k, A.sB + k);
     }
-    pdl_wait_previous();
-
     if (t == 0) {
-        const unsigned ep = *reinterpret_cast<volatile unsigned*>(&A.ctl->epoch);
-        s_epoch = ep;
         if (MODE == LARGE_INIT) {
             s_job = blockIdx.x;
+            s_epoch = 0;
         } else {
-            // tickets in launch order: ticket 0 is the wrap-around job, ticket k tile k - 1
-            const int tk = (int)atomicAdd(&A.ctl->ticket[ep & 1], 1u);
-            if (tk == A.nblocks) {
-                // every block of this launch holds its ticket: both counters can be reset
-                A.ctl->ticket[(ep + 1) & 1] = 0u;
-                A.ctl->ticket[ep & 1] = 0u;
-            }
-            s_job = tk - 1;
+            // tickets in launch order, nblocks + 1 a pass from epoch 1 on: the pass's first ticket is the
+            // wrap-around job, the (k+1)-th after it tile k. The row pass before this one has taken
+            // all of its tickets: its blocks take theirs before they let the column pass launch,
+            // whose blocks let this pass launch.
+            const unsigned long long tk = atomicAdd(&A.ctl->tickets, 1ull), per = (unsigned)A.nblocks + 1u;
+            const unsigned long long pass = tk / per;
+            const int idx = (int)(tk - pass * per);
+            s_epoch = (unsigned)pass + 1u;
+            s_job = idx - 1;
+            // FINAL does not end the squaring: its pass's tickets are handed out again
+            if (MODE == LARGE_FINAL && idx == A.nblocks) A.ctl->tickets = pass * per;
         }
         s_err = 0ull;
+        // the next pass may launch now that this block holds its ticket
+        if (!A.pdl_late) {
+            asm volatile("" ::"r"(s_job) : "memory");
+            pdl_launch_dependents();
+        }
     }
+    pdl_wait_previous();
     __syncthreads();
     const int job = s_job;  // -1: the wrap-around job (rows R-G .. R-1), else the tile
     const unsigned ep = s_epoch;
@@ -180,7 +215,8 @@ __global__ void __launch_bounds__(large_row_threads(LOG_C, G), large_row_min_blo
         //      from inside the tile (the carry-out of the lane above); hop 3 for rows 2 .. G-1 (the
         //      hop-2 carry-out of the row above, also known inside the tile). Row G-1 publishes its
         //      hop-1 and hop-2 carry-outs for the next tile (the wrap job: one column on). ----
-        const int slot = job + 1;
+        if (wrap_job && t == 0) *reinterpret_cast<volatile unsigned*>(A.wrap_read) = ep + 1u;  // its rows are read
+        LargeCarry* pub = A.carry + (size_t)(job + 1) * C;
         const double ia0 = __ldg(A.iwA + 2 * a), ia1 = __ldg(A.iwA + 2 * a + 1);
         double lerr = 0.0;
 #pragma unroll
@@ -206,30 +242,25 @@ __global__ void __launch_bounds__(large_row_threads(LOG_C, G), large_row_min_blo
             const double cin2 = __shfl_up_sync(FULL, c2, 1, G);
             if (ra > 1) x0 += cin2;
             if (ra == G - 1) {
-                const int col = wrap_job ? ((b + 1) & (C - 1)) : b;  // row R-1, column b feeds row 0, column b+1
-                A.carry[(size_t)slot * C + col] = c1;
-                A.carry2[(size_t)slot * C + col] = c2;
+                // row R-1, column b feeds row 0, column b+1
+                st_carry(pub + (wrap_job ? ((b + 1) & (C - 1)) : b), c1, (int)c2, ep + 1u);
             }
             v[i] = make_double2(x0, x1);
         }
+        if (wrap_job) return;
         // the tile's round-off max: one shared atomic per warp
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) lerr = fmax(lerr, __shfl_xor_sync(FULL, lerr, o));
         if ((t & 31) == 0) atomicMax(&s_err, (unsigned long long)__double_as_longlong(lerr));
-        if (ra == G - 1) __threadfence();  // each publisher orders its carry stores before the flag
-        __syncthreads();
+        __syncthreads();  // every thread has left the inverse FFT's exchange buffer
         if (t == 0) {
-            *reinterpret_cast<volatile unsigned*>(&A.flags[slot]) = ep + 1u;
-            if (!wrap_job) {
-                const unsigned long long eb = s_err;
-                atomicMax(&A.ctl->err_max, eb);
-                atomicMax(&A.ctl->err_since, eb);
-                if (A.errlog)
-                    atomicMax(reinterpret_cast<unsigned int*>(A.errlog + (ep % (unsigned)A.errlog_len)),
-                              __float_as_uint((float)__longlong_as_double((long long)eb)));
-            }
+            const unsigned long long eb = s_err;
+            atomicMax(&A.ctl->err_max, eb);
+            atomicMax(&A.ctl->err_since, eb);
+            if (A.errlog)
+                atomicMax(reinterpret_cast<unsigned int*>(A.errlog + (ep % (unsigned)A.errlog_len)),
+                          __float_as_uint((float)__longlong_as_double((long long)eb)));
         }
-        if (wrap_job) return;
         // ---- the tile's first row: hops 2 and 3 from the previous tile's last row (or the wrap);
         //      its hop-2 carry-outs are hop 3 of the second row. The row passes through the
         //      exchange buffer (free until the forward FFT's first stores), so that every thread
@@ -240,25 +271,26 @@ __global__ void __launch_bounds__(large_row_threads(LOG_C, G), large_row_min_blo
 #pragma unroll
             for (int i = 0; i < E; ++i) row0[tr + TR * i] = v[i];
         }
-        if (t == 0) wait_flag(&A.flags[job], ep + 1u, A.ctl, A.spin_limit);
-        __syncthreads();
         {
             const int a0 = job * G;
             const int s0a = __ldg(A.sA + 2 * a0), s1a = __ldg(A.sA + 2 * a0 + 1);
-            const double* cprev = A.carry + (size_t)job * C;
-            const double* c2prev = A.carry2 + (size_t)job * C;
             static_assert(C % T == 0, "whole columns per thread");
+            LargeCarry in[C / T];
+#pragma unroll
+            for (int k = 0; k < C / T; ++k) in[k] = ld_carry(A.carry + (size_t)job * C + t + T * k);
+            __syncthreads();
 #pragma unroll
             for (int k = 0; k < C / T; ++k) {
                 const int b = t + T * k;
                 const uint32_t kd = kind_at(s0a, s1a, b);
-                double cin = __ldcg(cprev + b);
+                if (in[k].tag != ep + 1u) in[k] = wait_carry(A.carry + (size_t)job * C + b, ep + 1u, A.ctl, A.spin_limit);
+                double cin = in[k].c1;
                 if (job == 0 && b == 0) cin -= 2.0;  // the "- 2" of s^2 - 2 (digit 0)
                 const double2 x = row0[b];
                 double c, c2;
                 const double x0 = dsplit_e(x.x + cin, A.q + (int)(kd & 1u), c);
                 const double x1 = dsplit_e(x.y + c, A.q + (int)((kd >> 1) & 1u), c2);
-                row0[b] = make_double2(x0 + __ldcg(c2prev + b), x1);
+                row0[b] = make_double2(x0 + (double)in[k].c2, x1);
                 hop3[b] = c2;
             }
         }
@@ -297,9 +329,10 @@ __global__ void __launch_bounds__(large_row_threads(LOG_C, G), large_row_min_blo
     forward_from<GC, 1, CtaSync, G, LE>(v, buf, qtw, tr, sync);
     if (MODE == LARGE_ITER && job == A.nblocks - 1) {
         // rows R-G .. R-1 are the wrap job's input: wait (bounded) until it has read them
-        if (t == 0) wait_flag(&A.flags[0], ep + 1u, A.ctl, A.spin_limit);
+        if (t == 0) wait_flag(A.wrap_read, ep + 1u, A.ctl, A.spin_limit);
         __syncthreads();
     }
+    if (A.pdl_late) pdl_launch_dependents();
     // the store addresses equal the load addresses; formed again here from an opaque base, so the
     // compiler does not keep sixteen 64-bit addresses live across the whole pass
     double2* vp = A.V + (size_t)(tr * E) * R + a;
@@ -311,15 +344,32 @@ __global__ void __launch_bounds__(large_row_threads(LOG_C, G), large_row_min_blo
 // Column pass: one block owns the column pair (c, C-c), one half of its threads per column; the
 // real-FFT split reads the partner column's spectrum from the other half's exchange buffer.
 // Block 0 holds column 0 and block C/2 column C/2, each of which pairs with itself.
-template <int LOG_R>
-__global__ void __launch_bounds__(2 * (1 << LOG_R) / (1 << kLargeLogE), (LOG_R <= 11 ? 2 : 1)) large_col(const LargeArgs A) {
+// log2 of the complex values per thread of the column pass: 8 up to R = 2^10, where a pass has few
+// blocks and twice the warps finish them sooner (R = 512 at N = 2^19: 14.9 us a squaring against 16.1
+// with 16); 16 above (R = 2^12 at 2^22: 72 against 80)
+__host__ __device__ constexpr int large_col_log_e(int log_r) { return log_r <= 10 ? 3 : 4; }
+
+template <int LOG_R, int LE>
+struct LargeColGeom {
     // quarter twiddle table in the spread layout (entry r at qpad_s(r)): the strided twiddle reads
     // of the radix passes spread over more bank groups than with qpad
-    using GR = SmallG<LOG_R, kLargeLogE, TW_QUARTER_S, true>;
-    constexpr int R = GR::M, TC = GR::T, E = GR::E;
+    using GR = SmallG<LOG_R, LE, TW_QUARTER_S, true>;
+    static constexpr int R = GR::M, TC = GR::T, E = GR::E;
+    static constexpr int PAD = R + R / (E < 16 ? E : 16);  // exchange slots of a column
+    static constexpr int PL = LE < 4 ? LE : 4;
+    static constexpr int T = 2 * TC;
+    // blocks per SM it is built for
+    static constexpr int MINB = LE >= 4 ? (LOG_R <= 11 ? 2 : 1) : (512 / T > 8 ? 8 : 512 / T < 1 ? 1 : 512 / T);
+    static size_t smem() { return sizeof(double2) * (2 * PAD + qpad_s_len(R / 4) + 2 * E); }
+};
+template <int LOG_R, int LE>
+__global__ void __launch_bounds__(LargeColGeom<LOG_R, LE>::T, LargeColGeom<LOG_R, LE>::MINB) large_col(const LargeArgs A) {
+    using CG = LargeColGeom<LOG_R, LE>;
+    using GR = typename CG::GR;
+    constexpr int R = CG::R, TC = CG::TC, E = CG::E, PAD = CG::PAD, PL = CG::PL;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     double2* bufs = reinterpret_cast<double2*>(smem_raw);  // 2 exchange buffers of PAD slots
-    double2* qtw = bufs + 2 * GR::PAD;                       // padded quarter table (R-point)
+    double2* qtw = bufs + 2 * PAD;                       // padded quarter table (R-point)
     constexpr int QL = (int)qpad_s_len(R / 4);
     const int t = threadIdx.x, half = t / TC, tc = t % TC;
     const int C = A.C;
@@ -328,15 +378,14 @@ __global__ void __launch_bounds__(2 * (1 << LOG_R) / (1 << kLargeLogE), (LOG_R <
     const bool self = (c1 == c2);
     const bool active = !(self && half == 1);
     const int c = half ? c2 : c1;
-    double2* buf = bufs + half * GR::PAD;
-    const double2* pbuf = self ? buf : bufs + (1 - half) * GR::PAD;  // partner column
+    double2* buf = bufs + half * PAD;
+    const double2* pbuf = self ? buf : bufs + (1 - half) * PAD;  // partner column
     // each column's FFT exchanges wait only on that column's warps (named barrier 1 + half)
     using ColSync = typename std::conditional<(TC >= 32), NamedSync, CtaSync>::type;
     ColSync gsync;
     if constexpr (TC >= 32) gsync = NamedSync{1u + (unsigned)half, (unsigned)TC};
-    // as in the row pass: the next pass may launch once every block has started; the constant
-    // tables are read before waiting for the previous pass
-    pdl_launch_dependents();
+    // as in the row pass: the constant tables are read before waiting for the previous pass
+    if (!A.pdl_late) pdl_launch_dependents();
     for (int k = t; k < QL; k += 2 * TC) qtw[k] = A.qtwR[k];
     double2* col = A.V + (size_t)__ldg(A.pos_of_c + c) * R;
     // four-step twiddle w_M^{a c} for a = tc + TC i, factored as w_M^{c tc} * w_M^{c TC i}: one
@@ -351,9 +400,9 @@ __global__ void __launch_bounds__(2 * (1 << LOG_R) / (1 << kLargeLogE), (LOG_R <
     __syncthreads();
 #pragma unroll
     for (int i = 0; i < E; ++i) v[i] = cmul(v[i], cmul(q, ptab[i]));
-    forward_from<GR, 0>(v, buf, qtw, tc, gsync);
+    forward_from<GR, 0, ColSync, 1, PL>(v, buf, qtw, tc, gsync);
 #pragma unroll
-    for (int j = 0; j < E; ++j) buf[phys(tc * E + j)] = v[j];
+    for (int j = 0; j < E; ++j) buf[physp<PL>(tc * E + j)] = v[j];
     __syncthreads();
     // w_M^{c + C d} for the column frequency d of position tc E + j: w_M^c times one table value
     // w_R^{freq_rev} per j / RLAST, times the exact rotation w_RLAST^(j % RLAST)
@@ -366,7 +415,7 @@ __global__ void __launch_bounds__(2 * (1 << LOG_R) / (1 << kLargeLogE), (LOG_R <
     for (int j = 0; j < E; ++j) {
         const int d = freq_of_pos<GR>(tc * E + j);
         const int dp = (c == 0) ? ((R - d) & (R - 1)) : (R - 1 - d);
-        const int xp = phys(pos_of_freq<GR>(dp));
+        const int xp = physp<PL>(pos_of_freq<GR>(dp));
         const double2 Av = v[j], Bc = conj2(pbuf[xp]);  // conj(U_{M-k})
         const double2 s = cadd(Av, Bc), dd = csub(Av, Bc);
         const double2 a3 = make_double2(3.0 * Av.x - Bc.x, 3.0 * Av.y - Bc.y);
@@ -374,7 +423,8 @@ __global__ void __launch_bounds__(2 * (1 << LOG_R) / (1 << kLargeLogE), (LOG_R <
         v[j] = csub(cmul(a3, s), cmul(wk[j / RL], rot_k<RL, false>(d2, j % RL)));
     }
     __syncthreads();  // partner reads done before either column overwrites its buffer
-    inverse_from<GR, GR::P - 1, false>(v, buf, qtw, tc, gsync);
+    inverse_from<GR, GR::P - 1, false, ColSync, 1, PL>(v, buf, qtw, tc, gsync);
+    if (A.pdl_late) pdl_launch_dependents();
     if (active) {
         const double2 q2 = twiddle_M(A, (uint32_t)c * (uint32_t)tc, false);  // recomputed: frees registers
 #pragma unroll
@@ -406,19 +456,22 @@ __device__ __forceinline__ double2 pair_term_r(double2 acc, double2 a, double2 b
     return make_double2(fma(-dy, w.y, fma(sx, w.x, acc.x)), fma(dx, w.y, fma(sy, w.x, acc.y)));
 }
 
-// Column pass at the non-power-of-two column lengths R = R0 L (R0 = 3 or 5, L = 2^LOG_L, 16 values
+// Column pass at the non-power-of-two column lengths R = R0 L (R0 = 3 or 5, L = 2^LOG_L, 8 values
 // per thread), for the {3, 5} x 2^k transform lengths of the reference (lucaslehmer.cpp:244-254).
 // One block owns the column pair (c, C-c) as in large_col; each column is split as R0 x L by
 // decimation in frequency (a = n + L r, d = R0 k' + k0):
 //   U[R0 k' + k0] = sum_n w_L^{n k'} w_R^{n k0} sum_r u[n + L r] w_R0^{r k0}
 // the radix-R0 step across the column's R0 segments, the twiddle w_R^{n k0}, R0 L-point FFTs
-// (one segment of L/16 threads each, a named barrier per segment), the real-FFT split and square
+// (one segment of L/8 threads each, a named barrier per segment), the real-FFT split and square
 // over the pair, and back. Thread (half, seg, tl) holds u[seg L + tl + TL i] of its column.
+constexpr int kMixedLogE = 3;
 template <int R0, int LOG_L>
-__global__ void __launch_bounds__(2 * R0 * (1 << LOG_L) / (1 << kLargeLogE), (2 * R0 * (1 << LOG_L) / (1 << kLargeLogE) <= 256 ? 2 : 1))
+__host__ __device__ constexpr int col_mixed_threads() { return 2 * R0 * (1 << LOG_L) / (1 << kMixedLogE); }
+template <int R0, int LOG_L>
+__global__ void __launch_bounds__(col_mixed_threads<R0, LOG_L>(), 1)
     large_col_mixed(const LargeArgs A) {
-    using GL = SmallG<LOG_L, kLargeLogE, TW_QUARTER, true>;
-    constexpr int L = GL::M, TL = GL::T, E = GL::E, R = R0 * L, TC = R0 * TL, PADL = GL::PAD;
+    using GL = SmallG<LOG_L, kMixedLogE, TW_QUARTER, true>;
+    constexpr int L = GL::M, TL = GL::T, E = GL::E, R = R0 * L, TC = R0 * TL, PADL = L + L / E, PL = kMixedLogE;
     constexpr int QLL = (int)qpad_len(L / 4), QLR = (int)qpad_len(R / 4);
     static_assert(TL % 32 == 0 && 2 * TC <= 1024, "whole warps per segment");
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -441,7 +494,7 @@ __global__ void __launch_bounds__(2 * R0 * (1 << LOG_L) / (1 << kLargeLogE), (2 
     // barriers: 1 + half for the column's threads, 3 + half R0 + seg for one segment's
     const NamedSync hsync{1u + (unsigned)half, (unsigned)TC};
     const NamedSync ssync{3u + (unsigned)(half * R0 + seg), (unsigned)TL};
-    pdl_launch_dependents();  // as in large_col: constant tables before the wait
+    if (!A.pdl_late) pdl_launch_dependents();  // as in large_col: constant tables before the wait
     for (int k = t; k < QLL; k += 2 * TC) qtwL[k] = A.qtwL[k];
     for (int k = t; k < QLR; k += 2 * TC) qtwR[k] = A.qtwR[k];
     if (t < R0 * R0) {
@@ -466,20 +519,20 @@ __global__ void __launch_bounds__(2 * R0 * (1 << LOG_L) / (1 << kLargeLogE), (2 
     for (int i = 0; i < E; ++i) v[i] = cmul(v[i], cmul(q, ptab[i]));
     // ---- radix-R0 step across the column's segments, then the twiddle w_R^{n k0} (k0 = seg) ----
 #pragma unroll
-    for (int i = 0; i < E; ++i) mybuf[phys(tl + TL * i)] = v[i];
+    for (int i = 0; i < E; ++i) mybuf[physp<PL>(tl + TL * i)] = v[i];
     hsync();
 #pragma unroll
     for (int i = 0; i < E; ++i) {
         const int n = tl + TL * i;
-        double2 acc = hb[phys(n)];
+        double2 acc = hb[physp<PL>(n)];
 #pragma unroll
-        for (int r = 1; 2 * r < R0; ++r) acc = pair_term_r(acc, hb[r * PADL + phys(n)], hb[(R0 - r) * PADL + phys(n)], omf[seg * R0 + r]);
+        for (int r = 1; 2 * r < R0; ++r) acc = pair_term_r(acc, hb[r * PADL + physp<PL>(n)], hb[(R0 - r) * PADL + physp<PL>(n)], omf[seg * R0 + r]);
         v[i] = cmul(acc, twiddle_r<R>(qtwR, (uint32_t)(n * seg), false));
     }
     hsync();  // every segment read before the L-point FFTs overwrite the buffers
-    forward_from<GL, 0>(v, mybuf, qtwL, tl, ssync);
+    forward_from<GL, 0, NamedSync, 1, PL>(v, mybuf, qtwL, tl, ssync);
 #pragma unroll
-    for (int j = 0; j < E; ++j) mybuf[phys(tl * E + j)] = v[j];
+    for (int j = 0; j < E; ++j) mybuf[physp<PL>(tl * E + j)] = v[j];
     __syncthreads();
     // ---- real-FFT split + square over the pair: frequency d = R0 kk + k0 of this column pairs with
     //      R - 1 - d of column C - c (c == 0: (R - d) mod R of itself) ----
@@ -504,7 +557,7 @@ __global__ void __launch_bounds__(2 * R0 * (1 << LOG_L) / (1 << kLargeLogE), (2 
                 kp = L - 1 - kk;
                 sp = R0 - 1 - seg;
             }
-            const int x = sp * PADL + phys(pos_of_freq<GL>(kp));
+            const int x = sp * PADL + physp<PL>(pos_of_freq<GL>(kp));
             const double2 Av = v[j], Bc = conj2(pb[x]);  // conj(U_{M-k})
             const double2 sm = cadd(Av, Bc), dd = csub(Av, Bc);
             const double2 a3 = make_double2(3.0 * Av.x - Bc.x, 3.0 * Av.y - Bc.y);
@@ -513,22 +566,22 @@ __global__ void __launch_bounds__(2 * R0 * (1 << LOG_L) / (1 << kLargeLogE), (2 
         }
     }
     __syncthreads();  // partner reads done before either column overwrites its buffers
-    inverse_from<GL, GL::P - 1, false>(v, mybuf, qtwL, tl, ssync);
+    inverse_from<GL, GL::P - 1, false, NamedSync, 1, PL>(v, mybuf, qtwL, tl, ssync);
     // ---- conjugate twiddle and the inverse radix-R0 step: thread (r = seg, tl) gets
     //      u[n + L r] = sum_k0 w_R0^{-r k0} w_R^{-n k0} z[k0][n] ----
 #pragma unroll
     for (int i = 0; i < E; ++i) v[i] = cmul(v[i], twiddle_r<R>(qtwR, (uint32_t)((tl + TL * i) * seg), true));
     ssync();  // this segment's last inverse pass read its buffer
 #pragma unroll
-    for (int i = 0; i < E; ++i) mybuf[phys(tl + TL * i)] = v[i];
+    for (int i = 0; i < E; ++i) mybuf[physp<PL>(tl + TL * i)] = v[i];
     hsync();
 #pragma unroll
     for (int i = 0; i < E; ++i) {
         const int n = tl + TL * i;
-        double2 acc = hb[phys(n)];
+        double2 acc = hb[physp<PL>(n)];
 #pragma unroll
         for (int k0 = 1; 2 * k0 < R0; ++k0)
-            acc = pair_term_r(acc, hb[k0 * PADL + phys(n)], hb[(R0 - k0) * PADL + phys(n)], omi[seg * R0 + k0]);
+            acc = pair_term_r(acc, hb[k0 * PADL + physp<PL>(n)], hb[(R0 - k0) * PADL + physp<PL>(n)], omi[seg * R0 + k0]);
         v[i] = acc;
     }
     if (active) {
@@ -545,12 +598,6 @@ static size_t row_smem() {
     return sizeof(double2) * (large_row_slots(LOG_C, G) + twiddle_table_len<GC>()) + (2 * sizeof(double) + sizeof(int)) * GC::M;
 }
 
-template <int LOG_R>
-static size_t col_smem() {
-    using GR = SmallGeom<LOG_R, kLargeLogE>;
-    return sizeof(double2) * 2 * GR::PAD + sizeof(double2) * qpad_s_len(GR::M / 4) + sizeof(double2) * 2 * GR::E;
-}
-
 // Shared-memory carve-out (percent of the SM's 228 KB) for `blocks` resident blocks of `bytes`
 // dynamic shared memory each: no more than they need, so the rest of the on-chip memory stays L1
 // (register spills and the weight-table reads hit there).
@@ -562,40 +609,51 @@ static int carveout_pct(size_t bytes, int blocks) {
 
 template <int R0, int LOG_L>
 static size_t col_mixed_smem() {
-    using GL = SmallGeom<LOG_L, kLargeLogE>;
+    using GL = SmallGeom<LOG_L, kMixedLogE>;
     constexpr int L = GL::M, R = R0 * L;
-    return sizeof(double2) * (2 * R0 * GL::PAD + qpad_len(L / 4) + qpad_len(R / 4) + 2 * R0 * R0 + 2 * GL::E);
+    return sizeof(double2) * (2 * R0 * (L + L / GL::E) + qpad_len(L / 4) + qpad_len(R / 4) + 2 * R0 * R0 + 2 * GL::E);
 }
 
-template <int R0, int LOG_L>
-constexpr int col_mixed_threads() { return 2 * R0 * (1 << LOG_L) / (1 << kLargeLogE); }
-
-template <int LOG_C, int G, int MODE>
+template <int LOG_C, int G, int MODE, bool DENSE>
 static cudaError_t row_attr() {
-    cudaError_t e = cudaFuncSetAttribute(large_row<LOG_C, G, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaError_t e = cudaFuncSetAttribute(large_row<LOG_C, G, MODE, DENSE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)row_smem<LOG_C, G>());
     if (!e)
-        e = cudaFuncSetAttribute(large_row<LOG_C, G, MODE>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                 carveout_pct(row_smem<LOG_C, G>(), large_row_min_blocks(LOG_C, G)));
+        e = cudaFuncSetAttribute(large_row<LOG_C, G, MODE, DENSE>, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                 carveout_pct(row_smem<LOG_C, G>(), large_row_min_blocks(LOG_C, G, DENSE)));
     return e;
 }
+
+// row shapes that have a dense build: tiles of 128 threads (4 blocks an SM, 5 dense)
+constexpr bool large_row_has_dense(int log_c, int g) { return log_c == 8 && g == 4; }
 
 template <int LOG_C, int G>
 static cudaError_t row_attrs() {
-    cudaError_t e = row_attr<LOG_C, G, LARGE_INIT>();
-    if (!e) e = row_attr<LOG_C, G, LARGE_ITER>();
-    if (!e) e = row_attr<LOG_C, G, LARGE_FINAL>();
+    cudaError_t e = row_attr<LOG_C, G, LARGE_INIT, false>();
+    if (!e) e = row_attr<LOG_C, G, LARGE_ITER, false>();
+    if (!e) e = row_attr<LOG_C, G, LARGE_FINAL, false>();
+    if constexpr (large_row_has_dense(LOG_C, G))
+        if (!e) e = row_attr<LOG_C, G, LARGE_ITER, true>();
     return e;
 }
 
+template <int LOG_R, int LE>
+static cudaError_t col_attr_le() {
+    using CG = LargeColGeom<LOG_R, LE>;
+    cudaError_t e = cudaFuncSetAttribute(large_col<LOG_R, LE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CG::smem());
+    if (!e)
+        e = cudaFuncSetAttribute(large_col<LOG_R, LE>, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                 carveout_pct(CG::smem(), CG::MINB));
+    return e;
+}
 template <int LOG_R>
 static cudaError_t col_attr() {
-    cudaError_t e = cudaFuncSetAttribute(large_col<LOG_R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)col_smem<LOG_R>());
-    if (!e)
-        e = cudaFuncSetAttribute(large_col<LOG_R>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                 carveout_pct(col_smem<LOG_R>(), LOG_R <= 11 ? 2 : 1));
-    return e;
+#ifdef LLG_PROBE_LE
+    if constexpr (LOG_R <= 10) { col_attr_le<LOG_R, 2>(); }
+    col_attr_le<LOG_R, 3>();
+    return col_attr_le<LOG_R, 4>();
+#endif
+    return col_attr_le<LOG_R, large_col_log_e(LOG_R)>();
 }
 
 template <int R0, int LOG_L>
@@ -604,15 +662,13 @@ static cudaError_t col_mixed_attr() {
                                          (int)col_mixed_smem<R0, LOG_L>());
     if (!e)
         e = cudaFuncSetAttribute(large_col_mixed<R0, LOG_L>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                 carveout_pct(col_mixed_smem<R0, LOG_L>(), col_mixed_threads<R0, LOG_L>() <= 256 ? 2 : 1));
+                                 carveout_pct(col_mixed_smem<R0, LOG_L>(), 1));
     return e;
 }
 
-// Launch with programmatic stream serialisation at the power-of-two lengths: the kernel may start
-// while the previous kernel of the stream finishes (griddepcontrol in the kernels orders their
-// state accesses after it). At the R0 2^k lengths (logN < 0) it measured slower (5 x 2^18: 37.2 ->
-// 40.7 us per squaring, against 154.1 -> 148.9 at 2^23), so those launch plainly and the
-// griddepcontrol instructions are no-ops.
+// Launch with programmatic stream serialisation: the kernel may start while the previous kernel of
+// the stream finishes (griddepcontrol in the kernels orders their state accesses after it, and
+// LargeArgs::pdl_late says when the previous one lets it).
 template <class... KArgs>
 static cudaError_t launch_pdl(void (*kernel)(KArgs...), int grid, int block, size_t smem, cudaStream_t st,
                               const LargeArgs& a) {
@@ -625,7 +681,7 @@ static cudaError_t launch_pdl(void (*kernel)(KArgs...), int grid, int block, siz
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
-    cfg.numAttrs = a.logN > 0 ? 1 : 0;
+    cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, kernel, a);
 }
 
@@ -640,12 +696,32 @@ static cudaError_t col_mixed_t(const LargeArgs& a, cudaStream_t st) {
 template <int LOG_C, int G, int MODE>
 static cudaError_t row_t(const LargeArgs& a, cudaStream_t st, int grid) {
     if (grid <= 0) grid = a.nblocks + (MODE == LARGE_INIT ? 0 : 1);
-    return launch_pdl(large_row<LOG_C, G, MODE>, grid, large_row_threads(LOG_C, G), row_smem<LOG_C, G>(), st, a);
+    // the dense build where it saves a wave: 641 tiles of 4 x 256 (N = 5 x 2^18) run as one wave of 740
+    // slots instead of two of 592 (28.2 against 29.7 us a squaring); elsewhere it is slower (1025
+    // tiles, N = 2^21: 34.2 against 32.9)
+    if constexpr (MODE == LARGE_ITER && large_row_has_dense(LOG_C, G)) {
+        const int sms = device_sms();
+        if (grid > large_row_min_blocks(LOG_C, G) * sms && grid <= large_row_min_blocks(LOG_C, G, true) * sms)
+            return launch_pdl(large_row<LOG_C, G, MODE, true>, grid, large_row_threads(LOG_C, G), row_smem<LOG_C, G>(), st, a);
+    }
+    return launch_pdl(large_row<LOG_C, G, MODE, false>, grid, large_row_threads(LOG_C, G), row_smem<LOG_C, G>(), st, a);
 }
 
+template <int LOG_R, int LE>
+static cudaError_t col_le(const LargeArgs& a, cudaStream_t st) {
+    using CG = LargeColGeom<LOG_R, LE>;
+    return launch_pdl(large_col<LOG_R, LE>, a.C / 2 + 1, CG::T, CG::smem(), st, a);
+}
 template <int LOG_R>
 static cudaError_t col_t(const LargeArgs& a, cudaStream_t st) {
-    return launch_pdl(large_col<LOG_R>, a.C / 2 + 1, 2 * (1 << LOG_R) / (1 << kLargeLogE), col_smem<LOG_R>(), st, a);
+#ifdef LLG_PROBE_LE
+    const char* ev = getenv("LLG_CLE");
+    const int le = ev ? atoi(ev) : 4;
+    if constexpr (LOG_R <= 10) if (le == 2) return col_le<LOG_R, 2>(a, st);
+    if (le == 3) return col_le<LOG_R, 3>(a, st);
+    return col_le<LOG_R, 4>(a, st);
+#endif
+    return col_le<LOG_R, large_col_log_e(LOG_R)>(a, st);
 }
 
 // Opts the kernels of one geometry into their dynamic shared memory (once per device, before

@@ -134,9 +134,12 @@ bool large_mixed_length_supported(uint64_t n, int* r0, int* log_c) {
     return false;
 }
 
-// Row length (2^log_c complex values) of the two-pass FP64 engine at N = 2^log_n by default.
+// Row length (2^log_c complex values) of the two-pass FP64 engine at N = 2^log_n by default, in
+// tiles of large_rows_per_block rows: the fastest of the supported shapes on a B200. us a squaring,
+// this shape / the default before: 2^14 7.3 / 9.8, 2^15 7.2 / 12.3, 2^16 7.9 / 13.1, 2^17 9.0 / 13.7, 2^18
+// 10.1 / 26.3, 2^19 12.3 / 29.9, 2^20 18.9 / 34.5, 2^21 32.9 / 41.2, 2^22 65.6 / 76.5, 2^23 145.6 / 156.3.
 int large_default_log_c(int log_n) {
-    return (log_n <= 15) ? log_n - 8 : (log_n <= 17) ? 8 : (log_n <= 19) ? 9 : 10;
+    return log_n <= 15 ? 6 : log_n <= 17 ? 7 : log_n == 19 ? 9 : log_n <= 21 ? 8 : log_n == 22 ? 9 : 10;
 }
 
 // Shapes of M = N/2 = 2^log_r rows of 2^log_c values (row blocks of `rows` rows) that the
@@ -147,9 +150,17 @@ bool large_split_supported(int log_n, int log_c, int rows) {
     return large_length_supported(log_n) && log_r >= 7 && log_r <= 12 && large_rows_supported(log_c, rows);
 }
 
+// Whether a pass lets the next one launch at its end rather than its start. Blocks launched early go
+// to the SMs that are free at that moment, several to one, and a pass of about one wave then runs
+// as long as its fullest SM; from several waves on the early start fills the last wave, and the
+// shortest passes are mostly launch latency. Measured at the default shapes, us a squaring, start /
+// end: N = 2^14 7.3 / 8.4, 2^16 7.9 / 9.0, 2^17 10.2 / 9.0, 2^18 13.9 / 10.1, 2^20 27 / 19, 2^21 32.9 / 33.2,
+// 2^23 145.6 / 149.7; 3 x 2^18 28.2 / 21.0, 5 x 2^19 58.8 / 60.1, 5 x 2^20 115.2 / 116.4.
+int large_pdl_late(uint64_t n) { return n > (1ull << 16) && n < (1ull << 21) ? 1 : 0; }
+
 LargeTest::~LargeTest() {
     if (exec) cudaGraphExecDestroy(exec);
-    void* ptrs[] = {V, carry, carry2, ctl, flags, digits, errlog, qtwC, qtwR, qtwL, tw1, tw2, pos_of_c, wA, iwA, sA, wB, iwB, sB};
+    void* ptrs[] = {V, carry, ctl, wrap_read, digits, errlog, qtwC, qtwR, qtwL, tw1, tw2, pos_of_c, wA, iwA, sA, wB, iwB, sB};
     for (void* p : ptrs)
         if (p) cudaFree(p);
 }
@@ -224,13 +235,12 @@ cudaError_t LargeTest::init(uint64_t p_, uint64_t n, int log_c, int rows_) {
     if ((e = upload(&sB, hsB))) return e;
     // state
     if ((e = cudaMalloc(&V, M * sizeof(double2)))) return e;
-    // carry slots and flags: one per tile plus slot 0 for the wrap-around job
-    if ((e = cudaMalloc(&carry, (size_t)(nblocks + 1) * C * sizeof(double)))) return e;
-    if ((e = cudaMalloc(&carry2, (size_t)(nblocks + 1) * C * sizeof(double)))) return e;
+    // carry slots: one per tile plus slot 0 for the wrap-around job
+    if ((e = cudaMalloc(&carry, (size_t)(nblocks + 1) * C * sizeof(LargeCarry)))) return e;
     if ((e = cudaMalloc(&ctl, sizeof(LargeCtl)))) return e;
     if ((e = cudaMemset(ctl, 0, sizeof(LargeCtl)))) return e;
-    if ((e = cudaMalloc(&flags, (size_t)(nblocks + 1) * sizeof(unsigned)))) return e;
-    if ((e = cudaMemset(flags, 0, (size_t)(nblocks + 1) * sizeof(unsigned)))) return e;
+    if ((e = cudaMalloc(&wrap_read, sizeof(unsigned)))) return e;
+    if ((e = cudaMemset(wrap_read, 0, sizeof(unsigned)))) return e;
     if ((e = cudaMalloc(&digits, N * sizeof(int)))) return e;
     errlog_len = 1 << 16;
     if ((e = cudaMalloc(&errlog, errlog_len * sizeof(float)))) return e;
@@ -252,9 +262,9 @@ cudaError_t LargeTest::init(uint64_t p_, uint64_t n, int log_c, int rows_) {
     A.iwB = iwB;
     A.sB = sB;
     A.carry = carry;
-    A.carry2 = carry2;
     A.ctl = ctl;
-    A.flags = flags;
+    A.wrap_read = wrap_read;
+    A.pdl_late = large_pdl_late(N);
     A.digits = digits;
     A.errlog = errlog;
     A.errlog_len = errlog_len;
@@ -279,7 +289,9 @@ cudaError_t LargeTest::start_seed(cudaStream_t st) {
 cudaError_t LargeTest::start_device(cudaStream_t st) {
     cudaError_t e;
     if ((e = cudaMemsetAsync(ctl, 0, sizeof(LargeCtl), st))) return e;
-    if ((e = cudaMemsetAsync(flags, 0, (size_t)(nblocks + 1) * sizeof(unsigned), st))) return e;
+    if ((e = cudaMemsetAsync(wrap_read, 0, sizeof(unsigned), st))) return e;
+    // no tag of an earlier run may pass for this one's
+    if ((e = cudaMemsetAsync(carry, 0, (size_t)(nblocks + 1) * C * sizeof(LargeCarry), st))) return e;
     if ((e = cudaMemsetAsync(errlog, 0, errlog_len * sizeof(float), st))) return e;
     if ((e = launch_large_row(logC, rows, LARGE_INIT, args, st))) return e;
     if ((e = launch_large_col(logR, args, st))) return e;
@@ -330,8 +342,9 @@ cudaError_t LargeTest::step(uint64_t k, cudaStream_t st) {
 cudaError_t LargeTest::final_pass(cudaStream_t st) {
     cudaError_t e;
     if ((e = launch_large_row(logC, rows, LARGE_FINAL, args, st))) return e;
-    // the squarings may resume from this state at the same epoch: clear the flags FINAL set
-    return cudaMemsetAsync(flags, 0, (size_t)(nblocks + 1) * sizeof(unsigned), st);
+    // the squarings may resume from this state at the same epoch: the wrap-around rows must be waited
+    // for again (the carries FINAL published are those the resumed pass publishes)
+    return cudaMemsetAsync(wrap_read, 0, sizeof(unsigned), st);
 }
 
 cudaError_t LargeTest::finish(cudaStream_t st, std::vector<int>& out) {
@@ -346,11 +359,11 @@ cudaError_t LargeTest::diag_withhold_wrap(unsigned long long spin_limit, cudaStr
     LargeCtl h;
     cudaError_t e = read_ctl(h, st);
     if (e) return e;
-    // tickets start at 1: ticket 0, the wrap-around job, is never handed out, so tile 0 and the
-    // last tile wait for its flag until their limit runs out; every index stays that of a tile
-    const unsigned one = 1u;
-    count_h2d(sizeof one);
-    if ((e = cudaMemcpyAsync(&ctl->ticket[h.epoch & 1u], &one, sizeof one, cudaMemcpyHostToDevice, st))) return e;
+    // skip the pass's first ticket: the wrap-around job is never handed out, so tile 0 and the last
+    // tile wait for it until their limit runs out; every index stays that of a tile
+    const unsigned long long next = h.tickets + 1;
+    count_h2d(sizeof next);
+    if ((e = cudaMemcpyAsync(&ctl->tickets, &next, sizeof next, cudaMemcpyHostToDevice, st))) return e;
     LargeArgs a = args;
     a.spin_limit = spin_limit;
     if ((e = launch_large_row(logC, rows, LARGE_ITER, a, st, nblocks))) return e;

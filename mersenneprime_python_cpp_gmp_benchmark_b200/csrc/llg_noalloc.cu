@@ -42,7 +42,7 @@ namespace llg {
 
 namespace {
 
-constexpr size_t kNoAllocScratchBytes = 640u * 1024u;  // covers N = 65,536 (about 603 KiB used)
+constexpr size_t kNoAllocScratchBytes = 640u * 1024u;  // covers N = 65,536 (about 609 KiB used)
 constexpr int kNoAllocMaxLog = 16;
 constexpr int kMaxDevices = 64;
 
@@ -65,7 +65,7 @@ struct TableKey {
 TableKey g_tables_for[kMaxDevices];
 
 struct Layout {
-    size_t V, carry, carry2, ctl, flags, qtwC, qtwR, tw1, tw2, pos_of_c, wA, iwA, sA, wB, iwB, sB, end;
+    size_t V, carry, ctl, wrap_read, qtwC, qtwR, tw1, tw2, pos_of_c, wA, iwA, sA, wB, iwB, sB, end;
 };
 
 size_t up256(size_t x) { return (x + 255) & ~(size_t)255; }
@@ -79,10 +79,9 @@ Layout layout(int logN, int logC, int logR, int s) {
     Layout L;
     size_t o = 0;
     L.V = o; o = up256(o + M * sizeof(double2));
-    L.carry = o; o = up256(o + (nblocks + 1) * C * sizeof(double));  // slot 0: the wrap-around job
-    L.carry2 = o; o = up256(o + (nblocks + 1) * C * sizeof(double));
+    L.carry = o; o = up256(o + (nblocks + 1) * C * sizeof(LargeCarry));  // slot 0: the wrap-around job
     L.ctl = o; o = up256(o + sizeof(LargeCtl));
-    L.flags = o; o = up256(o + (nblocks + 1) * sizeof(unsigned));
+    L.wrap_read = o; o = up256(o + sizeof(unsigned));
     L.qtwC = o; o = up256(o + qpad_len((uint32_t)C) * sizeof(double2));
     L.qtwR = o; o = up256(o + qpad_s_len((uint32_t)(R / 4)) * sizeof(double2));  // spread layout
     L.tw1 = o; o = up256(o + ((size_t)1 << s) * sizeof(double2));
@@ -153,7 +152,7 @@ extern "C" int llg_run_noalloc(uint64_t p, uint64_t iters, uint32_t n, int32_t* 
     // same usability rule as the allocating two-pass path: at least log2(N)/4 + 3 bits per digit
     if (4 * (p / N) < (uint64_t)logN + 12 || (p + N - 1) / N > 28)
         return set_error(LLG_E_UNSUPPORTED, "llg_run_noalloc: length not usable for this p (bits per digit)");
-    const int logC = (logN <= 15) ? logN - 8 : 8;
+    const int logC = 6;
     const int logR = logN - 1 - logC;
     const int C = 1 << logC, R = 1 << logR;
     const int s = logC > (logN / 2) ? logC : (logN / 2);
@@ -227,10 +226,9 @@ extern "C" int llg_run_noalloc(uint64_t p, uint64_t iters, uint32_t n, int32_t* 
     A.wB = reinterpret_cast<const double*>(base + L.wB);
     A.iwB = reinterpret_cast<const double*>(base + L.iwB);
     A.sB = reinterpret_cast<const int*>(base + L.sB);
-    A.carry = reinterpret_cast<double*>(base + L.carry);
-    A.carry2 = reinterpret_cast<double*>(base + L.carry2);
+    A.carry = reinterpret_cast<LargeCarry*>(base + L.carry);
     A.ctl = reinterpret_cast<LargeCtl*>(base + L.ctl);
-    A.flags = reinterpret_cast<unsigned*>(base + L.flags);
+    A.wrap_read = reinterpret_cast<unsigned*>(base + L.wrap_read);
     A.digits = digits_out;
     A.errlog = nullptr;
     A.errlog_len = 1;
@@ -240,6 +238,7 @@ extern "C" int llg_run_noalloc(uint64_t p, uint64_t iters, uint32_t n, int32_t* 
     A.C = C;
     A.R = R;
     A.nblocks = R / kTileRows;
+    A.pdl_late = large_pdl_late(N);
     A.q = (int)(p >> logN);
     A.rem = (int)(p & (N - 1));
     A.N = (int)N;
@@ -258,8 +257,9 @@ extern "C" int llg_run_noalloc(uint64_t p, uint64_t iters, uint32_t n, int32_t* 
     if ((e = cudaMemcpyAsync(digits_out, &four, sizeof four, cudaMemcpyHostToDevice, st)) != cudaSuccess)
         return fail_enqueued("writing s_0", e);
     if ((e = cudaMemsetAsync(A.ctl, 0, sizeof(LargeCtl), st)) != cudaSuccess) return fail_enqueued("clearing the control block", e);
-    if ((e = cudaMemsetAsync(A.flags, 0, (size_t)(A.nblocks + 1) * sizeof(unsigned), st)) != cudaSuccess)
-        return fail_enqueued("clearing the carry flags", e);
+    if ((e = cudaMemsetAsync(A.wrap_read, 0, sizeof(unsigned), st)) != cudaSuccess ||
+        (e = cudaMemsetAsync(A.carry, 0, (size_t)(A.nblocks + 1) * C * sizeof(LargeCarry), st)) != cudaSuccess)
+        return fail_enqueued("clearing the carry slots", e);
     const int G = kTileRows;
     if ((e = launch_large_row(logC, G, LARGE_INIT, A, st)) != cudaSuccess) return fail_enqueued("row pass launch", e);
     if ((e = launch_large_col(logR, A, st)) != cudaSuccess) return fail_enqueued("column pass launch", e);

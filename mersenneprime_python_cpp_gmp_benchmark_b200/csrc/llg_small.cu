@@ -25,7 +25,6 @@
 // it at the next larger N.
 #include <cuda_runtime.h>
 
-#include <atomic>
 #include <cstdint>
 #include <type_traits>
 
@@ -440,19 +439,6 @@ __global__ void ll_word(const SmallJob* __restrict__ jobs, int n, uint64_t* __re
 cudaError_t launch_word(const SmallJob* jobs, int njobs, uint64_t* res, cudaStream_t st) {
     ll_word<<<(njobs + 127) / 128, 128, 0, st>>>(jobs, njobs, res);
     return cudaGetLastError();
-}
-
-// SM count of the current device (148 when it cannot be asked).
-static int device_sms() {
-    static std::atomic<int> sms[64];
-    const int d = PerDeviceOnce::current();
-    if (d < 0) return 148;
-    int n = sms[d].load();
-    if (n == 0) {
-        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, d) != cudaSuccess || n <= 0) n = 148;
-        sms[d].store(n);
-    }
-    return n;
 }
 
 template <int LOG_M, int LE>
