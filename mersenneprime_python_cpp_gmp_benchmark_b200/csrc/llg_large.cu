@@ -110,7 +110,9 @@ template <int LOG_C, int G, int MODE, bool DENSE>
 __global__ void __launch_bounds__(large_row_threads(LOG_C, G), large_row_min_blocks(LOG_C, G, DENSE))
     large_row(const LargeArgs A) {
     constexpr int LE = large_row_log_e(LOG_C, G);
-    using GC = SmallG<LOG_C, LE, TW_FULL, true>;  // full twiddle table, factored twiddles
+    // full twiddle table; at 16 values a thread factored twiddles (at 8, three products fewer and the
+    // same time without)
+    using GC = SmallG<LOG_C, LE, TW_FULL, (LE >= 4)>;
     constexpr int C = GC::M, TR = GC::T, E = GC::E, T = G * TR;
     static_assert(T % 32 == 0 && 32 % G == 0, "whole warps of whole row groups");
     constexpr unsigned FULL = 0xffffffffu;
@@ -594,7 +596,7 @@ __global__ void __launch_bounds__(col_mixed_threads<R0, LOG_L>(), 1)
 
 template <int LOG_C, int G>
 static size_t row_smem() {
-    using GC = SmallG<LOG_C, large_row_log_e(LOG_C, G), TW_FULL, true>;
+    using GC = SmallG<LOG_C, large_row_log_e(LOG_C, G), TW_FULL, (large_row_log_e(LOG_C, G) >= 4)>;
     return sizeof(double2) * (large_row_slots(LOG_C, G) + twiddle_table_len<GC>()) + (2 * sizeof(double) + sizeof(int)) * GC::M;
 }
 
