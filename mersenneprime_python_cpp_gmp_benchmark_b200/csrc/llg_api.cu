@@ -289,6 +289,107 @@ uint32_t next_fp64_length(uint64_t p, uint32_t n) {
     return 0;
 }
 
+// ---- per-device resources kept between calls -----------------------------------------------------
+//
+// A call's device buffers come from a pool of the library's own, which keeps up to kPoolKeep bytes
+// when they are freed (the default pool gives everything back at each synchronisation, and a call
+// then waits for memory to be mapped again: 490 of the 730 us of a call on p = 127), and each
+// group's stream and event from a short free list. llg_release_cached gives both back. Stream-ordered
+// allocation orders reuse across streams; the lists are under one mutex.
+constexpr uint64_t kPoolKeep = 512ull << 20;
+constexpr size_t kStreamsKept = 16;
+
+struct StreamPair {
+    cudaStream_t st = nullptr;
+    cudaEvent_t done = nullptr;
+};
+struct DeviceResources {
+    cudaMemPool_t pool = nullptr;
+    std::vector<StreamPair> streams;
+};
+std::mutex g_res_mx;
+std::map<int, DeviceResources>& device_resources() {
+    static auto* m = new std::map<int, DeviceResources>();  // never destroyed: the context may be gone by then
+    return *m;
+}
+
+void destroy_pair(const StreamPair& sp) {
+    if (sp.st) cudaStreamDestroy(sp.st);
+    if (sp.done) cudaEventDestroy(sp.done);
+}
+
+cudaError_t take_stream(int dev, StreamPair& out) {
+    {
+        std::lock_guard<std::mutex> lk(g_res_mx);
+        std::vector<StreamPair>& v = device_resources()[dev].streams;
+        if (!v.empty()) {
+            out = v.back();
+            v.pop_back();
+            return cudaSuccess;
+        }
+    }
+    cudaError_t e = cudaStreamCreateWithFlags(&out.st, cudaStreamNonBlocking);
+    if (!e) e = cudaEventCreateWithFlags(&out.done, cudaEventDisableTiming);
+    if (e) {
+        destroy_pair(out);
+        out = StreamPair{};
+    }
+    return e;
+}
+
+// Takes back an idle stream and its event.
+void give_stream(int dev, const StreamPair& sp) {
+    {
+        std::lock_guard<std::mutex> lk(g_res_mx);
+        std::vector<StreamPair>& v = device_resources()[dev].streams;
+        if (v.size() < kStreamsKept) {
+            v.push_back(sp);
+            return;
+        }
+    }
+    destroy_pair(sp);
+}
+
+void release_resources() {
+    std::lock_guard<std::mutex> lk(g_res_mx);
+    for (auto& kv : device_resources()) {
+        for (const StreamPair& sp : kv.second.streams) destroy_pair(sp);
+        kv.second.streams.clear();
+        if (kv.second.pool) cudaMemPoolTrimTo(kv.second.pool, 0);
+    }
+}
+
+}  // namespace
+
+namespace llg {
+cudaError_t pool_malloc(void** out, size_t bytes, cudaStream_t st) {
+    int dev = -1;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e) return e;
+    cudaMemPool_t pool = nullptr;
+    {
+        std::lock_guard<std::mutex> lk(g_res_mx);
+        DeviceResources& R = device_resources()[dev];
+        if (!R.pool) {
+            cudaMemPoolProps props = {};
+            props.allocType = cudaMemAllocationTypePinned;
+            props.location.type = cudaMemLocationTypeDevice;
+            props.location.id = dev;
+            e = cudaMemPoolCreate(&R.pool, &props);
+            if (!e) {
+                uint64_t keep = kPoolKeep;
+                e = cudaMemPoolSetAttribute(R.pool, cudaMemPoolAttrReleaseThreshold, &keep);
+            }
+            if (e) return e;
+        }
+        pool = R.pool;
+    }
+    return cudaMallocFromPoolAsync(out, bytes, pool, st);
+}
+}  // namespace llg
+
+namespace {
+
 // ---- batches: exponents grouped by length, one launch per group, groups on their own streams --
 
 struct Item {
@@ -304,14 +405,17 @@ struct Group {
     std::vector<Item> items;
     cudaStream_t st = nullptr;
     cudaEvent_t done = nullptr;
+    void* d_mem = nullptr;  // one allocation: every buffer below, at 256-byte offsets
     void* d_jobs = nullptr;
+    uint64_t* d_word_off = nullptr;
     void* d_results = nullptr;  // SmallResult[] or uint64_t[] (word path)
-    void* d_digits = nullptr;
-    // the residues rebuilt on the device from d_digits: res64, flags (bit 0 zero), words (optional)
+    // the residues rebuilt on the device from d_digits: res64, flags (bit 0 zero), words (optional);
+    // results, res64 and flags are neighbours and come back in one copy of back_bytes
     uint64_t* d_res64 = nullptr;
     int32_t* d_rflags = nullptr;
+    size_t back_bytes = 0;
     uint64_t* d_words = nullptr;
-    uint64_t* d_word_off = nullptr;
+    void* d_digits = nullptr;
     uint64_t pmax = 0;
     size_t total_words = 0;
 };
@@ -339,68 +443,88 @@ struct llg_batch {
     bool collected = false;
     bool keep_words = false;
     std::vector<std::vector<uint64_t>> words;  // per exponent, when keep_words
+    // whole-test groups keep their words in one buffer each, word_view[i] points into it
+    struct WordView {
+        const uint64_t* p = nullptr;
+        size_t n = 0;
+    };
+    std::vector<WordView> word_view;
+    std::vector<std::unique_ptr<uint64_t[]>> word_bufs;
     float* d_errlog = nullptr;  // optional per-iteration round-off log (single-exponent batches)
     uint64_t errlog_len = 0;
 };
 
 namespace {
 
-void release_group(Group& g) {
+void release_group(Group& g, int dev) {
     if (g.st) {
-        for (void* ptr : {g.d_jobs, g.d_results, g.d_digits, (void*)g.d_res64, (void*)g.d_rflags, (void*)g.d_words,
-                          (void*)g.d_word_off})
-            if (ptr) cudaFreeAsync(ptr, g.st);
-        cudaStreamSynchronize(g.st);
-        cudaStreamDestroy(g.st);
+        if (g.d_mem) cudaFreeAsync(g.d_mem, g.st);
+        const bool idle = cudaStreamSynchronize(g.st) == cudaSuccess;
+        if (idle) give_stream(dev, StreamPair{g.st, g.done});
+        else destroy_pair(StreamPair{g.st, g.done});
     }
-    if (g.done) cudaEventDestroy(g.done);
     g = Group();
 }
 
 void destroy_batch(llg_batch* b) {
     if (!b) return;
-    for (Group& g : b->groups) release_group(g);
+    for (Group& g : b->groups) release_group(g, b->dev);
     if (b->fork) cudaEventDestroy(b->fork);
     if (b->joined) cudaEventDestroy(b->joined);
     if (b->d_errlog) cudaFree(b->d_errlog);
     delete b;
 }
 
-// Allocates and uploads one group's job list (synchronously on the group's stream).
-int setup_group(Group& g, bool keep_words) {
-    CK(cudaStreamCreateWithFlags(&g.st, cudaStreamNonBlocking));
-    CK(cudaEventCreateWithFlags(&g.done, cudaEventDisableTiming));
+// Allocates one group's buffers and uploads its job list (the pageable copy has left the host buffer
+// when the call returns).
+int setup_group(Group& g, int dev, bool keep_words) {
+    StreamPair sp;
+    CK(take_stream(dev, sp));
+    g.st = sp.st;
+    g.done = sp.done;
     const size_t cnt = g.items.size();
     // longest first: the block scheduler then hands out the tests in LPT order
     std::sort(g.items.begin(), g.items.end(), [](const Item& a, const Item& b) { return a.iters > b.iters; });
-    std::vector<SmallJob> jobs(cnt);
-    for (size_t i = 0; i < cnt; ++i) jobs[i] = SmallJob{g.items[i].p, g.items[i].iters};
-    CK(cudaMallocAsync(&g.d_jobs, cnt * sizeof(SmallJob), g.st));
-    if (g.n == 0) {
-        CK(cudaMallocAsync(&g.d_results, cnt * 4 * sizeof(uint64_t), g.st));
-    } else {
-        CK(cudaMallocAsync(&g.d_results, cnt * sizeof(SmallResult), g.st));
-        CK(cudaMallocAsync(&g.d_digits, cnt * (size_t)g.n * sizeof(int64_t), g.st));
-        CK(cudaMallocAsync(&g.d_res64, cnt * sizeof(uint64_t), g.st));
-        CK(cudaMallocAsync(&g.d_rflags, cnt * sizeof(int32_t), g.st));
-        g.pmax = 0;
-        for (const Item& it : g.items) g.pmax = std::max(g.pmax, it.p);
-        if (keep_words) {
-            std::vector<uint64_t> off(cnt);
-            g.total_words = 0;
-            for (size_t i = 0; i < cnt; ++i) {
-                off[i] = g.total_words;
-                g.total_words += (size_t)((g.items[i].p + 63) / 64);
-            }
-            CK(cudaMallocAsync(&g.d_words, g.total_words * sizeof(uint64_t), g.st));
-            CK(cudaMallocAsync(&g.d_word_off, cnt * sizeof(uint64_t), g.st));
-            CK(cudaMemcpyAsync(g.d_word_off, off.data(), cnt * sizeof(uint64_t), cudaMemcpyHostToDevice, g.st));
-            count_h2d(cnt * sizeof(uint64_t));
-        }
+    size_t o = 0;
+    auto place = [&](size_t bytes) {
+        const size_t at = o;
+        o = (o + bytes + 255) & ~(size_t)255;
+        return at;
+    };
+    const bool words = keep_words && g.n != 0;
+    const size_t o_jobs = place(cnt * sizeof(SmallJob)), o_off = place(words ? cnt * sizeof(uint64_t) : 0);
+    const size_t up_bytes = o;
+    std::vector<unsigned char> up(up_bytes, 0);
+    SmallJob* jobs = reinterpret_cast<SmallJob*>(up.data() + o_jobs);
+    uint64_t* off = reinterpret_cast<uint64_t*>(up.data() + o_off);
+    g.pmax = 0;
+    g.total_words = 0;
+    for (size_t i = 0; i < cnt; ++i) {
+        jobs[i] = SmallJob{g.items[i].p, g.items[i].iters};
+        g.pmax = std::max(g.pmax, g.items[i].p);
+        if (words) off[i] = g.total_words;
+        g.total_words += (size_t)((g.items[i].p + 63) / 64);
     }
-    CK(cudaMemcpyAsync(g.d_jobs, jobs.data(), cnt * sizeof(SmallJob), cudaMemcpyHostToDevice, g.st));
-    count_h2d(cnt * sizeof(SmallJob));
-    CK(cudaStreamSynchronize(g.st));
+    const size_t o_res = place(g.n == 0 ? cnt * 4 * sizeof(uint64_t) : cnt * sizeof(SmallResult));
+    const size_t o_r64 = place(g.n == 0 ? 0 : cnt * sizeof(uint64_t)), o_rfl = place(g.n == 0 ? 0 : cnt * sizeof(int32_t));
+    g.back_bytes = o - o_res;
+    const size_t o_words = place(words ? g.total_words * sizeof(uint64_t) : 0);
+    const size_t o_dig = place(g.n == 0 ? 0 : cnt * (size_t)g.n * sizeof(int64_t));
+    CK(pool_malloc(&g.d_mem, o, g.st));
+    unsigned char* base = static_cast<unsigned char*>(g.d_mem);
+    g.d_jobs = base + o_jobs;
+    g.d_results = base + o_res;
+    if (g.n) {
+        g.d_res64 = reinterpret_cast<uint64_t*>(base + o_r64);
+        g.d_rflags = reinterpret_cast<int32_t*>(base + o_rfl);
+        g.d_digits = base + o_dig;
+    }
+    if (words) {
+        g.d_word_off = reinterpret_cast<uint64_t*>(base + o_off);
+        g.d_words = reinterpret_cast<uint64_t*>(base + o_words);
+    }
+    CK(cudaMemcpyAsync(base, up.data(), up_bytes, cudaMemcpyHostToDevice, g.st));
+    count_h2d(up_bytes);
     return LLG_OK;
 }
 
@@ -467,17 +591,19 @@ int collect_group(llg_batch* b, Group& g, std::vector<Item>& retry) {
         return LLG_OK;
     }
     const uint32_t n = g.n;
-    std::vector<SmallResult> res(cnt);
-    std::vector<uint64_t> r64(cnt), words;
-    std::vector<int32_t> rfl(cnt);
-    CK(cudaMemcpyAsync(res.data(), g.d_results, cnt * sizeof(SmallResult), cudaMemcpyDeviceToHost, g.st));
-    CK(cudaMemcpyAsync(r64.data(), g.d_res64, cnt * sizeof(uint64_t), cudaMemcpyDeviceToHost, g.st));
-    CK(cudaMemcpyAsync(rfl.data(), g.d_rflags, cnt * sizeof(int32_t), cudaMemcpyDeviceToHost, g.st));
+    std::vector<unsigned char> back(g.back_bytes);
+    CK(cudaMemcpyAsync(back.data(), g.d_results, g.back_bytes, cudaMemcpyDeviceToHost, g.st));
+    const uint64_t* words = nullptr;
     if (b->keep_words) {
-        words.resize(g.total_words);
-        CK(cudaMemcpyAsync(words.data(), g.d_words, g.total_words * sizeof(uint64_t), cudaMemcpyDeviceToHost, g.st));
+        b->word_bufs.emplace_back(new uint64_t[g.total_words]);
+        words = b->word_bufs.back().get();
+        CK(cudaMemcpyAsync(b->word_bufs.back().get(), g.d_words, g.total_words * sizeof(uint64_t), cudaMemcpyDeviceToHost, g.st));
     }
     CK(cudaStreamSynchronize(g.st));
+    const unsigned char* d0 = static_cast<const unsigned char*>(g.d_results);
+    const SmallResult* res = reinterpret_cast<const SmallResult*>(back.data());
+    const uint64_t* r64 = reinterpret_cast<const uint64_t*>(back.data() + (reinterpret_cast<unsigned char*>(g.d_res64) - d0));
+    const int32_t* rfl = reinterpret_cast<const int32_t*>(back.data() + (reinterpret_cast<unsigned char*>(g.d_rflags) - d0));
     size_t woff = 0;
     for (size_t i = 0; i < cnt; ++i) {
         const Item& it = g.items[i];
@@ -505,7 +631,7 @@ int collect_group(llg_batch* b, Group& g, std::vector<Item>& retry) {
         r.n = n;
         r.escalations = it.escalations;
         if (rfl[i] & 2) return fail(LLG_E_CUDA, "device residue rebuild did not settle (p=%llu)", (unsigned long long)it.p);
-        if (b->keep_words) b->words[it.idx].assign(words.begin() + my_off, words.begin() + my_off + nw);
+        if (b->keep_words) b->word_view[it.idx] = llg_batch::WordView{words + my_off, nw};
         r.res64 = r64[i];
         r.is_zero = (rfl[i] & 1) ? 1 : 0;
         r.status = LLG_OK;
@@ -592,7 +718,7 @@ int device_residue(uint64_t p, uint32_t n, const int* d_digits, std::vector<uint
                    size_t host_cap, uint64_t* res64, int32_t* z, cudaStream_t st) {
     const size_t nw = (size_t)((p + 63) / 64);
     uint64_t* dw = nullptr;
-    if (vec || host) CK(cudaMallocAsync(&dw, nw * sizeof(uint64_t), st));
+    if (vec || host) CK(pool_malloc(reinterpret_cast<void**>(&dw), nw * sizeof(uint64_t), st));
     int rc = llg_residue_from_digits_device(p, n, d_digits, dw, res64, z, st);
     if (rc) rc = fail(rc, "residue rebuild on the device failed");
     if (!rc && dw) {
@@ -692,7 +818,7 @@ int run_large_t(const Item& item, llg_result& r, std::vector<uint64_t>* words, c
     };
     if (cudaEventCreate(&e0) != cudaSuccess || cudaEventCreate(&e1) != cudaSuccess)
         return bail(fail(LLG_E_CUDA, "creating events"));
-    if (kFp64 && item.iters > kCheckChunk && cudaMallocAsync(&snap, nw * sizeof(uint64_t), st) != cudaSuccess)
+    if (kFp64 && item.iters > kCheckChunk && pool_malloc(reinterpret_cast<void**>(&snap), nw * sizeof(uint64_t), st) != cudaSuccess)
         return bail(fail(LLG_E_NOMEM, "allocating the residue snapshot"));
     for (;;) {
         std::unique_ptr<TestT> held = take_kept<TestT>(p, n);
@@ -849,7 +975,7 @@ int make_batch(const uint64_t* ps, size_t count, uint64_t max_iters, int engine,
     // largest lengths first (they run longest)
     std::sort(b->groups.begin(), b->groups.end(), [](const Group& x, const Group& y) { return x.n > y.n; });
     for (Group& g : b->groups) {
-        if ((rc = setup_group(g, b->keep_words))) {
+        if ((rc = setup_group(g, b->dev, b->keep_words))) {
             destroy_batch(b);
             return rc;
         }
@@ -889,6 +1015,8 @@ int launch_batch(llg_batch* b, cudaStream_t caller) {
 // Collects every group; round-off aborts are rerun (synchronously) at longer lengths until done.
 int collect_batch(llg_batch* b) {
     if (b->collected) return LLG_OK;
+    b->word_bufs.clear();
+    b->word_view.assign(b->keep_words ? b->count : 0, llg_batch::WordView{});
     std::vector<Item> retry;
     for (Group& g : b->groups) {
         int rc = collect_group(b, g, retry);
@@ -908,13 +1036,13 @@ int collect_batch(llg_batch* b) {
             Group g;
             g.n = kv.first;
             g.items = std::move(kv.second);
-            int rc = setup_group(g, b->keep_words);
+            int rc = setup_group(g, b->dev, b->keep_words);
             if (!rc) {
                 CK(cudaEventRecord(b->fork, g.st));
                 rc = launch_group(b, g, g.st);
             }
             if (!rc) rc = collect_group(b, g, retry);
-            release_group(g);
+            release_group(g, b->dev);
             if (rc) return rc;
         }
     }
@@ -1053,7 +1181,13 @@ void run_pooled(int dev, Request& r) {
     // lead this round
     const auto window = P.last_round > 1 ? kGatherWindow : kGatherWindowAlone;
     lk.unlock();
-    std::this_thread::sleep_for(window);
+    if (window <= kGatherWindowAlone) {
+        // too short for a timed sleep, which takes five times as long
+        const auto until = std::chrono::steady_clock::now() + window;
+        while (std::chrono::steady_clock::now() < until) std::this_thread::yield();
+    } else {
+        std::this_thread::sleep_for(window);
+    }
     lk.lock();
     std::vector<Request*> round;
     round.swap(P.pending);
@@ -1080,6 +1214,7 @@ extern "C" uint64_t llg_h2d_bytes(void) { return llg::g_h2d_bytes.load(); }
 extern "C" void llg_release_cached(void) {
     keep<LargeTest>(nullptr, 0, 0);
     keep<NttLargeTest>(nullptr, 0, 0);
+    release_resources();
 }
 
 extern "C" {
@@ -1256,14 +1391,16 @@ int llg_batch_results(llg_batch* b, llg_result* out, uint64_t* words, size_t wor
         for (size_t i = 0; i < b->count; ++i) total += (size_t)((b->ps[i] + 63) / 64);
         if (words_cap < total) return fail(LLG_E_ARG, "words buffer too small (%zu < %zu)", words_cap, total);
         if (!b->keep_words) return fail(LLG_E_ARG, "batch created without LLG_BATCH_KEEP_WORDS");
-        std::memset(words, 0, words_cap * sizeof(uint64_t));
         size_t off = 0;
         for (size_t i = 0; i < b->count; ++i) {
             const size_t nw = (size_t)((b->ps[i] + 63) / 64);
-            const std::vector<uint64_t>& w = b->words[i];
-            std::memcpy(words + off, w.data(), std::min(nw, w.size()) * sizeof(uint64_t));
+            const llg_batch::WordView v = b->word_view[i].p ? b->word_view[i] : llg_batch::WordView{b->words[i].data(), b->words[i].size()};
+            const size_t n = std::min(nw, v.n);
+            if (n) std::memcpy(words + off, v.p, n * sizeof(uint64_t));
+            std::memset(words + off + n, 0, (nw - n) * sizeof(uint64_t));
             off += nw;
         }
+        std::memset(words + off, 0, (words_cap - off) * sizeof(uint64_t));
     }
     return LLG_OK;
 }
@@ -1395,7 +1532,7 @@ int llg_test_load(llg_test* t, const uint64_t* words, size_t nwords, uint64_t it
     if (p % 64 && (words[nw - 1] >> (p % 64)) != 0) return fail(LLG_E_ARG, "residue has bits at or above p");
     cudaStream_t st = stream ? (cudaStream_t)stream : default_stream_for_thread();
     uint64_t* dw = nullptr;
-    CK(cudaMallocAsync(&dw, nw * sizeof(uint64_t), st));
+    CK(pool_malloc(reinterpret_cast<void**>(&dw), nw * sizeof(uint64_t), st));
     cudaError_t e = cudaMemcpyAsync(dw, words, nw * sizeof(uint64_t), cudaMemcpyHostToDevice, st);
     count_h2d(nw * sizeof(uint64_t));
     int* digits = t->f ? t->f->digits : t->n->digits;

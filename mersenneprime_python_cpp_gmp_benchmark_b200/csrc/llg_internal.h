@@ -81,7 +81,7 @@ cudaError_t launch_small_fp64_mixed(uint32_t n, const SmallJob* jobs, int njobs,
                                     const double2* qtwM, int64_t* digits, SmallResult* results,
                                     float* errlog, double abort_err, cudaStream_t st);
 
-// p < 256: exact multi-limb word arithmetic, one thread per exponent (4 limbs out per exponent).
+// p < 256: exact multi-limb word arithmetic, one block per exponent (4 limbs out per exponent).
 cudaError_t launch_word(const SmallJob* jobs, int njobs, uint64_t* res, cudaStream_t st);
 
 // Goldilocks constants of one NTT length N (mod q): an N-th root of 2 and its inverse in Montgomery
@@ -95,6 +95,9 @@ struct NttConst {
 // N-point transform, gl::qpad8 layout, Montgomery form).
 cudaError_t launch_small_ntt(int log_n, const SmallJob* jobs, int njobs, const uint64_t* qtw, NttConst K,
                              int64_t* digits, SmallResult* results, cudaStream_t st);
+
+// cudaMallocAsync from the library's own pool of the current device (cudaFreeAsync frees).
+cudaError_t pool_malloc(void** out, size_t bytes, cudaStream_t st);
 
 // Adds `bytes` to the library's host-to-device copy count (llg_h2d_bytes).
 void count_h2d(size_t bytes);

@@ -346,7 +346,7 @@ extern "C" int llg_residue_from_digits_device(uint64_t p, uint32_t n, const int3
     // scratch: U, F (unless the caller's words), e, maps, chunk carries, scalars
     const size_t bytes = 2 * nw * sizeof(uint64_t) + nw + 2 * nc + 64;
     unsigned char* mem = nullptr;
-    if (cudaMallocAsync(&mem, bytes, st) != cudaSuccess) return LLG_E_NOMEM;
+    if (pool_malloc(reinterpret_cast<void**>(&mem), bytes, st) != cudaSuccess) return LLG_E_NOMEM;
     uint64_t* U = reinterpret_cast<uint64_t*>(mem);
     uint64_t* F = d_words ? d_words : U + nw;
     int8_t* e = reinterpret_cast<int8_t*>(mem + 2 * nw * sizeof(uint64_t));

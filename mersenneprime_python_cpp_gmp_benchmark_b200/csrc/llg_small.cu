@@ -344,100 +344,96 @@ __global__ void __launch_bounds__(SmallGeo<LOG_M, LE>::T, small_min_blocks(Small
     }
 }
 
-// p < 256: s <- s^2 - 2 mod 2^p - 1 on four 64-bit limbs (schoolbook square, shift-and-add
-// reduction as in lucaslehmer.cpp:42-48), one thread per exponent. Exact; used where digits of
-// an FFT length would hold too few bits for a stable balanced carry.
-__device__ __forceinline__ void word_reduce(uint64_t (&s)[4], const uint64_t (&w)[8], int p) {
-    // lo = w mod 2^p, hi = w >> p, s = lo + hi (both < 2^p), then conditional subtract of M
-    uint64_t lo[4], hi[4];
+// p < 256: s <- s^2 - 2 mod 2^p - 1 on L = ceil(p / 64) 64-bit limbs (schoolbook square, one shift
+// and add for the reduction as in lucaslehmer.cpp:42-48), one block per exponent. Exact; used where
+// digits of an FFT length would hold too few bits for a stable balanced carry. The limb count is a
+// template parameter, so every limb is a register (a runtime limb index put them in local memory:
+// 80 us for the 125 squarings of p = 127, 20 now, launch included).
+template <int L>
+__device__ __forceinline__ void word_test(int p, uint64_t iters, uint64_t (&out)[4]) {
+    // p is odd (or 2): bit p lies inside the top limb, never at a limb boundary
+    const int r = p & 63;
+    const uint64_t mask = (1ull << r) - 1ull;
+    uint64_t s[L];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int bit = 64 * i;
-        lo[i] = (bit + 64 <= p) ? w[i] : (bit < p ? (w[i] & ((1ull << (p - bit)) - 1ull)) : 0ull);
-        // hi limb i = bits [p + 64 i, p + 64 i + 64)
-        const int q = (p + bit) >> 6, r = (p + bit) & 63;
-        const uint64_t a0 = q < 8 ? w[q] : 0ull, a1 = q + 1 < 8 ? w[q + 1] : 0ull;
-        hi[i] = r ? ((a0 >> r) | (a1 << (64 - r))) : a0;
-    }
-    unsigned __int128 c = 0;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        c += (unsigned __int128)lo[i] + hi[i];
-        s[i] = (uint64_t)c;
-        c >>= 64;
-    }
-    // s < 2^(p+1): fold bit p back (2^p == 1) until s < 2^p, then s == M -> 0
-    for (int guard = 0; guard < 3; ++guard) {
-        const int q = p >> 6, r = p & 63;
-        const uint64_t top = (q < 4) ? (s[q] >> r) : 0ull;
-        if (!top) break;
-        if (q < 4) s[q] &= (r ? ((1ull << r) - 1ull) : 0ull);
-        unsigned __int128 cc = top;
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            cc += s[i];
-            s[i] = (uint64_t)cc;
-            cc >>= 64;
-        }
-    }
-    bool all = true;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int bit = 64 * i;
-        const uint64_t full = (bit + 64 <= p) ? ~0ull : (bit < p ? ((1ull << (p - bit)) - 1ull) : 0ull);
-        all = all && (s[i] == full);
-    }
-    if (all)
-#pragma unroll
-        for (int i = 0; i < 4; ++i) s[i] = 0ull;
-}
-
-__global__ void ll_word(const SmallJob* __restrict__ jobs, int n, uint64_t* __restrict__ res) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const int p = (int)jobs[i].p;
-    const uint64_t iters = jobs[i].iters;
-    uint64_t s[4] = {4ull, 0ull, 0ull, 0ull};
-    if (p == 2) s[0] = 1ull;  // 4 mod 3
+    for (int i = 0; i < L; ++i) s[i] = 0ull;
+    s[0] = 4ull;
+    if (L == 1 && p < 3) s[0] = 1ull;  // 4 mod 3
     for (uint64_t k = 0; k < iters; ++k) {
-        uint64_t w[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+        uint64_t w[2 * L];
 #pragma unroll
-        for (int a = 0; a < 4; ++a) {
+        for (int i = 0; i < 2 * L; ++i) w[i] = 0ull;
+#pragma unroll
+        for (int a = 0; a < L; ++a) {
             unsigned __int128 c = 0;
 #pragma unroll
-            for (int b = 0; b < 4; ++b) {
+            for (int b = 0; b < L; ++b) {
                 c += (unsigned __int128)s[a] * s[b] + w[a + b];
                 w[a + b] = (uint64_t)c;
                 c >>= 64;
             }
-            w[a + 4] = (uint64_t)c;
+            w[a + L] = (uint64_t)c;
         }
-        word_reduce(s, w, p);
-        // s - 2 mod M
-        if (s[0] >= 2 || s[1] || s[2] || s[3]) {
-            unsigned __int128 b = 2;
+        // s = (w mod 2^p) + (w >> p), below 2^(p+1); then bit p folded back (2^p == 1)
+        unsigned __int128 c = 0;
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const uint64_t x = s[j];
-                s[j] = x - (uint64_t)b;
-                b = (x < (uint64_t)b) ? 1 : 0;
+        for (int i = 0; i < L; ++i) {
+            const uint64_t lo = i == L - 1 ? w[i] & mask : w[i];
+            const uint64_t up = L + i < 2 * L ? w[L + i] : 0ull;
+            c += (unsigned __int128)lo + ((w[L - 1 + i] >> r) | (up << (64 - r)));
+            s[i] = (uint64_t)c;
+            c >>= 64;
+        }
+        c = s[L - 1] >> r;
+        s[L - 1] &= mask;
+#pragma unroll
+        for (int i = 0; i < L; ++i) {
+            c += s[i];
+            s[i] = (uint64_t)c;
+            c >>= 64;
+        }
+        // s - 2 (s may still be 2^p - 1 standing for 0)
+        uint64_t rest = 0ull;
+#pragma unroll
+        for (int i = 1; i < L; ++i) rest |= s[i];
+        if (rest || s[0] >= 2) {
+            uint64_t borrow = 2ull;
+#pragma unroll
+            for (int i = 0; i < L; ++i) {
+                const uint64_t x = s[i];
+                s[i] = x - borrow;
+                borrow = x < borrow ? 1ull : 0ull;
             }
-        } else {  // s in {0, 1}: s - 2 + M = M - (2 - s)
+        } else {  // s in {0, 1}: s - 2 + 2^p - 1
             const uint64_t v = s[0];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const int bit = 64 * j;
-                s[j] = (bit + 64 <= p) ? ~0ull : (bit < p ? ((1ull << (p - bit)) - 1ull) : 0ull);
-            }
+            for (int i = 0; i < L; ++i) s[i] = i == L - 1 ? mask : ~0ull;
             s[0] -= 2ull - v;
         }
     }
+    bool all = true;  // 2^p - 1 is 0
 #pragma unroll
-    for (int j = 0; j < 4; ++j) res[(size_t)i * 4 + j] = s[j];
+    for (int i = 0; i < L; ++i) all = all && s[i] == (i == L - 1 ? mask : ~0ull);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) out[i] = (i < L && !all) ? s[i < L ? i : 0] : 0ull;
+}
+
+__global__ void ll_word(const SmallJob* __restrict__ jobs, uint64_t* __restrict__ res) {
+    const int p = (int)jobs[blockIdx.x].p;
+    const uint64_t iters = jobs[blockIdx.x].iters;
+    uint64_t s[4];
+    switch (p >> 6) {
+        case 0: word_test<1>(p, iters, s); break;
+        case 1: word_test<2>(p, iters, s); break;
+        case 2: word_test<3>(p, iters, s); break;
+        default: word_test<4>(p, iters, s); break;
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) res[(size_t)blockIdx.x * 4 + j] = s[j];
 }
 
 cudaError_t launch_word(const SmallJob* jobs, int njobs, uint64_t* res, cudaStream_t st) {
-    ll_word<<<(njobs + 127) / 128, 128, 0, st>>>(jobs, njobs, res);
+    ll_word<<<njobs, 1, 0, st>>>(jobs, res);
     return cudaGetLastError();
 }
 
