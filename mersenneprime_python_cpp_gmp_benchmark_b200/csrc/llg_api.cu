@@ -66,9 +66,7 @@ constexpr int kSmallLogMax = 13;  // N = 8192
 // ---- device tables ------------------------------------------------------------------------
 
 struct DeviceTables {
-    std::map<uint32_t, double2*> qtw;      // quarter-wave twiddles of the M-point FFT, by M
-    std::map<uint32_t, double2*> qtw_s;    // the same in the spread layout (qpad_s), by M
-    std::map<uint32_t, double2*> qtw_p;    // twiddles in pass order (pass_twiddle_table), by 64 log2 M + log2 E
+    std::map<uint32_t, double2*> qtw;      // twiddles of the FP64 kernels, by get_table's key
     uint64_t* nqtw[kSmallLogMax + 1] = {}; // NTT: padded twiddle table of the N-point transform
     NttConst nk[kSmallLogMax + 1] = {};
 };
@@ -123,26 +121,15 @@ int device_ready(int* dev_out) {
     return LLG_OK;
 }
 
-int get_qtw(int dev, uint32_t m, const double2** out, bool spread = false) {
+// A twiddle table of the whole-test FP64 kernels, built and uploaded on its first use: key 64 log2 M
+// + log2 E (pass order), log2 M alone (spread quarter table), 4096 R0 + log2 L (mixed lengths).
+int get_table(int dev, uint32_t key, const double2** out) {
     std::lock_guard<std::mutex> lk(g_mx);
-    DeviceTables& T = g_tables[dev];
-    double2*& d = spread ? T.qtw_s[m] : T.qtw[m];
+    double2*& d = g_tables[dev].qtw[key];
     if (!d) {
-        // padded layout (qpad), or the spread one (qpad_s)
-        std::vector<double2> h = spread ? spread_quarter_table(m) : padded_quarter_table(m);
-        CK(cudaMalloc(&d, h.size() * sizeof(double2)));
-        CK(cudaMemcpy(d, h.data(), h.size() * sizeof(double2), cudaMemcpyHostToDevice));
-        count_h2d(h.size() * sizeof(double2));
-    }
-    *out = d;
-    return LLG_OK;
-}
-
-int get_pass_table(int dev, int log_m, int log_e, const double2** out) {
-    std::lock_guard<std::mutex> lk(g_mx);
-    double2*& d = g_tables[dev].qtw_p[64u * (uint32_t)log_m + (uint32_t)log_e];
-    if (!d) {
-        std::vector<double2> h = pass_twiddle_table(log_m, log_e);
+        const std::vector<double2> h = key >= 4096 ? mixed_twiddle_table((int)(key >> 12), (int)(key & 63))
+                                       : key >= 64 ? pass_twiddle_table((int)(key >> 6), (int)(key & 63))
+                                                   : spread_quarter_table(1ull << key);
         CK(cudaMalloc(&d, h.size() * sizeof(double2)));
         CK(cudaMemcpy(d, h.data(), h.size() * sizeof(double2), cudaMemcpyHostToDevice));
         count_h2d(h.size() * sizeof(double2));
@@ -543,7 +530,7 @@ int launch_group(llg_batch* b, Group& g, cudaStream_t caller) {
     } else if (is_small_pow2_length(g.n)) {
         const double2* qtw = nullptr;
         const int ln = ilog2_exact(g.n), le = small_fp64_log_e(ln, cnt);
-        int rc = small_fp64_pass_table(le) ? get_pass_table(b->dev, ln - 1, le, &qtw) : get_qtw(b->dev, g.n / 2, &qtw, true);
+        int rc = get_table(b->dev, (uint32_t)(small_fp64_pass_table(le) ? 64 * (ln - 1) + le : ln - 1), &qtw);
         if (rc) return rc;
         float* elog = (cnt == 1) ? b->d_errlog : nullptr;
         CK(launch_small_fp64(ln, le, (const SmallJob*)g.d_jobs, cnt, qtw, (int64_t*)g.d_digits,
@@ -551,12 +538,11 @@ int launch_group(llg_batch* b, Group& g, cudaStream_t caller) {
     } else {
         int r0 = 0, ll = 0;
         mixed_length_supported(g.n, &r0, &ll);
-        const double2 *qtwL = nullptr, *qtwM = nullptr;
-        int rc = get_qtw(b->dev, 1u << ll, &qtwL);
-        if (!rc) rc = get_qtw(b->dev, g.n / 2, &qtwM);
+        const double2* qtw = nullptr;
+        int rc = get_table(b->dev, 4096u * (uint32_t)r0 + (uint32_t)ll, &qtw);
         if (rc) return rc;
         float* elog = (cnt == 1) ? b->d_errlog : nullptr;
-        CK(launch_small_fp64_mixed(g.n, (const SmallJob*)g.d_jobs, cnt, qtwL, qtwM, (int64_t*)g.d_digits,
+        CK(launch_small_fp64_mixed(g.n, (const SmallJob*)g.d_jobs, cnt, qtw, (int64_t*)g.d_digits,
                                    (SmallResult*)g.d_results, elog, g_abort_err.load(), g.st));
     }
     if (g.n) {

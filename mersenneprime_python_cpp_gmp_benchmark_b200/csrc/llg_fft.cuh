@@ -272,6 +272,31 @@ struct SmallG : SmallGeom<LOG_M_T, LOG_E> {
     static constexpr bool TWF = TF;
 };
 
+// Real-FFT split twiddle e^{-2 pi i k / M} from a table that starts with the powers below LOW, LOW at
+// least M / 8: k folds to r < M / 4 by its quadrant (bits 13, 14: times (-i)^quad) and, at r >= LOW, by
+// swapping cosine and sine (bit 15). LOW = M / 8 (TW_PASS at 8 values a thread): r = M / 8 itself is
+// w^{2 (M/16)}, entry M/16 of the first pass's k1 = 2.
+template <int M, int LOW>
+__device__ __forceinline__ unsigned short split_code(int k) {
+    static_assert(LOW >= M / 8 && M / 4 <= 0x2000, "table too short, or slots beyond the code");
+    const int quad = k / (M / 4);
+    int r = k % (M / 4), swap = 0;
+    if (LOW < M / 4 && r >= LOW && 8 * r != M) {
+        r = M / 4 - r;
+        swap = 1;
+    }
+    if (8 * LOW == M && 8 * r == M) r = M / 8 + M / 16;
+    return (unsigned short)(r | (quad << 13) | (swap << 15));
+}
+__device__ __forceinline__ double2 split_twiddle(const double2* __restrict__ tw, unsigned code) {
+    const double2 w = tw[code & 0x1fffu];
+    const bool swap = (code & 0x8000u) != 0, odd = (code & 0x2000u) != 0;
+    // e^{-i(pi/2 - a)} = sin a - i cos a: (x, y) -> (-y, -x); times (-i): (x, y) -> (y, -x)
+    const double2 a = swap ? make_double2(-w.y, -w.x) : w;
+    const double2 b = odd ? make_double2(a.y, -a.x) : a;
+    return (code & 0x4000u) ? make_double2(-b.x, -b.y) : b;
+}
+
 // Length (16-byte slots) of the twiddle table a geometry reads.
 template <class G>
 __host__ __device__ constexpr uint32_t twiddle_table_len() {

@@ -87,6 +87,18 @@ std::vector<double2> pass_twiddle_table(int log_l, int log_e) {
     return t;
 }
 
+std::vector<double2> mixed_twiddle_table(int r0, int log_l) {
+    std::vector<double2> t = pass_twiddle_table(log_l, 3);
+    const uint64_t L = 1ull << log_l, M = (uint64_t)r0 * L;
+    const long double two_pi = 6.283185307179586476925286766559005768L;
+    for (uint64_t k0 = 1; k0 < (uint64_t)r0; ++k0)
+        for (uint64_t n = 0; n < L; ++n) {
+            const long double ang = two_pi * (long double)(n * k0) / (long double)M;
+            t.push_back(make_double2((double)cosl(ang), -(double)sinl(ang)));
+        }
+    return t;
+}
+
 std::vector<double2> padded_quarter_table(uint64_t L) {
     const uint64_t n = qpad_len((uint32_t)(L / 4));
     std::vector<double2> t(n);

@@ -62,30 +62,6 @@ using SmallGeo = SmallG<LOG_M, LE, small_tw_layout(LE), true>;
 // and cost 10 to 20% at N = 1024 and 2048)
 __host__ __device__ constexpr int small_min_blocks(int t) { return t < 32 ? 16 : 512 / t > 16 ? 16 : 512 / t; }
 
-// Real-FFT split twiddle e^{-2 pi i k / M} from the TW_PASS table, whose first M / E entries are the
-// powers below M / E (k1 = 1 of the first pass): k folds to r <= M/8 (E = 8) or r < M/4, by the
-// quadrant (bits 13, 14: times (-i)^quad) and, past an eighth, by swapping cosine and sine
-// (bit 15). r = M/8 itself is w^{2 (M/16)}, entry M/16 of k1 = 2.
-template <int M, int E>
-__device__ __forceinline__ unsigned short split_code(int k) {
-    const int quad = k / (M / 4);
-    int r = k % (M / 4), swap = 0;
-    if (E == 8 && r > M / 8) {
-        r = M / 4 - r;
-        swap = 1;
-    }
-    if (E == 8 && r == M / 8) r = M / 8 + M / 16;
-    return (unsigned short)(r | (quad << 13) | (swap << 15));
-}
-__device__ __forceinline__ double2 split_twiddle(const double2* __restrict__ tw, unsigned code) {
-    const double2 w = tw[code & 0x1fffu];
-    const bool swap = (code & 0x8000u) != 0, odd = (code & 0x2000u) != 0;
-    // e^{-i(pi/2 - a)} = sin a - i cos a: (x, y) -> (-y, -x); times (-i): (x, y) -> (y, -x)
-    const double2 a = swap ? make_double2(-w.y, -w.x) : w;
-    const double2 b = odd ? make_double2(a.y, -a.x) : a;
-    return (code & 0x4000u) ? make_double2(-b.x, -b.y) : b;
-}
-
 template <int LOG_M, int LE>
 __global__ void __launch_bounds__(SmallGeo<LOG_M, LE>::T, small_min_blocks(SmallGeo<LOG_M, LE>::T))
     ll_small_fp64(const SmallJob* __restrict__ jobs, const double2* __restrict__ qtw_g,
@@ -136,7 +112,7 @@ __global__ void __launch_bounds__(SmallGeo<LOG_M, LE>::T, small_min_blocks(Small
     }
     if constexpr (G::TWM == TW_PASS) {
 #pragma unroll
-        for (int h = 0; h < NBK; ++h) kslot[h * T + t] = split_code<M, E>(freq_rev<G>(t * NBK + h));
+        for (int h = 0; h < NBK; ++h) kslot[h * T + t] = split_code<M, M / E>(freq_rev<G>(t * NBK + h));
     }
     __syncthreads();
 
