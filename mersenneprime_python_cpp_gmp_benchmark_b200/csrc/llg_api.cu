@@ -122,12 +122,12 @@ int device_ready(int* dev_out) {
 }
 
 // A twiddle table of the whole-test FP64 kernels, built and uploaded on its first use: key 64 log2 M
-// + log2 E (pass order), log2 M alone (spread quarter table), 4096 R0 + log2 L (mixed lengths).
+// + log2 E (pass order), log2 M alone (spread quarter table), 4096 R0 + 64 log2 L + log2 E (mixed).
 int get_table(int dev, uint32_t key, const double2** out) {
     std::lock_guard<std::mutex> lk(g_mx);
     double2*& d = g_tables[dev].qtw[key];
     if (!d) {
-        const std::vector<double2> h = key >= 4096 ? mixed_twiddle_table((int)(key >> 12), (int)(key & 63))
+        const std::vector<double2> h = key >= 4096 ? mixed_twiddle_table((int)(key >> 12), (int)((key >> 6) & 63), (int)(key & 63))
                                        : key >= 64 ? pass_twiddle_table((int)(key >> 6), (int)(key & 63))
                                                    : spread_quarter_table(1ull << key);
         CK(cudaMalloc(&d, h.size() * sizeof(double2)));
@@ -539,7 +539,7 @@ int launch_group(llg_batch* b, Group& g, cudaStream_t caller) {
         int r0 = 0, ll = 0;
         mixed_length_supported(g.n, &r0, &ll);
         const double2* qtw = nullptr;
-        int rc = get_table(b->dev, 4096u * (uint32_t)r0 + (uint32_t)ll, &qtw);
+        int rc = get_table(b->dev, 4096u * (uint32_t)r0 + 64u * (uint32_t)ll + (uint32_t)small_fp64_mixed_log_e(g.n, cnt), &qtw);
         if (rc) return rc;
         float* elog = (cnt == 1) ? b->d_errlog : nullptr;
         CK(launch_small_fp64_mixed(g.n, (const SmallJob*)g.d_jobs, cnt, qtw, (int64_t*)g.d_digits,

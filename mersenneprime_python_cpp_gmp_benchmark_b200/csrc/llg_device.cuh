@@ -237,11 +237,39 @@ __device__ __forceinline__ double dsplit(double v, double inv, double pw, double
     return __fma_rn(-c, pw, v);
 }
 
-// dsplit with digit size e bits: 2^e and 2^-e built from the exponent field (few live registers).
-__device__ __forceinline__ double dsplit_e(double v, int e, double& c) {
-    const double pw = __hiloint2double((1023 + e) << 20, 0), inv = __hiloint2double((1023 - e) << 20, 0);
-    return dsplit(v, inv, pw, c);
+// The digit kinds of a test are fixed: 4 bits a value, bit 0 / 1: digit 2m / 2m+1 has q + 1 bits;
+// bit 2 / 3: its weight exponent s_A + s_B wrapped past N (the weight is the table product / 2). A
+// kind bit at position p (compile time) as 1 << 20 or 0, one unit of a double's exponent field: digit
+// sizes and weights are then integer additions to high words, no selects and no products by 1 or 2.
+__device__ __forceinline__ uint32_t kind_unit(uint32_t w, int p) {
+    return (p <= 20 ? w << (20 - p) : w >> (p - 20)) & 0x100000u;
 }
+// x * 2 (x / 2) for m = 1 << 20, x for m = 0; x a normal number
+__device__ __forceinline__ double scale_up(double x, uint32_t m) {
+    return __hiloint2double(__double2hiint(x) + (int)m, __double2loint(x));
+}
+__device__ __forceinline__ double scale_down(double x, uint32_t m) {
+    return __hiloint2double(__double2hiint(x) - (int)m, __double2loint(x));
+}
+
+// High words of 2^q and 2^-q.
+struct DigitBase {
+    int up, down;
+    __device__ __forceinline__ explicit DigitBase(int q) : up((1023 + q) << 20), down((1023 - q) << 20) {}
+};
+// dsplit with a digit of q bits (m = 0) or q + 1 bits (m = 1 << 20).
+__device__ __forceinline__ double dsplit_k(double v, const DigitBase& B, uint32_t m, double& c) {
+    return dsplit(v, __hiloint2double(B.down - (int)m, 0), __hiloint2double(B.up + (int)m, 0), c);
+}
+
+// Largest |d| of a run of differences, kept as the high word (20 bits of mantissa: |x - round(x)| of
+// the values met here has no more, and a maximum of integers needs no FP64 compare and selects).
+// Not-a-number counts as infinite.
+struct ErrMax {
+    uint32_t m = 0u;
+    __device__ __forceinline__ void add(double d) { m = max(m, (uint32_t)__double2hiint(d) & 0x7fffffffu); }
+    __device__ __forceinline__ double value() const { return __hiloint2double((int)min(m, 0x7ff00000u), 0); }
+};
 
 // An integer-valued double with |x| < 2^31 as int32 (the low word of x + 1.5 * 2^52).
 __device__ __forceinline__ int d2i_exact(double x) { return __double2loint(__dadd_rn(x, 6755399441055744.0)); }

@@ -29,8 +29,8 @@ double2 padded_quarter_slot(uint64_t L, uint64_t i);
 std::vector<double2> spread_quarter_table(uint64_t L);
 // The twiddles of an L-point FFT of 2^log_e values a thread, pass by pass (TW_PASS).
 std::vector<double2> pass_twiddle_table(int log_l, int log_e);
-// pass_twiddle_table(log_l, 3), then w_M^{n k0} over n < L for k0 = 1 .. r0 - 1 (M = r0 L, L = 2^log_l).
-std::vector<double2> mixed_twiddle_table(int r0, int log_l);
+// pass_twiddle_table(log_l, log_e), then w_M^{n k0} over n < L for k0 = 1 .. r0 - 1 (M = r0 L, L = 2^log_l).
+std::vector<double2> mixed_twiddle_table(int r0, int log_l, int log_e);
 
 struct LargeTest {
     uint64_t p = 0, N = 0, M = 0;
@@ -47,6 +47,7 @@ struct LargeTest {
     int* pos_of_c = nullptr;
     double *wA = nullptr, *iwA = nullptr, *wB = nullptr, *iwB = nullptr;
     int *sA = nullptr, *sB = nullptr;
+    uint32_t* kinds = nullptr;
     LargeArgs args{};
     cudaGraphExec_t exec = nullptr;
     uint64_t done = 0;  // squarings enqueued since start()

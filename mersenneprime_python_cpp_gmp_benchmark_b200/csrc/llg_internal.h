@@ -75,8 +75,9 @@ cudaError_t launch_small_fp64(int log_n, int log_e, const SmallJob* jobs, int nj
                               double abort_err, cudaStream_t st);
 
 // FP64 whole-test kernel for N = 2 R0 2^l (R0 = 3: l = 9..11; R0 = 5: l = 9..10); qtw: the twiddles
-// mixed_twiddle_table builds.
+// mixed_twiddle_table builds for the form's values a thread.
 bool mixed_length_supported(uint32_t n, int* r0, int* log_l);
+int small_fp64_mixed_log_e(uint32_t n, int njobs);  // log2 of the values a thread for that many tests
 cudaError_t launch_small_fp64_mixed(uint32_t n, const SmallJob* jobs, int njobs, const double2* qtw,
                                     int64_t* digits, SmallResult* results, float* errlog,
                                     double abort_err, cudaStream_t st);
@@ -187,10 +188,9 @@ struct LargeArgs {
     const int* pos_of_c;      // column slot of row-FFT frequency c
     const double* wA;         // [2R] 2^(sA/N) of digit 2a+e
     const double* iwA;        // [2R] 2^(-sA/N)
-    const int* sA;            // [2R] (-(2a+e) p) mod N
     const double* wB;         // [C] 2^(sB/N)
     const double* iwB;        // [C] 2^(-sB/N) / (4M)
-    const int* sB;            // [C] (-2Rb p) mod N
+    const uint32_t* kinds;    // digit kinds by tile and thread (fill_kinds): N / 16 words
     LargeCarry* carry;        // [nblocks + 1][C] carry-outs of a tile's last row: slot 0 the
                               // wrap-around job's (row R-1, one column on), k + 1 tile k's
     LargeCtl* ctl;
@@ -208,6 +208,10 @@ struct LargeArgs {
     int logN;                 // log2 N for a power of two
 };
 
+// Fills LargeArgs::kinds for tiles of g rows with 2^log_e values a thread from the weight exponents sA
+// ([2R] (-(2a+e) p) mod N) and sB ([C] (-2Rb p) mod N); R C / 8 words.
+cudaError_t launch_fill_kinds(uint32_t* kinds, const int* sA, const int* sB, int N, int rem, int C, int R, int g, int log_e,
+                              cudaStream_t st);
 // Row pass; grid > 0 overrides the block count (nblocks, + 1 for the wrap-around job unless INIT).
 cudaError_t launch_large_row(int log_c, int g, int mode, const LargeArgs& a, cudaStream_t st, int grid = 0);
 // Column-length code of the two-pass engine: log2 R for a power of two, 100 R0 + log2 L for the

@@ -122,14 +122,13 @@ __global__ void __launch_bounds__(large_row_threads(LOG_C, G), large_row_min_blo
     double2* qtw = xbuf + large_row_slots(LOG_C, G);               // padded twiddle table (C-point)
     double* swB = reinterpret_cast<double*>(qtw + QL);             // C column weights 2^(sB/N)
     double* siwB = swB + C;                                        // C inverse column weights
-    int* ssB = reinterpret_cast<int*>(siwB + C);                   // C column weight exponents sB
     __shared__ unsigned long long s_err;
     __shared__ int s_job;
     __shared__ unsigned s_epoch;
 
     const int t = threadIdx.x, ra = t % G, tr = t / G;
     double2* buf = xbuf + ra;
-    const int N = A.N, R = A.R;
+    const int R = A.R;
     const CtaSync sync;
 
     // The pass's constant tables are requested (asynchronous copies, completed before the barrier that
@@ -139,7 +138,6 @@ __global__ void __launch_bounds__(large_row_threads(LOG_C, G), large_row_min_blo
     for (int k = t; k < C; k += T) {
         cp_async<8>(swB + k, A.wB + k);
         if (MODE != LARGE_INIT) cp_async<8>(siwB + k, A.iwB + k);
-        cp_async<4>(ssB + k, A.sB + k);
     }
     if (t == 0) {
         if (MODE == LARGE_INIT) {
@@ -171,25 +169,13 @@ __global__ void __launch_bounds__(large_row_threads(LOG_C, G), large_row_min_blo
     const unsigned ep = s_epoch;
     const bool wrap_job = job < 0;
     const int a = (wrap_job ? R - G : job * G) + ra;  // this thread's row
-    // weight exponent s = (sA(2a+e) + sB(b)) mod N of digit 2m+e, sB(b) = (-2 R b p) mod N from
-    // the shared-memory copy of its table. digit_kind(b) gives bit 0 / 1: digit 0 / 1 of (a, b) has
-    // q + 1 bits (s < p mod N); bit 2 / 3: sA + sB wrapped past N, so the weight 2^(s/N) is the
-    // table product times 1/2 (and the inverse weight times 2). Recomputed where used: a few
-    // integer operations, fewer live registers than keeping them.
-    const int sA0 = __ldg(A.sA + 2 * a), sA1 = __ldg(A.sA + 2 * a + 1);
-    auto kind_at = [&](int s0a, int s1a, int b) {
-        const int sb = ssB[b];
-        const bool o0 = s0a + sb >= N, o1 = s1a + sb >= N;
-        const int s0 = o0 ? s0a + sb - N : s0a + sb, s1 = o1 ? s1a + sb - N : s1a + sb;
-        return (uint32_t)(s0 < A.rem) | ((uint32_t)(s1 < A.rem) << 1) | ((uint32_t)o0 << 2) | ((uint32_t)o1 << 3);
-    };
-    auto digit_kind = [&](int b) { return kind_at(sA0, sA1, b); };
-    // the digit kinds of this thread's E values, 4 bits each, from the carry to the re-weighting
-    // (at 16 values a thread; at 8, where registers are scarcer, recomputed)
-    constexpr bool KEEP_KINDS = LE >= 4;
-    uint32_t kinds[(E + 7) / 8];
+    // the digit kinds of this thread's E values, 4 bits each (kind_unit)
+    constexpr int KW = E / 8;
+    uint32_t kinds[KW];
 #pragma unroll
-    for (int w = 0; w < (E + 7) / 8; ++w) kinds[w] = 0u;
+    for (int w = 0; w < KW; ++w) kinds[w] = __ldg(A.kinds + ((size_t)(a / G) * T + t) * KW + w);
+    auto kind = [&](int i, int bit) { return kind_unit(kinds[i / 8], 4 * (i % 8) + bit); };
+    const DigitBase dq(A.q);
 
     double2 v[E];
     if constexpr (MODE == LARGE_INIT) {
@@ -220,40 +206,38 @@ __global__ void __launch_bounds__(large_row_threads(LOG_C, G), large_row_min_blo
         if (wrap_job && t == 0) *reinterpret_cast<volatile unsigned*>(A.wrap_read) = ep + 1u;  // its rows are read
         LargeCarry* pub = A.carry + (size_t)(job + 1) * C;
         const double ia0 = __ldg(A.iwA + 2 * a), ia1 = __ldg(A.iwA + 2 * a + 1);
-        double lerr = 0.0;
+        ErrMax err;
 #pragma unroll
         for (int i = 0; i < E; ++i) {
             const int b = tr + TR * i;
             const double iwb = siwB[b];
-            const uint32_t kd = digit_kind(b);
-            if (KEEP_KINDS) kinds[i / 8] |= kd << (4 * (i % 8));
-            const int w0 = kd & 1u, w1 = (kd >> 1) & 1u;
-            const double va = v[i].x * (ia0 * iwb) * ((kd & 4u) ? 2.0 : 1.0);
-            const double vb = v[i].y * (ia1 * iwb) * ((kd & 8u) ? 2.0 : 1.0);
+            const double va = v[i].x * scale_up(ia0 * iwb, kind(i, 2));
+            const double vb = v[i].y * scale_up(ia1 * iwb, kind(i, 3));
             long long ia, ib;
             const double r0 = round_shift(va, ia), r1 = round_shift(vb, ib);
-            lerr = fmax(lerr, fmax(fabs(va - r0), fabs(vb - r1)));
+            err.add(va - r0);
+            err.add(vb - r1);
             double c, c1, c2 = 0.0;
-            double x0 = dsplit_e(r0, A.q + w0, c);
-            double x1 = dsplit_e(r1 + c, A.q + w1, c1);
+            double x0 = dsplit_k(r0, dq, kind(i, 0), c);
+            double x1 = dsplit_k(r1 + c, dq, kind(i, 1), c1);
             const double cin = __shfl_up_sync(FULL, c1, 1, G);
             if (ra > 0) {
-                x0 = dsplit_e(x0 + cin, A.q + w0, c);
-                x1 = dsplit_e(x1 + c, A.q + w1, c2);
+                x0 = dsplit_k(x0 + cin, dq, kind(i, 0), c);
+                x1 = dsplit_k(x1 + c, dq, kind(i, 1), c2);
             }
-            const double cin2 = __shfl_up_sync(FULL, c2, 1, G);
-            if (ra > 1) x0 += cin2;
+            const int c2i = d2i_exact(c2);
+            const int cin2 = __shfl_up_sync(FULL, c2i, 1, G);
+            if (ra > 1) x0 += i2d_shift(cin2);
             if (ra == G - 1) {
                 // row R-1, column b feeds row 0, column b+1
-                st_carry(pub + (wrap_job ? ((b + 1) & (C - 1)) : b), c1, (int)c2, ep + 1u);
+                st_carry(pub + (wrap_job ? ((b + 1) & (C - 1)) : b), c1, c2i, ep + 1u);
             }
             v[i] = make_double2(x0, x1);
         }
         if (wrap_job) return;
         // the tile's round-off max: one shared atomic per warp
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) lerr = fmax(lerr, __shfl_xor_sync(FULL, lerr, o));
-        if ((t & 31) == 0) atomicMax(&s_err, (unsigned long long)__double_as_longlong(lerr));
+        err.m = __reduce_max_sync(FULL, err.m);
+        if ((t & 31) == 0) atomicMax(&s_err, (unsigned long long)__double_as_longlong(err.value()));
         __syncthreads();  // every thread has left the inverse FFT's exchange buffer
         if (t == 0) {
             const unsigned long long eb = s_err;
@@ -274,25 +258,27 @@ __global__ void __launch_bounds__(large_row_threads(LOG_C, G), large_row_min_blo
             for (int i = 0; i < E; ++i) row0[tr + TR * i] = v[i];
         }
         {
-            const int a0 = job * G;
-            const int s0a = __ldg(A.sA + 2 * a0), s1a = __ldg(A.sA + 2 * a0 + 1);
             static_assert(C % T == 0, "whole columns per thread");
             LargeCarry in[C / T];
+            uint32_t kd[C / T];  // kinds of row 0, columns t + T k: value (t + T k) / TR of its thread
 #pragma unroll
-            for (int k = 0; k < C / T; ++k) in[k] = ld_carry(A.carry + (size_t)job * C + t + T * k);
+            for (int k = 0; k < C / T; ++k) {
+                in[k] = ld_carry(A.carry + (size_t)job * C + t + T * k);
+                const int i = t / TR + G * k;
+                kd[k] = __ldg(A.kinds + ((size_t)job * T + (t % TR) * G) * KW + i / 8) >> (4 * (i % 8));
+            }
             __syncthreads();
 #pragma unroll
             for (int k = 0; k < C / T; ++k) {
                 const int b = t + T * k;
-                const uint32_t kd = kind_at(s0a, s1a, b);
                 if (in[k].tag != ep + 1u) in[k] = wait_carry(A.carry + (size_t)job * C + b, ep + 1u, A.ctl, A.spin_limit);
                 double cin = in[k].c1;
                 if (job == 0 && b == 0) cin -= 2.0;  // the "- 2" of s^2 - 2 (digit 0)
                 const double2 x = row0[b];
                 double c, c2;
-                const double x0 = dsplit_e(x.x + cin, A.q + (int)(kd & 1u), c);
-                const double x1 = dsplit_e(x.y + c, A.q + (int)((kd >> 1) & 1u), c2);
-                row0[b] = make_double2(x0 + (double)in[k].c2, x1);
+                const double x0 = dsplit_k(x.x + cin, dq, kind_unit(kd[k], 0), c);
+                const double x1 = dsplit_k(x.y + c, dq, kind_unit(kd[k], 1), c2);
+                row0[b] = make_double2(x0 + i2d_shift(in[k].c2), x1);
                 hop3[b] = c2;
             }
         }
@@ -319,9 +305,8 @@ __global__ void __launch_bounds__(large_row_threads(LOG_C, G), large_row_min_blo
 #pragma unroll
     for (int i = 0; i < E; ++i) {
         const double wb = swB[tr + TR * i];
-        const uint32_t kd = (MODE == LARGE_INIT || !KEEP_KINDS) ? digit_kind(tr + TR * i) : (kinds[i / 8] >> (4 * (i % 8)));
-        v[i].x *= (wa0 * wb) * ((kd & 4u) ? 0.5 : 1.0);
-        v[i].y *= (wa1 * wb) * ((kd & 8u) ? 0.5 : 1.0);
+        v[i].x *= scale_down(wa0 * wb, kind(i, 2));
+        v[i].y *= scale_down(wa1 * wb, kind(i, 3));
     }
     // the first forward pass stores after a barrier: the first row's carry may still be read from
     // the exchange buffer
@@ -594,10 +579,37 @@ __global__ void __launch_bounds__(col_mixed_threads<R0, LOG_L>(), 1)
     if (cb == 0 && t == 0) atomicAdd(&A.ctl->epoch, 1u);
 }
 
+// LargeArgs::kinds: word w of thread t of tile k holds the kinds of that thread's values 8w .. 8w+7.
+// Digit 2m+e of (row a, column b) has weight exponent s = (sA(2a+e) + sB(b)) mod N; its bit 0 / 1: it
+// has q + 1 bits (s < p mod N); bit 2 / 3: sA + sB >= N.
+__global__ void fill_kinds(uint32_t* kinds, const int* __restrict__ sA, const int* __restrict__ sB, int N, int rem,
+                           int C, int G, int log_e, long long words) {
+    const long long w = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (w >= words) return;
+    const int KW = (1 << log_e) / 8, TR = C >> log_e, T = G * TR;
+    const int part = (int)(w % KW), t = (int)((w / KW) % T);
+    const int a = (int)(w / KW / T) * G + t % G;
+    const int s0a = sA[2 * a], s1a = sA[2 * a + 1];
+    uint32_t k = 0u;
+    for (int i = 0; i < 8; ++i) {
+        const int sb = sB[t / G + TR * (8 * part + i)];
+        const bool o0 = s0a + sb >= N, o1 = s1a + sb >= N;
+        const int s0 = o0 ? s0a + sb - N : s0a + sb, s1 = o1 ? s1a + sb - N : s1a + sb;
+        k |= ((uint32_t)(s0 < rem) | ((uint32_t)(s1 < rem) << 1) | ((uint32_t)o0 << 2) | ((uint32_t)o1 << 3)) << (4 * i);
+    }
+    kinds[w] = k;
+}
+cudaError_t launch_fill_kinds(uint32_t* kinds, const int* sA, const int* sB, int N, int rem, int C, int R, int g, int log_e,
+                              cudaStream_t st) {
+    const long long words = (long long)R * C / 8;
+    fill_kinds<<<(unsigned)((words + 255) / 256), 256, 0, st>>>(kinds, sA, sB, N, rem, C, g, log_e, words);
+    return cudaGetLastError();
+}
+
 template <int LOG_C, int G>
 static size_t row_smem() {
     using GC = SmallG<LOG_C, large_row_log_e(LOG_C, G), TW_FULL, (large_row_log_e(LOG_C, G) >= 4)>;
-    return sizeof(double2) * (large_row_slots(LOG_C, G) + twiddle_table_len<GC>()) + (2 * sizeof(double) + sizeof(int)) * GC::M;
+    return sizeof(double2) * (large_row_slots(LOG_C, G) + twiddle_table_len<GC>()) + 2 * sizeof(double) * GC::M;
 }
 
 // Shared-memory carve-out (percent of the SM's 228 KB) for `blocks` resident blocks of `bytes`

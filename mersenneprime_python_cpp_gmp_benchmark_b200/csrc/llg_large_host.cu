@@ -87,8 +87,8 @@ std::vector<double2> pass_twiddle_table(int log_l, int log_e) {
     return t;
 }
 
-std::vector<double2> mixed_twiddle_table(int r0, int log_l) {
-    std::vector<double2> t = pass_twiddle_table(log_l, 3);
+std::vector<double2> mixed_twiddle_table(int r0, int log_l, int log_e) {
+    std::vector<double2> t = pass_twiddle_table(log_l, log_e);
     const uint64_t L = 1ull << log_l, M = (uint64_t)r0 * L;
     const long double two_pi = 6.283185307179586476925286766559005768L;
     for (uint64_t k0 = 1; k0 < (uint64_t)r0; ++k0)
@@ -172,7 +172,7 @@ int large_pdl_late(uint64_t n) { return n > (1ull << 16) && n < (1ull << 21) ? 1
 
 LargeTest::~LargeTest() {
     if (exec) cudaGraphExecDestroy(exec);
-    void* ptrs[] = {V, carry, ctl, wrap_read, digits, errlog, qtwC, qtwR, qtwL, tw1, tw2, pos_of_c, wA, iwA, sA, wB, iwB, sB};
+    void* ptrs[] = {V, carry, ctl, wrap_read, digits, errlog, qtwC, qtwR, qtwL, tw1, tw2, pos_of_c, wA, iwA, sA, wB, iwB, sB, kinds};
     for (void* p : ptrs)
         if (p) cudaFree(p);
 }
@@ -245,6 +245,9 @@ cudaError_t LargeTest::init(uint64_t p_, uint64_t n, int log_c, int rows_) {
     if ((e = upload(&wB, hwB))) return e;
     if ((e = upload(&iwB, hiwB))) return e;
     if ((e = upload(&sB, hsB))) return e;
+    if ((e = cudaMalloc(&kinds, M / 8 * sizeof(uint32_t)))) return e;
+    if ((e = launch_fill_kinds(kinds, sA, sB, (int)N, (int)(p % N), C, R, rows, large_row_log_e(logC, rows), nullptr))) return e;
+    if ((e = cudaStreamSynchronize(nullptr))) return e;  // before any other stream reads them
     // state
     if ((e = cudaMalloc(&V, M * sizeof(double2)))) return e;
     // carry slots: one per tile plus slot 0 for the wrap-around job
@@ -269,10 +272,9 @@ cudaError_t LargeTest::init(uint64_t p_, uint64_t n, int log_c, int rows_) {
     A.pos_of_c = pos_of_c;
     A.wA = wA;
     A.iwA = iwA;
-    A.sA = sA;
     A.wB = wB;
     A.iwB = iwB;
-    A.sB = sB;
+    A.kinds = kinds;
     A.carry = carry;
     A.ctl = ctl;
     A.wrap_read = wrap_read;

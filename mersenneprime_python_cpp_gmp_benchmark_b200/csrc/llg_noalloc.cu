@@ -42,7 +42,7 @@ namespace llg {
 
 namespace {
 
-constexpr size_t kNoAllocScratchBytes = 640u * 1024u;  // covers N = 65,536 (about 609 KiB used)
+constexpr size_t kNoAllocScratchBytes = 640u * 1024u;  // covers N = 65,536 (about 625 KiB used)
 constexpr int kNoAllocMaxLog = 16;
 constexpr int kMaxDevices = 64;
 
@@ -65,7 +65,7 @@ struct TableKey {
 TableKey g_tables_for[kMaxDevices];
 
 struct Layout {
-    size_t V, carry, ctl, wrap_read, qtwC, qtwR, tw1, tw2, pos_of_c, wA, iwA, sA, wB, iwB, sB, end;
+    size_t V, carry, ctl, wrap_read, qtwC, qtwR, tw1, tw2, pos_of_c, wA, iwA, sA, wB, iwB, sB, kinds, end;
 };
 
 size_t up256(size_t x) { return (x + 255) & ~(size_t)255; }
@@ -93,6 +93,7 @@ Layout layout(int logN, int logC, int logR, int s) {
     L.wB = o; o = up256(o + C * sizeof(double));
     L.iwB = o; o = up256(o + C * sizeof(double));
     L.sB = o; o = up256(o + C * sizeof(int));
+    L.kinds = o; o = up256(o + M / 8 * sizeof(uint32_t));
     L.end = o;
     return L;
 }
@@ -159,7 +160,7 @@ extern "C" int llg_run_noalloc(uint64_t p, uint64_t iters, uint32_t n, int32_t* 
     const Layout L = layout(logN, logC, logR, s);
     if (L.end > kNoAllocScratchBytes) return set_error(LLG_E_UNSUPPORTED, "llg_run_noalloc: state exceeds the array");
 
-    if (L.end - L.qtwC > kStageBytes) return set_error(LLG_E_UNSUPPORTED, "llg_run_noalloc: tables exceed the host stage");
+    if (L.kinds - L.qtwC > kStageBytes) return set_error(LLG_E_UNSUPPORTED, "llg_run_noalloc: tables exceed the host stage");
 
     std::lock_guard<std::mutex> lk(g_noalloc_mx);
     int dev = 0;
@@ -183,7 +184,7 @@ extern "C" int llg_run_noalloc(uint64_t p, uint64_t iters, uint32_t n, int32_t* 
         g_tables_for[dev] = TableKey{};  // invalid until the upload below has completed
         const long double Nl = (long double)N;
         const size_t o = L.qtwC;
-        std::memset(g_stage, 0, L.end - o);
+        std::memset(g_stage, 0, L.kinds - o);
         stage_table<double2>(L.qtwC - o, qpad_len((uint32_t)C), [&](size_t i) { return padded_quarter_slot(C, i); });
         {  // the column pass's quarter table in the spread layout: entry r at qpad_s(r)
             double2* q = reinterpret_cast<double2*>(g_stage + (L.qtwR - o));
@@ -202,8 +203,12 @@ extern "C" int llg_run_noalloc(uint64_t p, uint64_t iters, uint32_t n, int32_t* 
                             [&](size_t i) { return (double)(exp2l(-(long double)sBb(i) / Nl) / (4.0L * (long double)M)); });
         stage_table<int>(L.sB - o, (size_t)C, [&](size_t i) { return (int)sBb(i); });
         // pageable source: the copy has consumed the stage once the stream has finished it
-        e = cudaMemcpyAsync(base + o, g_stage, L.end - o, cudaMemcpyHostToDevice, st);
-        count_h2d(L.end - o);
+        e = cudaMemcpyAsync(base + o, g_stage, L.kinds - o, cudaMemcpyHostToDevice, st);
+        count_h2d(L.kinds - o);
+        if (e == cudaSuccess)
+            e = launch_fill_kinds(reinterpret_cast<uint32_t*>(base + L.kinds), reinterpret_cast<const int*>(base + L.sA),
+                                  reinterpret_cast<const int*>(base + L.sB), (int)N, (int)(p & (N - 1)), C, R, kTileRows,
+                                  large_row_log_e(logC, kTileRows), st);
         if (e == cudaSuccess) e = cudaStreamSynchronize(st);
         if (e != cudaSuccess) {
             cudaStreamSynchronize(st);
@@ -222,10 +227,9 @@ extern "C" int llg_run_noalloc(uint64_t p, uint64_t iters, uint32_t n, int32_t* 
     A.pos_of_c = reinterpret_cast<const int*>(base + L.pos_of_c);
     A.wA = reinterpret_cast<const double*>(base + L.wA);
     A.iwA = reinterpret_cast<const double*>(base + L.iwA);
-    A.sA = reinterpret_cast<const int*>(base + L.sA);
     A.wB = reinterpret_cast<const double*>(base + L.wB);
     A.iwB = reinterpret_cast<const double*>(base + L.iwB);
-    A.sB = reinterpret_cast<const int*>(base + L.sB);
+    A.kinds = reinterpret_cast<const uint32_t*>(base + L.kinds);
     A.carry = reinterpret_cast<LargeCarry*>(base + L.carry);
     A.ctl = reinterpret_cast<LargeCtl*>(base + L.ctl);
     A.wrap_read = reinterpret_cast<unsigned*>(base + L.wrap_read);

@@ -143,7 +143,8 @@ __global__ void __launch_bounds__(SmallGeo<LOG_M, LE>::T, small_min_blocks(Small
         const uint32_t kd = (uint32_t)(s0 < rem) | ((uint32_t)(s1 < rem) << 1) | ((uint32_t)o0 << 2) | ((uint32_t)o1 << 3);
         kinds[i / 8] |= kd << (4 * (i % 8));
     }
-    auto kind = [&](int i) { return kinds[i / 8] >> (4 * (i % 8)); };
+    const DigitBase dq(q);
+    auto kind = [&](int i, int bit) { return kind_unit(kinds[i / 8], 4 * (i % 8) + bit); };
     // made opaque before each use: the weights and digit sizes derived from the kinds are then
     // formed where used, not hoisted into registers held across the transforms
     auto refresh_kinds = [&]() {
@@ -197,7 +198,8 @@ __global__ void __launch_bounds__(SmallGeo<LOG_M, LE>::T, small_min_blocks(Small
 
         // unweight, round, error, local carry (even -> odd digit); the carry-out of column i goes
         // to thread t+1 (lane shuffle) or, at a warp boundary, through cbuf after the barrier
-        double lerr = 0.0;
+        ErrMax err;
+        double lerr;
         int bad;
         refresh_kinds();
         if constexpr (W == 1) {
@@ -205,16 +207,16 @@ __global__ void __launch_bounds__(SmallGeo<LOG_M, LE>::T, small_min_blocks(Small
             double x0[E], x1[E], c[E];
 #pragma unroll
             for (int i = 0; i < E; ++i) {
-                const uint32_t kd = kind(i);
                 const double iw = iwB[i];
-                const double a = v[i].x * (iwA0 * iw) * ((kd & 4u) ? 2.0 : 1.0);
-                const double b = v[i].y * (iwA1 * iw) * ((kd & 8u) ? 2.0 : 1.0);
+                const double a = v[i].x * scale_up(iwA0 * iw, kind(i, 2));
+                const double b = v[i].y * scale_up(iwA1 * iw, kind(i, 3));
                 long long la, lb;
                 const double ra = round_shift(a, la), rb = round_shift(b, lb);
-                lerr = fmax(lerr, fmax(fabs(a - ra), fabs(b - rb)));
+                err.add(a - ra);
+                err.add(b - rb);
                 double cy;
-                x0[i] = dsplit_e(ra, q + (int)(kd & 1u), cy);
-                x1[i] = dsplit_e(rb + cy, q + (int)((kd >> 1) & 1u), c[i]);
+                x0[i] = dsplit_k(ra, dq, kind(i, 0), cy);
+                x1[i] = dsplit_k(rb + cy, dq, kind(i, 1), c[i]);
                 c[i] = __shfl_sync(wmask, c[i], (t + T - 1) & (T - 1));
             }
             const double wrap = c[E - 1];
@@ -224,9 +226,10 @@ __global__ void __launch_bounds__(SmallGeo<LOG_M, LE>::T, small_min_blocks(Small
 #pragma unroll
             for (int i = 0; i < E; ++i) {
                 double cy;
-                x0s[i] = d2i_exact(dsplit_e(x0[i] + c[i], q + (int)(kind(i) & 1u), cy));
+                x0s[i] = d2i_exact(dsplit_k(x0[i] + c[i], dq, kind(i, 0), cy));
                 x1s[i] = d2i_exact(x1[i] + cy);
             }
+            lerr = err.value();
             if (errlog) {
                 atomicMax(&serr[it & 1], (unsigned long long)__double_as_longlong(lerr));
                 __syncwarp(wmask);
@@ -235,28 +238,28 @@ __global__ void __launch_bounds__(SmallGeo<LOG_M, LE>::T, small_min_blocks(Small
         } else {
 #pragma unroll
             for (int i = 0; i < E; ++i) {
-                const uint32_t kd = kind(i);
                 const double iw = iwB[i];
-                const double a = v[i].x * (iwA0 * iw) * ((kd & 4u) ? 2.0 : 1.0);
-                const double b = v[i].y * (iwA1 * iw) * ((kd & 8u) ? 2.0 : 1.0);
+                const double a = v[i].x * scale_up(iwA0 * iw, kind(i, 2));
+                const double b = v[i].y * scale_up(iwA1 * iw, kind(i, 3));
                 long long la, lb;
                 const double ra = round_shift(a, la), rb = round_shift(b, lb);
-                lerr = fmax(lerr, fmax(fabs(a - ra), fabs(b - rb)));
-                const int b0 = q + (int)(kd & 1u), b1 = q + (int)((kd >> 1) & 1u);  // digit sizes
+                err.add(a - ra);
+                err.add(b - rb);
                 double c;
-                double x0 = dsplit_e(ra, b0, c);
-                const double x1 = dsplit_e(rb + c, b1, c);
+                double x0 = dsplit_k(ra, dq, kind(i, 0), c);
+                const double x1 = dsplit_k(rb + c, dq, kind(i, 1), c);
                 const double cout = c;
                 if (lane == 31) cbuf[warp * E + i] = cout;
                 const double cin = __shfl_up_sync(0xffffffffu, cout, 1);
                 if (lane != 0) {
-                    x0 = dsplit_e(x0 + cin, b0, c);
+                    x0 = dsplit_k(x0 + cin, dq, kind(i, 0), c);
                     x1s[i] = d2i_exact(x1 + c);
                 } else {
                     x1s[i] = d2i_exact(x1);
                 }
                 x0s[i] = d2i_exact(x0);
             }
+            lerr = err.value();
             if (errlog) atomicMax(&serr[it & 1], (unsigned long long)__double_as_longlong(lerr));
             bad = __syncthreads_or(lerr > abort_err);
         }
@@ -273,7 +276,7 @@ __global__ void __launch_bounds__(SmallGeo<LOG_M, LE>::T, small_min_blocks(Small
                                         : cbuf[(W - 1) * E + ((i + E - 1) % E)];  // m-1 wraps at m=0
                 if (t == 0 && i == 0) cin -= 2.0;  // the "- 2" of s^2 - 2
                 double c;
-                x0s[i] = d2i_exact(dsplit_e((double)x0s[i] + cin, q + (int)(kind(i) & 1u), c));
+                x0s[i] = d2i_exact(dsplit_k((double)x0s[i] + cin, dq, kind(i, 0), c));
                 x1s[i] += (int)c;
             }
         }
@@ -286,10 +289,9 @@ __global__ void __launch_bounds__(SmallGeo<LOG_M, LE>::T, small_min_blocks(Small
         refresh_kinds();
 #pragma unroll
         for (int i = 0; i < E; ++i) {
-            const uint32_t kd = kind(i);
             const double w = wB[i];
-            v[i].x = i2d_shift(x0s[i]) * (wA0 * w) * ((kd & 4u) ? 0.5 : 1.0);
-            v[i].y = i2d_shift(x1s[i]) * (wA1 * w) * ((kd & 8u) ? 0.5 : 1.0);
+            v[i].x = i2d_shift(x0s[i]) * scale_down(wA0 * w, kind(i, 2));
+            v[i].y = i2d_shift(x1s[i]) * scale_down(wA1 * w, kind(i, 3));
         }
     }
 

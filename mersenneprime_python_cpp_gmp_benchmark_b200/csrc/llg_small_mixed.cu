@@ -8,7 +8,7 @@
 // transform is split as R0 x L (decimation in frequency, m = n + L r, k = R0 k' + k0):
 //   X[R0 k' + k0] = sum_n w_L^{n k'} w_M^{n k0} sum_r u[n + L r] w_R0^{r k0}
 // so a squaring is: the radix-R0 step with the twiddle w_M^{n k0}; R0 independent L-point FFTs (the
-// power-of-two radix-8 passes, one segment of L/8 threads each, named barriers per segment); the
+// power-of-two radix passes, one segment of L/8 or L/16 threads each, named barriers per segment); the
 // real-FFT split and square on the pair (k, M - k), which pairs segment k0 with segment R0 - k0; the
 // inverse L-point FFTs; the conjugate twiddle and the inverse radix-R0 step; then unweight, round,
 // carry and weight in registers.
@@ -24,11 +24,11 @@
 //
 // Twiddles are read where they are used: the passes' in pass order (TW_PASS), w_M^{n k0} as a table
 // of R0 - 1 rows over n, the radix-R0 constants as immediates. Against quarter-wave tables with a fold
-// and factored products, us a squaring: N = 3072 5.65 -> 5.35 for one test, 28.9 -> 26.4 for 1184; 5120
-// 7.2 -> 6.3, 50.3 -> 45.0; 6144 10.2 -> 9.5, 32.1 -> 32.0 (592 tests); 10240 and 12288, which had read
-// R0 values from shared memory for every output of a radix-R0 step, 16.5 -> 13.5 and 17.4 -> 16.9,
-// 33.3 -> 27.3 and 35.1 -> 34.5 (296 tests). Fewer FP64 instructions and no integer fold; barriers
-// and the latency of the shared-memory exchanges bound it now.
+// and factored products, us a squaring: N = 3072 5.65 -> 4.27 for one test, 28.9 -> 25.7 for 1184; 5120
+// 7.2 -> 5.9, 50.3 -> 43.9; 6144 10.2 -> 7.8, 32.1 -> 28.7 (592 tests); 10240 and 12288, which had read R0
+// values from shared memory for every output of a radix-R0 step, 16.5 -> 12.3 and 17.4 -> 15.0, 33.3
+// -> 24.9 and 35.1 -> 30.6 (296 tests). Fewer FP64 instructions and no integer fold; barriers and the
+// latency of the shared-memory exchanges bound it now.
 
 #include <cuda_runtime.h>
 
@@ -40,17 +40,17 @@
 
 namespace llg {
 
-template <int R0_, int LOG_L>
+// LE: log2 of the values per FFT thread; MINB: blocks per SM the kernel is built for (mixed_form)
+template <int R0_, int LOG_L, int LE_, int MINB_>
 struct MixedGeom {
-    using GL = SmallG<LOG_L, 3, TW_PASS, true>;
+    static constexpr int LE = LE_, MINB = MINB_;
+    using GL = SmallG<LOG_L, LE, TW_PASS, true>;
     static constexpr int R0 = R0_;
     static constexpr int L = GL::M, TL = GL::T, E = GL::E;
     static constexpr int M = R0 * L, N = 2 * M;
-    static constexpr int NPT = R0 == 5 ? 2 : 4;  // columns n per digit thread
+    static constexpr int NPT = (R0 == 5 ? 2 : 4) << (LE - 3);  // columns n per digit thread
     static constexpr int TA = L / NPT, CA = NPT * R0, WA = TA / 32;
     static constexpr int T = R0 * TL;
-    // blocks per SM the kernel is built for
-    static constexpr int MINB = T <= 192 ? 4 : T <= 384 ? 2 : 1;
     static constexpr int PADL = L + L / E;                       // exchange slots of one segment
     static constexpr int QL = (int)twiddle_table_len<GL>();      // pass twiddles of the L-point FFT
     static constexpr int NB = E / GL::RLAST;                     // split twiddles a thread reads
@@ -96,15 +96,15 @@ __device__ __forceinline__ void dft_r0(double2 (&x)[R0]) {
     x[0] = x0;
 }
 
-template <int R0, int LOG_L>
-__global__ void __launch_bounds__(MixedGeom<R0, LOG_L>::T, MixedGeom<R0, LOG_L>::MINB)
+template <int R0, int LOG_L, int LE, int MINB>
+__global__ void __launch_bounds__(MixedGeom<R0, LOG_L, LE, MINB>::T, MINB)
     ll_small_fp64_mixed(const SmallJob* __restrict__ jobs, const double2* __restrict__ qtw_g,
                         int64_t* __restrict__ digits_out, SmallResult* __restrict__ results,
                         float* __restrict__ errlog, double abort_err) {
-    using MG = MixedGeom<R0, LOG_L>;
+    using MG = MixedGeom<R0, LOG_L, LE, MINB>;
     using GL = typename MG::GL;
     constexpr int L = MG::L, TL = MG::TL, E = MG::E, M = MG::M, N = MG::N, T = MG::T, TA = MG::TA,
-                  CA = MG::CA, WA = MG::WA, NPT = MG::NPT, PADL = MG::PADL, QL = MG::QL, PL = 3;
+                  CA = MG::CA, WA = MG::WA, NPT = MG::NPT, PADL = MG::PADL, QL = MG::QL, PL = LE;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     double2* bufs = reinterpret_cast<double2*>(smem_raw);  // R0 segment buffers of PADL slots
     double2* qtwL = bufs + R0 * PADL;                        // pass twiddles of the L-point FFT
@@ -173,7 +173,8 @@ __global__ void __launch_bounds__(MixedGeom<R0, LOG_L>::T, MixedGeom<R0, LOG_L>:
         const uint32_t kd = (uint32_t)(s0 < rem) | ((uint32_t)(s1 < rem) << 1) | ((uint32_t)o0 << 2) | ((uint32_t)o1 << 3);
         kinds[c / 8] |= kd << (4 * (c % 8));
     }
-    auto kind = [&](int c) { return kinds[c / 8] >> (4 * (c % 8)); };
+    const DigitBase dq(q);
+    auto kind = [&](int c, int bit) { return kind_unit(kinds[c / 8], 4 * (c % 8) + bit); };
     // made opaque before each use: the weights and digit sizes derived from the kinds are then
     // formed where used, not hoisted into registers held across the transforms
     auto refresh_kinds = [&]() {
@@ -205,10 +206,9 @@ __global__ void __launch_bounds__(MixedGeom<R0, LOG_L>::T, MixedGeom<R0, LOG_L>:
 #pragma unroll
                 for (int r = 0; r < R0; ++r) {
                     const int c = i + NPT * r;
-                    const uint32_t kd = kind(c);
-                    const double w = wB[c];
-                    z[r] = make_double2(i2d_shift(x0s[c]) * (wA0 * w) * ((kd & 4u) ? 0.5 : 1.0),
-                                        i2d_shift(x1s[c]) * (wA1 * w) * ((kd & 8u) ? 0.5 : 1.0));
+                        const double w = wB[c];
+                    z[r] = make_double2(i2d_shift(x0s[c]) * scale_down(wA0 * w, kind(c, 2)),
+                                        i2d_shift(x1s[c]) * scale_down(wA1 * w, kind(c, 3)));
                 }
                 dft_r0<R0, false>(z);
                 bufs[physp<PL>(n)] = z[0];
@@ -258,7 +258,7 @@ __global__ void __launch_bounds__(MixedGeom<R0, LOG_L>::T, MixedGeom<R0, LOG_L>:
 
         // ---- inverse radix-R0 DFT back to the thread's columns, then unweight, round and carry
         //      each column (the columns' carries are independent until the exchange below) ----
-        double lerr = 0.0;
+        ErrMax err;
         refresh_kinds();
         if (holds) {
 #pragma unroll
@@ -271,22 +271,21 @@ __global__ void __launch_bounds__(MixedGeom<R0, LOG_L>::T, MixedGeom<R0, LOG_L>:
 #pragma unroll
                 for (int r = 0; r < R0; ++r) {
                 const int c = i + NPT * r;
-                const uint32_t kd = kind(c);
                 const double iw = iwB[c];
-                const double a = z[r].x * (iwA0 * iw) * ((kd & 4u) ? 2.0 : 1.0);
-                const double b = z[r].y * (iwA1 * iw) * ((kd & 8u) ? 2.0 : 1.0);
+                const double a = z[r].x * scale_up(iwA0 * iw, kind(c, 2));
+                const double b = z[r].y * scale_up(iwA1 * iw, kind(c, 3));
                 long long la, lb;
                 const double ra = round_shift(a, la), rb = round_shift(b, lb);
-                lerr = fmax(lerr, fmax(fabs(a - ra), fabs(b - rb)));
-                const int b0 = q + (int)(kd & 1u), b1 = q + (int)((kd >> 1) & 1u);  // digit sizes
+                err.add(a - ra);
+                err.add(b - rb);
                 double cy;
-                double x0 = dsplit_e(ra, b0, cy);
-                const double x1 = dsplit_e(rb + cy, b1, cy);
+                double x0 = dsplit_k(ra, dq, kind(c, 0), cy);
+                const double x1 = dsplit_k(rb + cy, dq, kind(c, 1), cy);
                 const double cout = cy;
                 if (lane == 31) cbuf[warp * CA + c] = cout;
                 const double cin = __shfl_up_sync(0xffffffffu, cout, 1);
                 if (lane != 0) {
-                    x0 = dsplit_e(x0 + cin, b0, cy);
+                    x0 = dsplit_k(x0 + cin, dq, kind(c, 0), cy);
                     x1s[c] = d2i_exact(x1 + cy);
                 } else {
                     x1s[c] = d2i_exact(x1);
@@ -295,6 +294,7 @@ __global__ void __launch_bounds__(MixedGeom<R0, LOG_L>::T, MixedGeom<R0, LOG_L>:
                 }
             }
         }
+        const double lerr = err.value();
         maxerr = fmax(maxerr, lerr);
         if (errlog) atomicMax(&serr[it & 1], (unsigned long long)__double_as_longlong(lerr));
         const int bad = __syncthreads_or(lerr > abort_err);
@@ -311,7 +311,7 @@ __global__ void __launch_bounds__(MixedGeom<R0, LOG_L>::T, MixedGeom<R0, LOG_L>:
                 double cin = (warp > 0) ? cbuf[(warp - 1) * CA + c] : cbuf[(WA - 1) * CA + ((c + CA - 1) % CA)];
                 if (t == 0 && c == 0) cin -= 2.0;  // the "- 2" of s^2 - 2
                 double cy;
-                x0s[c] = d2i_exact(dsplit_e((double)x0s[c] + cin, q + (int)(kind(c) & 1u), cy));
+                x0s[c] = d2i_exact(dsplit_k((double)x0s[c] + cin, dq, kind(c, 0), cy));
                 x1s[c] += (int)cy;
             }
         }
@@ -349,20 +349,20 @@ __global__ void __launch_bounds__(MixedGeom<R0, LOG_L>::T, MixedGeom<R0, LOG_L>:
     }
 }
 
-template <int R0, int LOG_L>
+template <int R0, int LOG_L, int LE, int MINB>
 static cudaError_t launch_mixed_t(const SmallJob* jobs, int njobs, const double2* qtw, int64_t* digits,
                                   SmallResult* results, float* errlog, double abort_err, cudaStream_t st) {
-    using MG = MixedGeom<R0, LOG_L>;
+    using MG = MixedGeom<R0, LOG_L, LE, MINB>;
     const size_t smem = MG::smem();
     static PerDeviceOnce configured;
     if (!configured.done()) {
-        cudaError_t e = cudaFuncSetAttribute(ll_small_fp64_mixed<R0, LOG_L>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaError_t e = cudaFuncSetAttribute(ll_small_fp64_mixed<R0, LOG_L, LE, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(ll_small_fp64_mixed<R0, LOG_L>, cudaFuncAttributePreferredSharedMemoryCarveout, kWholeTestCarveout);
+            e = cudaFuncSetAttribute(ll_small_fp64_mixed<R0, LOG_L, LE, MINB>, cudaFuncAttributePreferredSharedMemoryCarveout, kWholeTestCarveout);
         if (e != cudaSuccess) return e;
         configured.mark();
     }
-    ll_small_fp64_mixed<R0, LOG_L><<<njobs, MG::T, smem, st>>>(jobs, qtw, digits, results, errlog, abort_err);
+    ll_small_fp64_mixed<R0, LOG_L, LE, MINB><<<njobs, MG::T, smem, st>>>(jobs, qtw, digits, results, errlog, abort_err);
     return cudaGetLastError();
 }
 
@@ -377,24 +377,36 @@ bool mixed_length_supported(uint32_t n, int* r0, int* log_l) {
     return false;
 }
 
+// Values a thread and blocks per SM, by length and whether each test has its SM to itself. Measured,
+// us a squaring: one test, N = 3072 4.27 (8 values, one block per SM; 5.10 built for four, 8.0 with 16
+// values), 5120 5.94 (6.20 for two, 8.5), 6144 7.79 (9.8, 9.8); more tests than SMs: N = 3072 13.1 (8
+// values, four blocks; 592 tests; 17.5 with 16), 5120 22.1 (two blocks; 25.1), 6144 28.7 (16 values, two
+// blocks; 32.5 with 8). One block fits an SM at 10240 and 12288: 16 values, 12.3 and 15.0 (8: 13.1, 17.2).
+int small_fp64_mixed_log_e(uint32_t n, int njobs) {
+    int r0 = 0, l = 0;
+    if (!mixed_length_supported(n, &r0, &l)) return 0;
+    if (l == 9) return 3;
+    return r0 == 3 && l == 10 && njobs <= device_sms() ? 3 : 4;
+}
+
 cudaError_t launch_small_fp64_mixed(uint32_t n, const SmallJob* jobs, int njobs, const double2* qtw,
                                     int64_t* digits, SmallResult* results, float* errlog,
                                     double abort_err, cudaStream_t st) {
-    int r0 = 0, l = 0;
-    if (!mixed_length_supported(n, &r0, &l)) return cudaErrorInvalidValue;
-    if (r0 == 3) {
-        switch (l) {
-            case 9: return launch_mixed_t<3, 9>(jobs, njobs, qtw, digits, results, errlog, abort_err, st);
-            case 10: return launch_mixed_t<3, 10>(jobs, njobs, qtw, digits, results, errlog, abort_err, st);
-            case 11: return launch_mixed_t<3, 11>(jobs, njobs, qtw, digits, results, errlog, abort_err, st);
-        }
-    } else {
-        switch (l) {
-            case 9: return launch_mixed_t<5, 9>(jobs, njobs, qtw, digits, results, errlog, abort_err, st);
-            case 10: return launch_mixed_t<5, 10>(jobs, njobs, qtw, digits, results, errlog, abort_err, st);
-        }
+    const bool alone = njobs <= device_sms();
+    switch (n) {
+        case 3072:
+            return alone ? launch_mixed_t<3, 9, 3, 1>(jobs, njobs, qtw, digits, results, errlog, abort_err, st)
+                         : launch_mixed_t<3, 9, 3, 4>(jobs, njobs, qtw, digits, results, errlog, abort_err, st);
+        case 5120:
+            return alone ? launch_mixed_t<5, 9, 3, 1>(jobs, njobs, qtw, digits, results, errlog, abort_err, st)
+                         : launch_mixed_t<5, 9, 3, 2>(jobs, njobs, qtw, digits, results, errlog, abort_err, st);
+        case 6144:
+            return alone ? launch_mixed_t<3, 10, 3, 1>(jobs, njobs, qtw, digits, results, errlog, abort_err, st)
+                         : launch_mixed_t<3, 10, 4, 2>(jobs, njobs, qtw, digits, results, errlog, abort_err, st);
+        case 10240: return launch_mixed_t<5, 10, 4, 1>(jobs, njobs, qtw, digits, results, errlog, abort_err, st);
+        case 12288: return launch_mixed_t<3, 11, 4, 1>(jobs, njobs, qtw, digits, results, errlog, abort_err, st);
+        default: return cudaErrorInvalidValue;
     }
-    return cudaErrorInvalidValue;
 }
 
 }  // namespace llg

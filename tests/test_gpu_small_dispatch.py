@@ -1,14 +1,13 @@
 """The whole-test FP64 kernel takes more threads a test when each test has its SM to itself: both
-forms at every power-of-two length, full residues against each other and the oracle, and the
+forms at every length, full residues against each other and the oracle, and the
 per-squaring round-off log of the form that runs in one warp."""
 import pytest
 
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("logn", range(5, 14))
-def test_alone_and_batch_forms_agree(gpu, oracle, logn):
-    n = 1 << logn
+@pytest.mark.parametrize("n", [1 << k for k in range(5, 14)] + [3072, 5120, 6144, 10240, 12288])
+def test_alone_and_batch_forms_agree(gpu, oracle, n):
     sms = gpu.device_info()[1]
     lo = max(257, int(17.2 * n))
     ps = [p for p in range(lo | 1, 18 * n) if p % 2 and gpu.fft_length(p) == n]
