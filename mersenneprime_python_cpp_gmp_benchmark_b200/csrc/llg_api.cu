@@ -1258,7 +1258,7 @@ int llg_get_large_split(int log_n, int* rows) {
     if (!large_length_supported(log_n)) return -1;
     const int v = g_large_shape[log_n].load();
     const int lc = v >= 0 ? shape_log_c(v) : large_default_log_c(log_n);
-    if (rows) *rows = v >= 0 ? shape_rows(v) : large_rows_per_block(lc);
+    if (rows) *rows = v >= 0 ? shape_rows(v) : large_default_rows(log_n);
     return lc;
 }
 

@@ -16,6 +16,7 @@ bool large_length_supported(int log_n);
 // N = R0 2^k two-pass lengths (R0 = 3, 5; k = 18 .. 21): R0 and the log2 row length they use.
 bool large_mixed_length_supported(uint64_t n, int* r0, int* log_c);
 int large_default_log_c(int log_n);
+int large_default_rows(int log_n);
 int large_pdl_late(uint64_t n);  // LargeArgs::pdl_late at length n
 bool large_split_supported(int log_n, int log_c, int rows);
 int set_error(int code, const char* msg);  // records this thread's llg_last_error() text

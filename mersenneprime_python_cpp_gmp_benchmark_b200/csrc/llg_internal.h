@@ -133,12 +133,16 @@ __host__ __device__
 #endif
 constexpr int large_rows_per_block(int log_c) { return log_c >= 11 ? 2 : 4; }
 constexpr unsigned long long kSpinLimit = 1ull << 22;  // x ~64 ns sleeps: ~0.3 s, then give up + flag
-// log2 of the complex values per thread in the row pass of g rows of 2^log_c complex: 8 values
-// (radix-8 passes, two or more blocks per SM) for rows of up to 2^9, 16 (radix-16 passes) for longer
+// log2 of the complex values per thread in the row pass of g rows of 2^log_c complex: 16 for rows
+// longer than 2^9, 8 up to there (two or more blocks per SM), 4 in the tiles of the shortest lengths,
+// whose passes are a few blocks of a few warps (N = 2^14 7.2 -> 6.2 us a squaring, 2^16 7.6 -> 7.0, 2^18 9.6
+// -> 8.9; rows of 2^8 by 4, which the longer lengths use, were slower: 2^20 18.3 -> 21.0)
 #ifdef __CUDACC__
 __host__ __device__
 #endif
-constexpr int large_row_log_e(int log_c, int g) { return (void)g, log_c <= 9 ? 3 : 4; }
+constexpr int large_row_log_e(int log_c, int g) {
+    return log_c > 9 ? 4 : ((log_c <= 7 && g <= 4) || (log_c == 8 && g == 2)) ? 2 : 3;
+}
 
 struct LargeCtl {
     unsigned long long tickets;      // FP64 row-pass tickets taken since the start
@@ -190,7 +194,7 @@ struct LargeArgs {
     const double* iwA;        // [2R] 2^(-sA/N)
     const double* wB;         // [C] 2^(sB/N)
     const double* iwB;        // [C] 2^(-sB/N) / (4M)
-    const uint32_t* kinds;    // digit kinds by tile and thread (fill_kinds): N / 16 words
+    const uint32_t* kinds;    // digit kinds by tile and thread (fill_kinds)
     LargeCarry* carry;        // [nblocks + 1][C] carry-outs of a tile's last row: slot 0 the
                               // wrap-around job's (row R-1, one column on), k + 1 tile k's
     LargeCtl* ctl;
@@ -208,8 +212,9 @@ struct LargeArgs {
     int logN;                 // log2 N for a power of two
 };
 
+constexpr size_t large_kind_words(size_t rc, int log_e) { return rc >> (log_e < 3 ? log_e : 3); }
 // Fills LargeArgs::kinds for tiles of g rows with 2^log_e values a thread from the weight exponents sA
-// ([2R] (-(2a+e) p) mod N) and sB ([C] (-2Rb p) mod N); R C / 8 words.
+// ([2R] (-(2a+e) p) mod N) and sB ([C] (-2Rb p) mod N); large_kind_words of them.
 cudaError_t launch_fill_kinds(uint32_t* kinds, const int* sA, const int* sB, int N, int rem, int C, int R, int g, int log_e,
                               cudaStream_t st);
 // Row pass; grid > 0 overrides the block count (nblocks, + 1 for the wrap-around job unless INIT).

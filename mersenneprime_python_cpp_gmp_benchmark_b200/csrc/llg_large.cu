@@ -170,7 +170,7 @@ __global__ void __launch_bounds__(large_row_threads(LOG_C, G), large_row_min_blo
     const bool wrap_job = job < 0;
     const int a = (wrap_job ? R - G : job * G) + ra;  // this thread's row
     // the digit kinds of this thread's E values, 4 bits each (kind_unit)
-    constexpr int KW = E / 8;
+    constexpr int KW = E < 8 ? 1 : E / 8;
     uint32_t kinds[KW];
 #pragma unroll
     for (int w = 0; w < KW; ++w) kinds[w] = __ldg(A.kinds + ((size_t)(a / G) * T + t) * KW + w);
@@ -579,20 +579,22 @@ __global__ void __launch_bounds__(col_mixed_threads<R0, LOG_L>(), 1)
     if (cb == 0 && t == 0) atomicAdd(&A.ctl->epoch, 1u);
 }
 
-// LargeArgs::kinds: word w of thread t of tile k holds the kinds of that thread's values 8w .. 8w+7.
+// LargeArgs::kinds: word w of thread t of tile k holds the kinds of that thread's values 8w .. 8w+7 (at 4 values a
+// thread, of its 4).
 // Digit 2m+e of (row a, column b) has weight exponent s = (sA(2a+e) + sB(b)) mod N; its bit 0 / 1: it
 // has q + 1 bits (s < p mod N); bit 2 / 3: sA + sB >= N.
 __global__ void fill_kinds(uint32_t* kinds, const int* __restrict__ sA, const int* __restrict__ sB, int N, int rem,
                            int C, int G, int log_e, long long words) {
     const long long w = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (w >= words) return;
-    const int KW = (1 << log_e) / 8, TR = C >> log_e, T = G * TR;
+    const int KW = log_e < 3 ? 1 : (1 << log_e) / 8, VW = log_e < 3 ? 1 << log_e : 8;  // words, values a word
+    const int TR = C >> log_e, T = G * TR;
     const int part = (int)(w % KW), t = (int)((w / KW) % T);
     const int a = (int)(w / KW / T) * G + t % G;
     const int s0a = sA[2 * a], s1a = sA[2 * a + 1];
     uint32_t k = 0u;
-    for (int i = 0; i < 8; ++i) {
-        const int sb = sB[t / G + TR * (8 * part + i)];
+    for (int i = 0; i < VW; ++i) {
+        const int sb = sB[t / G + TR * (VW * part + i)];
         const bool o0 = s0a + sb >= N, o1 = s1a + sb >= N;
         const int s0 = o0 ? s0a + sb - N : s0a + sb, s1 = o1 ? s1a + sb - N : s1a + sb;
         k |= ((uint32_t)(s0 < rem) | ((uint32_t)(s1 < rem) << 1) | ((uint32_t)o0 << 2) | ((uint32_t)o1 << 3)) << (4 * i);
@@ -601,7 +603,7 @@ __global__ void fill_kinds(uint32_t* kinds, const int* __restrict__ sA, const in
 }
 cudaError_t launch_fill_kinds(uint32_t* kinds, const int* sA, const int* sB, int N, int rem, int C, int R, int g, int log_e,
                               cudaStream_t st) {
-    const long long words = (long long)R * C / 8;
+    const long long words = (long long)large_kind_words((size_t)R * C, log_e);
     fill_kinds<<<(unsigned)((words + 255) / 256), 256, 0, st>>>(kinds, sA, sB, N, rem, C, g, log_e, words);
     return cudaGetLastError();
 }

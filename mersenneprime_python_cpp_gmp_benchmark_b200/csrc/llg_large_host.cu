@@ -146,13 +146,14 @@ bool large_mixed_length_supported(uint64_t n, int* r0, int* log_c) {
     return false;
 }
 
-// Row length (2^log_c complex values) of the two-pass FP64 engine at N = 2^log_n by default, in
-// tiles of large_rows_per_block rows: the fastest of the supported shapes on a B200. us a squaring,
-// this shape / the default before: 2^14 7.3 / 9.8, 2^15 7.2 / 12.3, 2^16 7.9 / 13.1, 2^17 9.0 / 13.7, 2^18
-// 10.1 / 26.3, 2^19 12.3 / 29.9, 2^20 18.9 / 34.5, 2^21 32.9 / 41.2, 2^22 65.6 / 76.5, 2^23 145.6 / 156.3.
+// Row length (2^log_c complex values) and rows per tile of the two-pass FP64 engine at N = 2^log_n by
+// default: the fastest of the supported shapes on a B200. us a squaring, this shape / the default
+// before: 2^14 6.2 / 9.8, 2^15 6.4 / 12.3, 2^16 7.0 / 13.1, 2^17 7.9 / 13.7, 2^18 8.9 / 26.3, 2^19 12.1 / 29.9, 2^20
+// 18.3 / 34.5, 2^21 32.3 / 41.2, 2^22 64.7 / 76.5, 2^23 138 / 156.
 int large_default_log_c(int log_n) {
     return log_n <= 15 ? 6 : log_n <= 17 ? 7 : log_n == 19 ? 9 : log_n <= 21 ? 8 : log_n == 22 ? 9 : 10;
 }
+int large_default_rows(int log_n) { return log_n >= 16 && log_n <= 18 ? 2 : 4; }
 
 // Shapes of M = N/2 = 2^log_r rows of 2^log_c values (row blocks of `rows` rows) that the
 // kernels implement: rows of 2^6 .. 2^11, columns of 2^7 .. 2^12; rows == 0: the default.
@@ -165,9 +166,8 @@ bool large_split_supported(int log_n, int log_c, int rows) {
 // Whether a pass lets the next one launch at its end rather than its start. Blocks launched early go
 // to the SMs that are free at that moment, several to one, and a pass of about one wave then runs
 // as long as its fullest SM; from several waves on the early start fills the last wave, and the
-// shortest passes are mostly launch latency. Measured at the default shapes, us a squaring, start /
-// end: N = 2^14 7.3 / 8.4, 2^16 7.9 / 9.0, 2^17 10.2 / 9.0, 2^18 13.9 / 10.1, 2^20 27 / 19, 2^21 32.9 / 33.2,
-// 2^23 145.6 / 149.7; 3 x 2^18 28.2 / 21.0, 5 x 2^19 58.8 / 60.1, 5 x 2^20 115.2 / 116.4.
+// shortest passes are mostly launch latency. Measured, us a squaring, start / end: N = 2^14 7.3 / 8.4,
+// 2^16 7.9 / 9.0, 2^17 10.2 / 9.0, 2^18 13.9 / 10.1, 2^20 27 / 19, 2^21 32.9 / 33.2, 2^23 145.6 / 149.7; 3 x 2^18 28.2 / 21.0, 5 x 2^19 58.8 / 60.1, 5 x 2^20 115.2 / 116.4.
 int large_pdl_late(uint64_t n) { return n > (1ull << 16) && n < (1ull << 21) ? 1 : 0; }
 
 LargeTest::~LargeTest() {
@@ -198,7 +198,7 @@ cudaError_t LargeTest::init(uint64_t p_, uint64_t n, int log_c, int rows_) {
         if ((1ull << logN) != N) return cudaErrorInvalidValue;
         logC = large_default_log_c(logN);
         if (log_c >= 0) logC = log_c;
-        rows = rows_ ? rows_ : large_rows_per_block(logC);
+        rows = rows_ ? rows_ : log_c >= 0 ? large_rows_per_block(logC) : large_default_rows(logN);
         if (!large_split_supported(logN, logC, rows)) return cudaErrorInvalidValue;
         logR = logN - 1 - logC;
         C = 1 << logC;
@@ -245,7 +245,7 @@ cudaError_t LargeTest::init(uint64_t p_, uint64_t n, int log_c, int rows_) {
     if ((e = upload(&wB, hwB))) return e;
     if ((e = upload(&iwB, hiwB))) return e;
     if ((e = upload(&sB, hsB))) return e;
-    if ((e = cudaMalloc(&kinds, M / 8 * sizeof(uint32_t)))) return e;
+    if ((e = cudaMalloc(&kinds, large_kind_words(M, large_row_log_e(logC, rows)) * sizeof(uint32_t)))) return e;
     if ((e = launch_fill_kinds(kinds, sA, sB, (int)N, (int)(p % N), C, R, rows, large_row_log_e(logC, rows), nullptr))) return e;
     if ((e = cudaStreamSynchronize(nullptr))) return e;  // before any other stream reads them
     // state

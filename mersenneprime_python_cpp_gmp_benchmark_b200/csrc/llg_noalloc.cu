@@ -93,7 +93,7 @@ Layout layout(int logN, int logC, int logR, int s) {
     L.wB = o; o = up256(o + C * sizeof(double));
     L.iwB = o; o = up256(o + C * sizeof(double));
     L.sB = o; o = up256(o + C * sizeof(int));
-    L.kinds = o; o = up256(o + M / 8 * sizeof(uint32_t));
+    L.kinds = o; o = up256(o + large_kind_words(M, large_row_log_e(logC, kTileRows)) * sizeof(uint32_t));
     L.end = o;
     return L;
 }
