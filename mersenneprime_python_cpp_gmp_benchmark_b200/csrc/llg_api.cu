@@ -28,10 +28,6 @@
 
 namespace {
 
-// padded layout of the NTT twiddle tables (same as gl::qpad8 in llg_ntt.cuh)
-constexpr uint32_t gl_qpad8(uint32_t r) { return r + (r >> 4); }
-constexpr uint32_t gl_qpad8_len(uint32_t qm) { return qm + (qm >> 4) + 1; }
-
 using namespace llg;
 
 thread_local std::string t_last_error;
@@ -67,7 +63,7 @@ constexpr int kSmallLogMax = 13;  // N = 8192
 
 struct DeviceTables {
     std::map<uint32_t, double2*> qtw;      // twiddles of the FP64 kernels, by get_table's key
-    uint64_t* nqtw[kSmallLogMax + 1] = {}; // NTT: padded twiddle table of the N-point transform
+    uint64_t* nqtw[kSmallLogMax + 1] = {}; // NTT: twiddles of the N-point transform in pass order
     NttConst nk[kSmallLogMax + 1] = {};
 };
 
@@ -145,13 +141,7 @@ int get_ntt(int dev, int log_n, const uint64_t** qtw, NttConst* K) {
         uint64_t omega;
         NttConst k;
         if (!ntt_constants(log_n, omega, k)) return fail(LLG_E_UNSUPPORTED, "no N-th root of 2 for N=2^%d", log_n);
-        const uint32_t QL = 1u << log_n;
-        std::vector<uint64_t> h(gl_qpad8_len(QL), 0ull);
-        uint64_t w = 0xFFFFFFFFull;  // 1 in Montgomery form
-        for (uint32_t r = 0; r < QL; ++r) {
-            h[gl_qpad8(r)] = w;
-            w = hmul(w, omega);
-        }
+        const std::vector<uint64_t> h = ntt_pass_table(log_n, small_ntt_values(log_n));
         uint64_t* d = nullptr;
         CK(cudaMalloc(&d, h.size() * sizeof(uint64_t)));
         CK(cudaMemcpy(d, h.data(), h.size() * sizeof(uint64_t), cudaMemcpyHostToDevice));

@@ -33,6 +33,10 @@ std::vector<double2> pass_twiddle_table(int log_l, int log_e);
 // pass_twiddle_table(log_l, log_e), then w_M^{n k0} over n < L for k0 = 1 .. r0 - 1 (M = r0 L, L = 2^log_l).
 std::vector<double2> mixed_twiddle_table(int r0, int log_l, int log_e);
 
+// Twiddles of the 2^log_l-point NTT of 2^log_e values a thread, pass by pass (TW_PASS), Montgomery
+// form: the forward ones, then the inverse ones.
+std::vector<uint64_t> ntt_pass_table(int log_l, int log_e);
+
 struct LargeTest {
     uint64_t p = 0, N = 0, M = 0;
     // logN: log2 N (-1 for N = R0 2^k); logR: large_col_code of the column length R

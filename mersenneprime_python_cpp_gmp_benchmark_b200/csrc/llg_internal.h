@@ -92,8 +92,9 @@ struct NttConst {
     uint64_t root2, inv_root2, invN;
 };
 
-// Exact NTT whole-test kernel, N = 2^log_n with 6 <= log_n <= 13 (qtw: padded twiddle table of the
-// N-point transform, gl::qpad8 layout, Montgomery form).
+// Exact NTT whole-test kernel, N = 2^log_n with 6 <= log_n <= 13 (qtw: ntt_pass_table of the form's
+// values a thread).
+int small_ntt_values(int log_n);  // log2 of the values a thread
 cudaError_t launch_small_ntt(int log_n, const SmallJob* jobs, int njobs, const uint64_t* qtw, NttConst K,
                              int64_t* digits, SmallResult* results, cudaStream_t st);
 
@@ -229,17 +230,16 @@ cudaError_t launch_large_col(int log_r, const LargeArgs& a, cudaStream_t st);
 struct NttLargeArgs {
     uint64_t* V;              // state: element (row a, column slot pos) at pos * R + a
     // every constant in Montgomery form (llg_ntt.cuh)
-    const uint64_t* qtwC;     // padded twiddle table of the C-point row NTT (gl::qpad8)
-    const uint64_t* qtwR;     // padded twiddle table of the R-point column NTT
+    const uint64_t* qtwC;     // twiddles of the C-point row NTT in pass order (ntt_pass_table)
+    const uint64_t* qtwR;     // twiddles of the R-point column NTT
     const uint64_t* tw1;      // w_N^x, x < 2^tw_shift
     const uint64_t* tw2;      // w_N^(y 2^tw_shift)
     const int* pos_of_c;      // column slot of row-NTT frequency c
     const uint64_t* wA;       // [R] w^sA(a), w an N-th root of 2
     const uint64_t* iwA;      // [R] w^-sA(a)
-    const int* sA;            // [R] (-a p) mod N
     const uint64_t* wB;       // [C] w^sB(b)
     const uint64_t* iwB;      // [C] w^-sB(b) / N, times the square's 2^64
-    const int* sB;            // [C] (-R b p) mod N
+    const uint32_t* kinds;    // digit kinds by tile and thread (fill_ntt_kinds): N / 8 words
     long long* c1;            // [nblocks + 1][C] hop-1 carry-outs of a tile's last row: slot 0 the
                               // wrap-around job's (row R-1, one column on), k + 1 tile k's
     int* c2;                  // [nblocks + 1][C] hop-2 carry-outs
@@ -248,12 +248,14 @@ struct NttLargeArgs {
     unsigned int* flags;      // [nblocks + 1] epoch + 1 once the job of that slot published its carries
     int* digits;              // N int32, natural order (INIT input; dump / FINAL output)
     int dump;
+    int pdl_late;             // as LargeArgs::pdl_late
     int tw_shift;
     int C, R, nblocks;
     int q, rem;
     int logN;
 };
 
+cudaError_t launch_fill_ntt_kinds(uint32_t* kinds, const int* sA, const int* sB, int N, int rem, int C, int R, cudaStream_t st);
 cudaError_t launch_ntt_row(int log_c, int mode, const NttLargeArgs& a, cudaStream_t st);
 cudaError_t launch_ntt_col(int log_r, const NttLargeArgs& a, cudaStream_t st);
 cudaError_t configure_ntt_large(int log_c, int log_r);

@@ -472,19 +472,25 @@ uint64_t qpow(uint64_t a, uint64_t e) {
 
 uint64_t to_mont(uint64_t x) { return qmul(x, 0xFFFFFFFFull); }  // x 2^64 mod q
 
-std::vector<uint64_t> ntt_table(int log_l) {  // w_L^r at gl::qpad8(r), r < L, Montgomery form
-    const uint32_t L = 1u << log_l;
-    std::vector<uint64_t> t(L + (L >> 4) + 1, 0ull);
-    const uint64_t w = qpow(7, (kQ - 1) / L);
-    uint64_t x = to_mont(1);
-    for (uint32_t r = 0; r < L; ++r) {
-        t[r + (r >> 4)] = x;
-        x = qmul(x, w);
+}  // namespace
+
+std::vector<uint64_t> ntt_pass_table(int log_l, int log_e) {
+    const uint64_t L = 1ull << log_l, E = 1ull << log_e;
+    std::vector<uint64_t> t;
+    for (int inv = 0; inv < 2; ++inv) {
+        const uint64_t w = inv ? qpow(qpow(7, (kQ - 1) / L), kQ - 2) : qpow(7, (kQ - 1) / L);
+        // pass s: groups of len values in E strides of st; w_len^(n2 k1) = w^(n2 k1 L / len)
+        for (uint64_t len = L; len / E > 1; len /= E) {
+            const uint64_t st = len / E, wl = qpow(w, L / len);
+            uint64_t wk = wl;
+            for (uint64_t k1 = 1; k1 < E; ++k1, wk = qmul(wk, wl)) {
+                uint64_t x = to_mont(1);
+                for (uint64_t n2 = 0; n2 < st; ++n2, x = qmul(x, wk)) t.push_back(x);
+            }
+        }
     }
     return t;
 }
-
-}  // namespace
 
 bool ntt_host_constants(int log_n, uint64_t& omega, uint64_t& root2, uint64_t& inv_root2, uint64_t& invN) {
     // cuda/ll_ntt.cu:182-195: w_N = 7^((q-1)/N); an N-th root of 2 from a primitive (192N)-th root
@@ -515,7 +521,8 @@ cudaError_t NttLargeTest::init(uint64_t p_, int log_n) {
     p = p_;
     logN = log_n;
     N = 1ull << logN;
-    logC = std::min(10, std::max(7, logN / 2));
+    // us a squaring: 2^17 18.9 with rows of 2^9, 21.1 of 2^8; 2^20 56.1 of 2^9, 62.2 of 2^10
+    logC = logN <= 15 ? 7 : logN == 16 ? 8 : logN <= 20 ? 9 : 10;
     logR = logN - logC;
     C = 1 << logC;
     R = 1 << logR;
@@ -542,7 +549,7 @@ cudaError_t NttLargeTest::init(uint64_t p_, int log_n) {
     };
     NttLargeArgs& A = args;
     std::memset(&A, 0, sizeof A);
-    std::vector<uint64_t> qc = ntt_table(logC), qr = ntt_table(logR);
+    std::vector<uint64_t> qc = ntt_pass_table(logC, 3), qr = ntt_pass_table(logR, 3);  // the kernels' radix-8 passes
     std::vector<uint64_t> t1(1ull << s), t2(N >> s);
     {
         uint64_t x = to_mont(1);
@@ -578,7 +585,10 @@ cudaError_t NttLargeTest::init(uint64_t p_, int log_n) {
         (e = up(pc, &cpc)) || (e = up(hwA, &cwA)) || (e = up(hiwA, &ciwA)) || (e = up(hsA, &csA)) ||
         (e = up(hwB, &cwB)) || (e = up(hiwB, &ciwB)) || (e = up(hsB, &csB)))
         return e;
-    void *dV, *dc1, *dc2, *dc3, *dctl, *dd, *dfl;
+    void *dV, *dc1, *dc2, *dc3, *dctl, *dd, *dfl, *dk;
+    if ((e = alloc(N / 8 * sizeof(uint32_t), &dk))) return e;
+    if ((e = launch_fill_ntt_kinds(static_cast<uint32_t*>(dk), csA, csB, (int)N, (int)(p & (N - 1)), C, R, nullptr))) return e;
+    if ((e = cudaStreamSynchronize(nullptr))) return e;  // before any other stream reads them
     if ((e = alloc(N * sizeof(uint64_t), &dV)) || (e = alloc((size_t)(nblocks + 1) * C * sizeof(long long), &dc1)) ||
         (e = alloc((size_t)(nblocks + 1) * C * sizeof(int), &dc2)) ||
         (e = alloc((size_t)(nblocks + 1) * C * sizeof(int), &dc3)) ||
@@ -597,10 +607,9 @@ cudaError_t NttLargeTest::init(uint64_t p_, int log_n) {
     A.pos_of_c = cpc;
     A.wA = cwA;
     A.iwA = ciwA;
-    A.sA = csA;
     A.wB = cwB;
     A.iwB = ciwB;
-    A.sB = csB;
+    A.kinds = static_cast<const uint32_t*>(dk);
     A.c1 = static_cast<long long*>(dc1);
     A.c2 = static_cast<int*>(dc2);
     A.c3 = static_cast<int*>(dc3);
@@ -608,6 +617,7 @@ cudaError_t NttLargeTest::init(uint64_t p_, int log_n) {
     A.flags = static_cast<unsigned*>(dfl);
     A.digits = digits;
     A.dump = 0;
+    A.pdl_late = large_pdl_late(N);
     A.tw_shift = s;
     A.C = C;
     A.R = R;

@@ -176,17 +176,6 @@ struct NDft<8, INV> {
     }
 };
 
-// Table of the L-point transform: w_L^r in Montgomery form at slot qpad8(r) = r + r/16, r < L
-// (strided pass indices spread over the 8-byte banks).
-__host__ __device__ constexpr uint32_t qpad8(uint32_t r) { return r + (r >> 4); }
-__host__ __device__ constexpr uint32_t qpad8_len(uint32_t n) { return n + (n >> 4) + 1; }
-
-template <int LOG_L>
-__device__ __forceinline__ uint64_t twiddle(const uint64_t* __restrict__ t, uint32_t x, bool inv) {
-    constexpr uint32_t L = 1u << LOG_L;
-    return t[qpad8(inv ? (L - x) & (L - 1) : x)];  // w^-x = w^(L - x)
-}
-
 }  // namespace gl
 }  // namespace llg
 
@@ -200,6 +189,12 @@ namespace gl {
 // unrolled radix-16 kernels waited for instruction fetch 4 to 5.5 cycles per issued instruction)
 // and twice the threads share the work.
 constexpr int kLogE = 3;
+
+// Length of a geometry's twiddle table (TW_PASS order, Montgomery form): the forward passes' twiddles,
+// then the inverse ones. A pass reads consecutive slots at constant offsets: no index arithmetic on
+// the ALU that binds these kernels (25 of about 280 ALU instructions a value before).
+template <class G>
+__host__ __device__ constexpr int table_len() { return 2 * G::pass_offset(G::P - 1); }
 
 // Radix pass S of the L-point NTT on the register array (same geometry, positions and exchange
 // pattern as the FP64 passes of llg_fft.cuh; 8-byte field elements in the exchange buffer; ES and
@@ -219,6 +214,7 @@ __device__ __forceinline__ void radix_pass(uint64_t (&v)[G::E], uint64_t* __rest
         const int g = beta / ST, n2 = beta % ST;
         const int base = g * L + n2;
         uint64_t* vv = v + h * R;
+        const uint64_t* w = qtw + (INV ? G::pass_offset(G::P - 1) : 0) + G::pass_offset(S) + n2;
         if constexpr (LOAD) {
 #pragma unroll
             for (int n1 = 0; n1 < R; ++n1) vv[n1] = buf[physp<PADLOG>(base + n1 * ST) * ES];
@@ -226,13 +222,13 @@ __device__ __forceinline__ void radix_pass(uint64_t (&v)[G::E], uint64_t* __rest
         if constexpr (INV && ST > 1) {
 #pragma unroll
             for (int k1 = 1; k1 < R; ++k1)
-                vv[k1] = mul(vv[k1], twiddle<G::LOG_M_>(qtw, (uint32_t)(n2 * k1) << (G::LE * S), true));
+                vv[k1] = mul(vv[k1], w[(k1 - 1) * ST]);
         }
         NDft<R, INV>::run(vv);
         if constexpr (!INV && ST > 1) {
 #pragma unroll
             for (int k1 = 1; k1 < R; ++k1)
-                vv[k1] = mul(vv[k1], twiddle<G::LOG_M_>(qtw, (uint32_t)(n2 * k1) << (G::LE * S), false));
+                vv[k1] = mul(vv[k1], w[(k1 - 1) * ST]);
         }
         if constexpr (STORE && !SYNC_BEFORE_STORE) {
 #pragma unroll

@@ -23,10 +23,11 @@
 //
 // Both passes are bound by the integer ALU (the arithmetic of llg_ntt.cuh). Measured, us a squaring
 // replayed from graphs, against radix-16 passes of one row per warp group with the 128-bit
-// reduction: N = 2^16 55.5 -> 18.5, 2^18 67.3 -> 39.1, 2^21 176.8 -> 107.0, 2^23 654 -> 436. At 2^21 the
-// row pass issues 37.2 M warp instructions (47.3 M before) at 57% of the ALU's rate (39%), the
+// reduction: N = 2^16 55.5 -> 17.5, 2^18 67.3 -> 23.2, 2^21 176.8 -> 106.9, 2^23 654 -> 432. At 2^21 the
+// row pass issued 37.2 M warp instructions (47.3 M before) at 57% of the ALU's rate (39%), the
 // column pass 31.1 M at 67% (58%); neither waits for instruction fetch any more (5.5 cycles per
-// issued instruction before).
+// issued instruction before). Kinds from a table and pass-ordered twiddles then took the row pass at
+// 2^21 from 71 to 66.5 us.
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -63,31 +64,29 @@ __global__ void __launch_bounds__(kNttRowG * NttRowG<LOG_C>::T, 1024 / (kNttRowG
     ntt_row(const NttLargeArgs A) {
     using GC = NttRowG<LOG_C>;
     constexpr int C = GC::M, TR = GC::T, E = GC::E, G = kNttRowG, T = G * TR, PL = gl::kLogE;
-    constexpr int QL = (int)gl::qpad8_len(C);
+    constexpr int QL = gl::table_len<GC>();
     constexpr unsigned FULL = 0xffffffffu;
     static_assert(T % 32 == 0 && 32 % G == 0 && G >= 4 && C % T == 0, "whole warps of whole row groups");
     extern __shared__ __align__(16) unsigned char smem_raw[];
     uint64_t* xbuf = reinterpret_cast<uint64_t*>(smem_raw);  // exchange: slot physp(x) * G + row
-    uint64_t* qtw = xbuf + ntt_row_slots<LOG_C>();            // padded twiddle table
+    uint64_t* qtw = xbuf + ntt_row_slots<LOG_C>();            // twiddles in pass order
     uint64_t* swB = qtw + QL;                                 // C column weights
     uint64_t* siwB = swB + C;                                 // C inverse column weights
-    int* ssB = reinterpret_cast<int*>(siwB + C);              // C column weight exponents
     __shared__ int s_job;
     __shared__ unsigned s_epoch;
 
     const int t = threadIdx.x, ra = t % G, tr = t / G;
     uint64_t* buf = xbuf + ra;
-    const int N = 1 << A.logN, R = A.R;
+    const int R = A.R;
     const CtaSync sync;
 
-    // the next pass may launch once every block of this one has started; constant tables first,
-    // nothing the previous pass writes before the wait
-    pdl_launch_dependents();
+    // the next pass may launch once every block of this one has started (or, pdl_late, is near its
+    // end); constant tables first, nothing the previous pass writes before the wait
+    if (!A.pdl_late) pdl_launch_dependents();
     for (int k = t; k < QL; k += T) cp_async<8>(qtw + k, A.qtwC + k);
     for (int k = t; k < C; k += T) {
         cp_async<8>(swB + k, A.wB + k);
         if (MODE != LARGE_INIT) cp_async<8>(siwB + k, A.iwB + k);
-        cp_async<4>(ssB + k, A.sB + k);
     }
     pdl_wait_previous();
     if (t == 0) {
@@ -111,21 +110,12 @@ __global__ void __launch_bounds__(kNttRowG * NttRowG<LOG_C>::T, 1024 / (kNttRowG
     const unsigned ep = s_epoch;
     const bool wrap_job = job < 0;
     const int a = (wrap_job ? R - G : job * G) + ra;  // this thread's row
-    const int sA = __ldg(A.sA + a);
 
     uint64_t v[E];
     int x[E];
-    uint32_t big = 0u, wrap = 0u;  // bit i: the digit has q + 1 bits; sA + sB >= N
-    auto kinds = [&]() {
-#pragma unroll
-        for (int i = 0; i < E; ++i) {
-            const int sb = ssB[tr + TR * i];
-            const bool o = sA + sb >= N;
-            const int s = o ? sA + sb - N : sA + sb;
-            big |= (uint32_t)(s < A.rem) << i;
-            wrap |= (uint32_t)o << i;
-        }
-    };
+    // bit i of big: the digit has q + 1 bits; of wrap: sA + sB >= N (fill_ntt_kinds)
+    const uint32_t kw = __ldg(A.kinds + (size_t)(a / G) * T + t);
+    const uint32_t big = kw & 0xffu, wrap = kw >> 8;
     auto bits = [&](int i) { return A.q + (int)((big >> i) & 1u); };
 
     if constexpr (MODE == LARGE_INIT) {
@@ -133,7 +123,6 @@ __global__ void __launch_bounds__(kNttRowG * NttRowG<LOG_C>::T, 1024 / (kNttRowG
         for (int i = 0; i < E; ++i) x[i] = A.digits[(size_t)a + (size_t)R * (tr + TR * i)];
         cp_async_wait_all();
         __syncthreads();  // the tables are in shared memory
-        kinds();
     } else {
         {
             const uint64_t* lp = A.V + (size_t)(tr * E) * R + a;
@@ -143,7 +132,6 @@ __global__ void __launch_bounds__(kNttRowG * NttRowG<LOG_C>::T, 1024 / (kNttRowG
         cp_async_wait_all();
         __syncthreads();  // the tables are in shared memory
         gl::inverse_from<GC, GC::P - 1, false, CtaSync, G, PL>(v, buf, qtw, tr, sync);
-        kinds();
 
         // ---- unweight, lift, hop 1 of every row; hops 2 to 4 of the rows whose carry-in comes from
         //      inside the tile. Row G-1 publishes its three carry-outs (the wrap job: one column on).
@@ -194,14 +182,12 @@ __global__ void __launch_bounds__(kNttRowG * NttRowG<LOG_C>::T, 1024 / (kNttRowG
         if (t == 0) wait_flag(&A.flags[job], ep + 1u, A.ctl, kSpinLimit);
         __syncthreads();
         {
-            const int s0 = __ldg(A.sA + job * G);
             const size_t o = (size_t)job * C;
 #pragma unroll
             for (int k = 0; k < C / T; ++k) {
                 const int b = t + T * k;
-                const int sb = ssB[b];
-                const int s = (s0 + sb >= N) ? s0 + sb - N : s0 + sb;
-                const int nb = A.q + (s < A.rem);
+                // row 0's thread t % TR, value t / TR + G k
+                const int nb = A.q + (int)((__ldg(A.kinds + (size_t)job * T + (t % TR) * G) >> (t / TR + G * k)) & 1u);
                 long long cin = __ldcg(A.c1 + o + b), c;
                 if (job == 0 && b == 0) cin -= 2;  // the "- 2" of s^2 - 2 (digit 0)
                 int y = gl::balance64((long long)row0[b] + cin, nb, c), c3;
@@ -245,65 +231,96 @@ __global__ void __launch_bounds__(kNttRowG * NttRowG<LOG_C>::T, 1024 / (kNttRowG
         if (t == 0) wait_flag(&A.flags[0], ep + 1u, A.ctl, kSpinLimit);
         __syncthreads();
     }
+    if (A.pdl_late) pdl_launch_dependents();
     uint64_t* vp = A.V + (size_t)(tr * E) * R + a;
 #pragma unroll
     for (int j = 0; j < E; ++j) __stcg(vp + (size_t)j * R, v[j]);
 }
 
+// Each block runs columns blockIdx.x, + gridDim.x, ...: its twiddle tables are read once.
 template <int LOG_R>
 __global__ void __launch_bounds__(NttColG<LOG_R>::T, 1024 / NttColG<LOG_R>::T > 16 ? 16 : 1024 / NttColG<LOG_R>::T)
     ntt_col(const NttLargeArgs A) {
     using GR = NttColG<LOG_R>;
     constexpr int R = GR::M, TC = GR::T, E = GR::E;
-    constexpr int QL = (int)gl::qpad8_len(R);
+    constexpr int QL = gl::table_len<GR>();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     uint64_t* buf = reinterpret_cast<uint64_t*>(smem_raw);
     uint64_t* qtw = buf + GR::PAD;
-    uint64_t* ptab = qtw + QL;  // E forward, E inverse
+    uint64_t* ptabs = qtw + QL;  // two columns' tables in turn: E forward, E inverse
     const int tc = threadIdx.x;
-    const int c = blockIdx.x;
     const int N = 1 << A.logN;
-    pdl_launch_dependents();  // as in ntt_row
+    if (!A.pdl_late) pdl_launch_dependents();  // as in ntt_row
     for (int k = tc; k < QL; k += TC) cp_async<8>(qtw + k, A.qtwR + k);
-    // four-step twiddle w_N^{a c}, a = tc + TC i: w_N^{c tc} * w_N^{c TC i}
-    for (int i = tc; i < E; i += TC) {
-        const uint32_t xi = (uint32_t)(((uint64_t)c * TC * i) & (uint64_t)(N - 1));
-        ptab[i] = twiddle_N(A, xi);
-        ptab[E + i] = twiddle_N(A, (uint32_t)((N - xi) & (N - 1)));
-    }
-    const uint32_t xq = (uint32_t)(((uint64_t)c * tc) & (uint64_t)(N - 1));
-    uint64_t* col = A.V + (size_t)__ldg(A.pos_of_c + c) * R;
-    const uint64_t q = twiddle_N(A, xq);
-    pdl_wait_previous();
-    uint64_t v[E];
+    bool first = true;
+    for (int c = blockIdx.x; c < A.C; c += gridDim.x) {
+        uint64_t* ptab = ptabs + (c / (int)gridDim.x & 1) * 2 * E;
+        // four-step twiddle w_N^{a c}, a = tc + TC i: w_N^{c tc} * w_N^{c TC i}
+        for (int i = tc; i < E; i += TC) {
+            const uint32_t xi = (uint32_t)(((uint64_t)c * TC * i) & (uint64_t)(N - 1));
+            ptab[i] = twiddle_N(A, xi);
+            ptab[E + i] = twiddle_N(A, (uint32_t)((N - xi) & (N - 1)));
+        }
+        const uint32_t xq = (uint32_t)(((uint64_t)c * tc) & (uint64_t)(N - 1));
+        uint64_t* col = A.V + (size_t)__ldg(A.pos_of_c + c) * R;
+        const uint64_t q = twiddle_N(A, xq);
+        if (first) pdl_wait_previous();
+        uint64_t v[E];
 #pragma unroll
-    for (int i = 0; i < E; ++i) v[i] = col[tc + TC * i];
-    cp_async_wait_all();
-    __syncthreads();
+        for (int i = 0; i < E; ++i) v[i] = __ldcg(col + tc + TC * i);
+        if (first) cp_async_wait_all();
+        first = false;
+        __syncthreads();  // ptab, and the tables
 #pragma unroll
-    for (int i = 0; i < E; ++i) v[i] = gl::mul(v[i], gl::mul(q, ptab[i]));
-    gl::forward_from<GR, 0>(v, buf, qtw, tc);
+        for (int i = 0; i < E; ++i) v[i] = gl::mul(v[i], gl::mul(q, ptab[i]));
+        gl::forward_from<GR, 0>(v, buf, qtw, tc);
 #pragma unroll
-    for (int j = 0; j < E; ++j) v[j] = gl::mul(v[j], v[j]);
-    gl::inverse_from<GR, GR::P - 1, false>(v, buf, qtw, tc);
-    {
+        for (int j = 0; j < E; ++j) v[j] = gl::mul(v[j], v[j]);
+        gl::inverse_from<GR, GR::P - 1, false>(v, buf, qtw, tc);
         const uint64_t qi = twiddle_N(A, (uint32_t)((N - xq) & (N - 1)));
 #pragma unroll
         for (int i = 0; i < E; ++i) col[tc + TC * i] = gl::mul(v[i], gl::mul(qi, ptab[E + i]));
+        // the next column's first stores to buf are to slots this thread read itself
     }
-    if (c == 0 && tc == 0) atomicAdd(&A.ctl->epoch, 1u);
+    if (A.pdl_late) pdl_launch_dependents();
+    if (blockIdx.x == 0 && tc == 0) atomicAdd(&A.ctl->epoch, 1u);
+}
+
+// NttLargeArgs::kinds: word t of tile k holds the kinds of thread t's values (row t % G of the tile,
+// columns t / G + TR i): bit i: the digit has q + 1 bits (s < p mod N, s = (sA(a) + sB(b)) mod N);
+// bit 8 + i: sA + sB >= N.
+__global__ void fill_ntt_kinds(uint32_t* kinds, const int* __restrict__ sA, const int* __restrict__ sB, int N, int rem,
+                               int C, int words) {
+    const int w = blockIdx.x * blockDim.x + threadIdx.x;
+    if (w >= words) return;
+    constexpr int E = 1 << gl::kLogE;
+    const int TR = C / E, T = kNttRowG * TR, t = w % T;
+    const int sa = sA[w / T * kNttRowG + t % kNttRowG];
+    uint32_t k = 0u;
+    for (int i = 0; i < E; ++i) {
+        const int sb = sB[t / kNttRowG + TR * i];
+        const bool o = sa + sb >= N;
+        const int s = o ? sa + sb - N : sa + sb;
+        k |= ((uint32_t)(s < rem) << i) | ((uint32_t)o << (8 + i));
+    }
+    kinds[w] = k;
+}
+cudaError_t launch_fill_ntt_kinds(uint32_t* kinds, const int* sA, const int* sB, int N, int rem, int C, int R, cudaStream_t st) {
+    const int words = (int)((long long)R * C >> gl::kLogE);
+    fill_ntt_kinds<<<(words + 255) / 256, 256, 0, st>>>(kinds, sA, sB, N, rem, C, words);
+    return cudaGetLastError();
 }
 
 template <int LOG_C>
 static size_t ntt_row_smem() {
     constexpr int C = 1 << LOG_C;
-    return sizeof(uint64_t) * (ntt_row_slots<LOG_C>() + gl::qpad8_len(C) + 2 * C) + sizeof(int) * C;
+    return sizeof(uint64_t) * (ntt_row_slots<LOG_C>() + gl::table_len<NttRowG<LOG_C>>() + 2 * C);
 }
 
 template <int LOG_R>
 static size_t ntt_col_smem() {
     using GR = NttColG<LOG_R>;
-    return sizeof(uint64_t) * (GR::PAD + gl::qpad8_len(GR::M) + 2 * GR::E);
+    return sizeof(uint64_t) * (GR::PAD + gl::table_len<GR>() + 4 * GR::E);
 }
 
 // Programmatic stream serialisation, as the FP64 passes at power-of-two lengths.
@@ -325,8 +342,9 @@ static cudaError_t launch_pdl(void (*kernel)(KArgs...), int grid, int block, siz
 
 template <int LOG_C, int MODE>
 static cudaError_t ntt_row_attr() {
-    return cudaFuncSetAttribute(ntt_row<LOG_C, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)ntt_row_smem<LOG_C>());
+    cudaError_t e = cudaFuncSetAttribute(ntt_row<LOG_C, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)ntt_row_smem<LOG_C>());
+    return e;
 }
 
 // INIT: one block per tile. ITER / FINAL: one block more, for the wrap-around job.
@@ -338,13 +356,17 @@ static cudaError_t ntt_row_t(const NttLargeArgs& a, cudaStream_t st) {
 
 template <int LOG_R>
 static cudaError_t ntt_col_t(const NttLargeArgs& a, cudaStream_t st) {
-    return launch_pdl(ntt_col<LOG_R>, a.C, NttColG<LOG_R>::T, ntt_col_smem<LOG_R>(), st, a);
+    // one resident wave of blocks where a single block fits an SM (N = 2^23: 224 us a pass against 234);
+    // a block per column elsewhere (R = 2^11: 49 against 55)
+    const int most = LOG_R >= 13 ? device_sms() : a.C;
+    return launch_pdl(ntt_col<LOG_R>, a.C < most ? a.C : most, NttColG<LOG_R>::T, ntt_col_smem<LOG_R>(), st, a);
 }
 
 template <int LOG_R>
 static cudaError_t ntt_col_attr() {
-    return cudaFuncSetAttribute(ntt_col<LOG_R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)ntt_col_smem<LOG_R>());
+    cudaError_t e = cudaFuncSetAttribute(ntt_col<LOG_R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)ntt_col_smem<LOG_R>());
+    return e;
 }
 
 template <int LOG_C>

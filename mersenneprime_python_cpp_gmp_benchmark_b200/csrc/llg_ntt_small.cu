@@ -30,7 +30,8 @@ namespace llg {
 // test then spreads over the SM's four schedulers; 8 above. Measured, one test alone, us a
 // squaring, 4 values against 8: N = 256 1.73 / 3.75, 512 2.09 / 4.58, 1024 3.62 / 5.49, 2048 7.23 / 6.69,
 // 4096 16.4 / 14.4; 592 tests at once: N = 512 5.62 / 6.93, 1024 11.5 / 13.4, 2048 26.2 / 24.4. (The
-// radix-16 kernel before: N = 512 31.8 alone, 31.4 with 592; N = 2048 35.3 and 70.2.)
+// radix-16 kernel before: N = 512 31.8 alone, 31.4 with 592; N = 2048 35.3 and 70.2. With the twiddles in
+// pass order now 2.07 and 5.42, 6.57 and 23.6.)
 __host__ __device__ constexpr int small_ntt_log_e(int log_n) { return log_n <= 10 ? 2 : 3; }
 
 template <int LOG_N>
@@ -39,7 +40,7 @@ struct SmallNtt {
     using G = SmallG<LOG_N, LE>;
     static constexpr int N = G::M, E = G::E, T = G::T, W = G::W;
     static constexpr bool WT = LOG_N <= 11;  // whole weight tables in shared memory
-    static constexpr int QL = (int)gl::qpad8_len(N);
+    static constexpr int QL = gl::table_len<G>();
     static constexpr int NW = WT ? N : E;
     // blocks per SM the kernel is built for (64 registers a thread at 8 values)
     static constexpr int MINB = 1024 / T > 16 ? 16 : (1024 / T < 1 ? 1 : 1024 / T);
@@ -87,7 +88,7 @@ __global__ void __launch_bounds__(SmallNtt<LOG_N>::T, SmallNtt<LOG_N>::MINB)
     constexpr bool WT = SN::WT;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     uint64_t* buf = reinterpret_cast<uint64_t*>(smem_raw);    // exchange buffer, PAD slots
-    uint64_t* qtw = buf + G::PAD;                              // padded twiddle table
+    uint64_t* qtw = buf + G::PAD;                              // twiddles in pass order
     uint64_t* wT = qtw + QL;                                   // WT: w^s of digit m; else w^sB(i)
     uint64_t* iwT = wT + SN::NW;                               // WT: w^-s / N of digit m; else w^-sB(i) / N
     long long* cbuf = reinterpret_cast<long long*>(iwT + SN::NW);  // hop 1: W x E carry slots
@@ -209,6 +210,8 @@ static cudaError_t launch_small_ntt_t(const SmallJob* jobs, int njobs, const uin
     ll_small_ntt<LOG_N><<<njobs, SN::T, smem, st>>>(jobs, qtw, K, digits, results);
     return cudaGetLastError();
 }
+
+int small_ntt_values(int log_n) { return small_ntt_log_e(log_n); }
 
 cudaError_t launch_small_ntt(int log_n, const SmallJob* jobs, int njobs, const uint64_t* qtw, NttConst K,
                              int64_t* digits, SmallResult* results, cudaStream_t st) {
