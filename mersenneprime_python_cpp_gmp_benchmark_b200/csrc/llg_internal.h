@@ -145,6 +145,15 @@ constexpr int large_row_log_e(int log_c, int g) {
     return log_c > 9 ? 4 : ((log_c <= 7 && g <= 4) || (log_c == 8 && g == 2)) ? 2 : 3;
 }
 
+// Whether the row pass reads its twiddles in pass order (pass_twiddle_table), as below 16 values a
+// thread, or from the full padded table with factored products: at 16 values fifteen reads a pass
+// were no faster than six and nine products (N = 2^23 138.7 against 138.0), at 8 they were (5 x 2^18 26.6
+// against 27.3).
+#ifdef __CUDACC__
+__host__ __device__
+#endif
+constexpr bool large_row_pass_table(int log_c, int g) { return large_row_log_e(log_c, g) < 4; }
+
 struct LargeCtl {
     unsigned long long tickets;      // FP64 row-pass tickets taken since the start
     unsigned int epoch;              // squarings whose column pass has finished; +1 per column pass
@@ -184,7 +193,7 @@ struct __align__(16) LargeCarry {
 
 struct LargeArgs {
     double2* V;               // state: element (row a, column slot pos) at pos * R + a
-    const double2* qtwC;      // full padded twiddle table of the C-point row FFT
+    const double2* qtwC;      // twiddles of the C-point row FFT (large_row_pass_table)
     const double2* qtwR;      // quarter table of the R-point column FFT (spread layout for a
                               // power-of-two R, padded for R = R0 L)
     const double2* qtwL;      // R = R0 L: padded quarter table of the L-point column sub-FFTs

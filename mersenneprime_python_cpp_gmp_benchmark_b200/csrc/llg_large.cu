@@ -110,16 +110,14 @@ template <int LOG_C, int G, int MODE, bool DENSE>
 __global__ void __launch_bounds__(large_row_threads(LOG_C, G), large_row_min_blocks(LOG_C, G, DENSE))
     large_row(const LargeArgs A) {
     constexpr int LE = large_row_log_e(LOG_C, G);
-    // full twiddle table; at 16 values a thread factored twiddles (at 8, three products fewer and the
-    // same time without)
-    using GC = SmallG<LOG_C, LE, TW_FULL, (LE >= 4)>;
+    using GC = SmallG<LOG_C, LE, large_row_pass_table(LOG_C, G) ? TW_PASS : TW_FULL, true>;
     constexpr int C = GC::M, TR = GC::T, E = GC::E, T = G * TR;
     static_assert(T % 32 == 0 && 32 % G == 0, "whole warps of whole row groups");
     constexpr unsigned FULL = 0xffffffffu;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     constexpr int QL = (int)twiddle_table_len<GC>();
     double2* xbuf = reinterpret_cast<double2*>(smem_raw);          // exchange: slot physp(x) * G + row
-    double2* qtw = xbuf + large_row_slots(LOG_C, G);               // padded twiddle table (C-point)
+    double2* qtw = xbuf + large_row_slots(LOG_C, G);               // twiddles of the C-point FFT
     double* swB = reinterpret_cast<double*>(qtw + QL);             // C column weights 2^(sB/N)
     double* siwB = swB + C;                                        // C inverse column weights
     __shared__ unsigned long long s_err;
@@ -610,7 +608,7 @@ cudaError_t launch_fill_kinds(uint32_t* kinds, const int* sA, const int* sB, int
 
 template <int LOG_C, int G>
 static size_t row_smem() {
-    using GC = SmallG<LOG_C, large_row_log_e(LOG_C, G), TW_FULL, (large_row_log_e(LOG_C, G) >= 4)>;
+    using GC = SmallG<LOG_C, large_row_log_e(LOG_C, G), large_row_pass_table(LOG_C, G) ? TW_PASS : TW_FULL, true>;
     return sizeof(double2) * (large_row_slots(LOG_C, G) + twiddle_table_len<GC>()) + 2 * sizeof(double) * GC::M;
 }
 

@@ -212,7 +212,7 @@ cudaError_t LargeTest::init(uint64_t p_, uint64_t n, int log_c, int rows_) {
     cudaError_t e;
     if ((e = configure_large(logC, rows, logR))) return e;
     // tables
-    if ((e = upload(&qtwC, padded_full_table(C)))) return e;
+    if ((e = upload(&qtwC, large_row_pass_table(logC, rows) ? pass_twiddle_table(logC, large_row_log_e(logC, rows)) : padded_full_table(C)))) return e;
     if (r0 == 1) {
         if ((e = upload(&qtwR, spread_quarter_table(R)))) return e;  // the column pass reads qpad_s
     } else {

@@ -32,6 +32,7 @@
 #include <cstdio>
 #include <cstring>
 #include <mutex>
+#include <vector>
 
 #include "../../include/llgpu.h"
 #include "llg_device.cuh"
@@ -82,7 +83,7 @@ Layout layout(int logN, int logC, int logR, int s) {
     L.carry = o; o = up256(o + (nblocks + 1) * C * sizeof(LargeCarry));  // slot 0: the wrap-around job
     L.ctl = o; o = up256(o + sizeof(LargeCtl));
     L.wrap_read = o; o = up256(o + sizeof(unsigned));
-    L.qtwC = o; o = up256(o + qpad_len((uint32_t)C) * sizeof(double2));
+    L.qtwC = o; o = up256(o + C * sizeof(double2));
     L.qtwR = o; o = up256(o + qpad_s_len((uint32_t)(R / 4)) * sizeof(double2));  // spread layout
     L.tw1 = o; o = up256(o + ((size_t)1 << s) * sizeof(double2));
     L.tw2 = o; o = up256(o + (M >> s) * sizeof(double2));
@@ -185,7 +186,10 @@ extern "C" int llg_run_noalloc(uint64_t p, uint64_t iters, uint32_t n, int32_t* 
         const long double Nl = (long double)N;
         const size_t o = L.qtwC;
         std::memset(g_stage, 0, L.kinds - o);
-        stage_table<double2>(L.qtwC - o, qpad_len((uint32_t)C), [&](size_t i) { return padded_quarter_slot(C, i); });
+        {
+            const std::vector<double2> t = pass_twiddle_table(logC, large_row_log_e(logC, kTileRows));  // < C values
+            std::memcpy(g_stage + (L.qtwC - o), t.data(), t.size() * sizeof(double2));
+        }
         {  // the column pass's quarter table in the spread layout: entry r at qpad_s(r)
             double2* q = reinterpret_cast<double2*>(g_stage + (L.qtwR - o));
             for (uint32_t r = 0; r < (uint32_t)R / 4; ++r) q[qpad_s(r)] = padded_quarter_slot(R, qpad(r));
