@@ -152,6 +152,8 @@ __global__ void __launch_bounds__(SmallGeo<LOG_M, LE>::T, small_min_blocks(Small
         for (int w = 0; w < (E + 7) / 8; ++w) asm volatile("" : "+r"(kinds[w]));
     };
 
+    // the weighted digits, the transform, and from the carry to the next weighting the digits: doubles
+    // throughout (as integers in between they cost four FP64 conversions a value)
     double2 v[E];
     // s_0 = 4: digit 0 (thread 0, i = 0, even) has weight a_0 = 1
 #pragma unroll
@@ -166,7 +168,6 @@ __global__ void __launch_bounds__(SmallGeo<LOG_M, LE>::T, small_min_blocks(Small
     double maxerr = 0.0;
     uint64_t it = 0;
     uint32_t status = LLG_ST_OK;
-    int x0s[E], x1s[E];
 
     for (;;) {
         forward_from<G, 0, Sync, 1, PL>(v, buf, qtw, t, sync);
@@ -226,8 +227,8 @@ __global__ void __launch_bounds__(SmallGeo<LOG_M, LE>::T, small_min_blocks(Small
 #pragma unroll
             for (int i = 0; i < E; ++i) {
                 double cy;
-                x0s[i] = d2i_exact(dsplit_k(x0[i] + c[i], dq, kind(i, 0), cy));
-                x1s[i] = d2i_exact(x1[i] + cy);
+                v[i].x = dsplit_k(x0[i] + c[i], dq, kind(i, 0), cy);
+                v[i].y = x1[i] + cy;
             }
             lerr = err.value();
             if (errlog) {
@@ -246,18 +247,16 @@ __global__ void __launch_bounds__(SmallGeo<LOG_M, LE>::T, small_min_blocks(Small
                 err.add(a - ra);
                 err.add(b - rb);
                 double c;
-                double x0 = dsplit_k(ra, dq, kind(i, 0), c);
+                const double x0 = dsplit_k(ra, dq, kind(i, 0), c);
                 const double x1 = dsplit_k(rb + c, dq, kind(i, 1), c);
                 const double cout = c;
                 if (lane == 31) cbuf[warp * E + i] = cout;
                 const double cin = __shfl_up_sync(0xffffffffu, cout, 1);
+                v[i] = make_double2(x0, x1);
                 if (lane != 0) {
-                    x0 = dsplit_k(x0 + cin, dq, kind(i, 0), c);
-                    x1s[i] = d2i_exact(x1 + c);
-                } else {
-                    x1s[i] = d2i_exact(x1);
+                    v[i].x = dsplit_k(x0 + cin, dq, kind(i, 0), c);
+                    v[i].y = x1 + c;
                 }
-                x0s[i] = d2i_exact(x0);
             }
             lerr = err.value();
             if (errlog) atomicMax(&serr[it & 1], (unsigned long long)__double_as_longlong(lerr));
@@ -276,8 +275,8 @@ __global__ void __launch_bounds__(SmallGeo<LOG_M, LE>::T, small_min_blocks(Small
                                         : cbuf[(W - 1) * E + ((i + E - 1) % E)];  // m-1 wraps at m=0
                 if (t == 0 && i == 0) cin -= 2.0;  // the "- 2" of s^2 - 2
                 double c;
-                x0s[i] = d2i_exact(dsplit_k((double)x0s[i] + cin, dq, kind(i, 0), c));
-                x1s[i] += (int)c;
+                v[i].x = dsplit_k(v[i].x + cin, dq, kind(i, 0), c);
+                v[i].y += c;
             }
         }
         ++it;
@@ -290,8 +289,8 @@ __global__ void __launch_bounds__(SmallGeo<LOG_M, LE>::T, small_min_blocks(Small
 #pragma unroll
         for (int i = 0; i < E; ++i) {
             const double w = wB[i];
-            v[i].x = i2d_shift(x0s[i]) * scale_down(wA0 * w, kind(i, 2));
-            v[i].y = i2d_shift(x1s[i]) * scale_down(wA1 * w, kind(i, 3));
+            v[i].x *= scale_down(wA0 * w, kind(i, 2));
+            v[i].y *= scale_down(wA1 * w, kind(i, 3));
         }
     }
 
@@ -300,8 +299,8 @@ __global__ void __launch_bounds__(SmallGeo<LOG_M, LE>::T, small_min_blocks(Small
 #pragma unroll
         for (int i = 0; i < E; ++i) {
             const int m = t + T * i;
-            out[2 * m] = x0s[i];
-            out[2 * m + 1] = x1s[i];
+            out[2 * m] = d2i_exact(v[i].x);
+            out[2 * m + 1] = d2i_exact(v[i].y);
         }
     }
     // block max of the round-off (non-negative doubles order like their bit patterns)

@@ -182,7 +182,8 @@ __global__ void __launch_bounds__(MixedGeom<R0, LOG_L, LE, MINB>::T, MINB)
         for (int w = 0; w < (CA + 7) / 8; ++w) asm volatile("" : "+r"(kinds[w]));
     };
 
-    // the digits between squarings: s_0 = 4 (digit 0 has weight 1)
+    // the digits between squarings, as integers (as doubles they spilled: N = 6144 28.7 -> 34.0 us a
+    // squaring): s_0 = 4 (digit 0 has weight 1)
     int x0s[CA], x1s[CA];
 #pragma unroll
     for (int c = 0; c < CA; ++c) x0s[c] = x1s[c] = 0;
@@ -311,8 +312,8 @@ __global__ void __launch_bounds__(MixedGeom<R0, LOG_L, LE, MINB>::T, MINB)
                 double cin = (warp > 0) ? cbuf[(warp - 1) * CA + c] : cbuf[(WA - 1) * CA + ((c + CA - 1) % CA)];
                 if (t == 0 && c == 0) cin -= 2.0;  // the "- 2" of s^2 - 2
                 double cy;
-                x0s[c] = d2i_exact(dsplit_k((double)x0s[c] + cin, dq, kind(c, 0), cy));
-                x1s[c] += (int)cy;
+                x0s[c] = d2i_exact(dsplit_k(i2d_shift(x0s[c]) + cin, dq, kind(c, 0), cy));
+                x1s[c] += d2i_exact(cy);
             }
         }
         ++it;
