@@ -83,10 +83,9 @@ uint64_t hpow(uint64_t a, uint64_t e) {
 }
 uint64_t hinv(uint64_t a) { return hpow(a, kGQ - 2); }
 
-// w_N = 7^((q-1)/N) and an N-th root of 2 from a primitive (192 N)-th root (2 has order 192)
-bool ntt_constants(int log_n, uint64_t& omega, NttConst& K) {
+// An N-th root of 2 from a primitive (192 N)-th root (2 has order 192)
+bool ntt_constants(int log_n, NttConst& K) {
     const uint64_t N = 1ull << log_n;
-    omega = hpow(7, (kGQ - 1) / N);
     const uint64_t om = hpow(7, (kGQ - 1) / (192 * N)), r192 = hpow(om, N);
     uint64_t pw = 1, s = 0;
     for (; s < 192; ++s) {
@@ -138,9 +137,8 @@ int get_ntt(int dev, int log_n, const uint64_t** qtw, NttConst* K) {
     std::lock_guard<std::mutex> lk(g_mx);
     DeviceTables& T = g_tables[dev];
     if (!T.nqtw[log_n]) {
-        uint64_t omega;
         NttConst k;
-        if (!ntt_constants(log_n, omega, k)) return fail(LLG_E_UNSUPPORTED, "no N-th root of 2 for N=2^%d", log_n);
+        if (!ntt_constants(log_n, k)) return fail(LLG_E_UNSUPPORTED, "no N-th root of 2 for N=2^%d", log_n);
         const std::vector<uint64_t> h = ntt_pass_table(log_n, small_ntt_values(log_n));
         uint64_t* d = nullptr;
         CK(cudaMalloc(&d, h.size() * sizeof(uint64_t)));

@@ -1,12 +1,11 @@
-// Shared-memory-exchanged in-register FFT of L = 2^LOG_L complex points (radix-16 passes, the
-// last one radix 2/4/8/16), used for the whole-test kernel (L = M = N/2) and for the row and
-// column passes of the two-pass engine. A group of T = L/16 threads owns one transform; thread t
-// holds 16 values. Forward = decimation in frequency: natural order in (thread t holds element
-// t + T*i in v[i]), mixed-radix digit-reversed order out (thread t holds positions 16t + j in
+// Shared-memory-exchanged in-register FFT of L = 2^LOG_M complex points (radix-E passes, E = 2^LOG_E
+// of 2 to 16, the last one whatever is left), used for the whole-test kernels and for the row and
+// column passes of the two-pass engine. A group of T = L/E threads owns one transform; thread t
+// holds E values. Forward = decimation in frequency: natural order in (thread t holds element
+// t + T*i in v[i]), mixed-radix digit-reversed order out (thread t holds positions E t + j in
 // v[j]; freq_of_pos / pos_of_freq translate). Inverse = the same passes retraced, back to natural
-// order, unscaled (x L). The exchange buffer is one array of L + L/16 complex (16-byte) slots;
-// phys() pads one slot per 16, which keeps every pass's access pattern at the minimum of four
-// shared-memory wavefronts per warp access (at most five).
+// order, unscaled (x L). The exchange buffer is one padded array of L complex (16-byte) slots and
+// spare ones.
 #pragma once
 
 #include <cstdint>
@@ -16,12 +15,11 @@
 namespace llg {
 
 // Twiddle table of a geometry: e^{-2 pi i r / M} at slot qpad(r) for r < M/4 (TW_QUARTER: the
-// other quadrants by rotation), r < M/2 (TW_HALF: the other half by negation), or r < M (TW_FULL:
-// one table read, no fold); TW_QUARTER_S: the quarter table at slot qpad_s(r); TW_PASS: the twiddles
+// other quadrants by rotation), or r < M (TW_FULL: one table read, no fold); TW_QUARTER_S: the quarter table at slot qpad_s(r); TW_PASS: the twiddles
 // of every radix pass in the order the pass reads them, entry (k1 - 1) ST + n2 of pass S holds
 // w^(n2 k1 E^S) (pass_offset(S) on): consecutive lanes read consecutive slots, and nothing is folded
 // or multiplied up from other entries. About M entries, where the quarter table has M / 4.
-enum { TW_QUARTER = 0, TW_HALF = 1, TW_FULL = 2, TW_QUARTER_S = 3, TW_PASS = 4 };
+enum { TW_QUARTER, TW_FULL, TW_QUARTER_S, TW_PASS };
 
 // L = 2^LOG_M points, E = 2^LOG_E values per thread (radix-E passes, the last one RLAST).
 template <int LOG_M, int LOG_E = 4>
@@ -122,11 +120,6 @@ __device__ __forceinline__ double2 twiddle_g(const double2* __restrict__ q, uint
     if constexpr (G::TWM == TW_FULL) {
         const double2 w = q[qpad(x & (uint32_t)(G::M - 1))];
         return inv ? conj2(w) : w;
-    } else if constexpr (G::TWM == TW_HALF) {
-        constexpr uint32_t H = (uint32_t)G::M / 2;
-        const double2 w = q[qpad(x & (H - 1))];
-        const bool ng = (x & H) != 0;  // e^{-2 pi i (r + M/2) / M} = -e^{-2 pi i r / M}
-        return make_double2(ng ? -w.x : w.x, (ng != inv) ? -w.y : w.y);
     } else if constexpr (G::TWM == TW_QUARTER_S) {
         return twiddle<G::LOG_M_, true>(q, x, inv);
     } else {
@@ -302,7 +295,7 @@ template <class G>
 __host__ __device__ constexpr uint32_t twiddle_table_len() {
     if (G::TWM == TW_QUARTER_S) return qpad_s_len((uint32_t)G::M >> 2);
     if (G::TWM == TW_PASS) return (uint32_t)G::pass_offset(G::P - 1);
-    return qpad_len((uint32_t)G::M >> (G::TWM == TW_FULL ? 0 : G::TWM == TW_HALF ? 1 : 2));
+    return qpad_len((uint32_t)G::M >> (G::TWM == TW_FULL ? 0 : 2));
 }
 
 }  // namespace llg

@@ -117,7 +117,7 @@ cudaError_t rebuild_batch(const int64_t* d_digits, const SmallJob* d_jobs, int c
                           uint64_t* d_res64, int32_t* d_flags, uint64_t* d_words, const uint64_t* d_word_off,
                           cudaStream_t st);
 
-// ---- two-pass engine (N = 2^16 .. 2^23): state resident in HBM ------------------------------
+// ---- two-pass engine (N = 2^14 .. 2^23): state resident in HBM ------------------------------
 
 // Row-pass tiles of g rows of 2^log_c complex values that have kernels (LLG_ROW_SHAPES lists
 // them as X(log_c, g)): g * 2^log_c / (values per thread) threads, a multiple of 32 up to 512,
@@ -218,8 +218,6 @@ struct LargeArgs {
     int tw_shift;
     int C, R, nblocks;
     int q, rem;               // p / N, p % N
-    int N;                    // transform length: 2^k, or 3 x 2^k / 5 x 2^k (R = R0 L)
-    int logN;                 // log2 N for a power of two
 };
 
 constexpr size_t large_kind_words(size_t rc, int log_e) { return rc >> (log_e < 3 ? log_e : 3); }

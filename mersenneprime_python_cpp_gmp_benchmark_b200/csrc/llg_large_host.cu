@@ -290,8 +290,6 @@ cudaError_t LargeTest::init(uint64_t p_, uint64_t n, int log_c, int rows_) {
     A.nblocks = nblocks;
     A.q = (int)(p / N);
     A.rem = (int)(p % N);
-    A.N = (int)N;
-    A.logN = logN;
     return cudaSuccess;
 }
 
