@@ -75,7 +75,7 @@ double llg_get_roundoff_limit(void);
  * Replaces ntt_length(), cuda/ll_ntt.cu:172-180. */
 uint32_t llg_ntt_length(uint64_t p);
 /* Shape of the two-pass FP64 engine at N = 2^log_n (2^14 .. 2^23): rows of 2^log_c complex
- * values, columns of 2^(log_n - 1 - log_c), `rows` rows per row-pass block (2 or 4; 0: the
+ * values, columns of 2^(log_n - 1 - log_c), `rows` rows per row-pass block (2, 4 or 8; 0: the
  * default for log_c). Tests created afterwards use it; log_c < 0 restores the built-in shape. The
  * autotuner (llgpu.autotune) times the supported shapes and sets the fastest. No reference
  * counterpart (FFTW_MEASURE planning, lucaslehmer.cpp:232-242, is the nearest).
@@ -206,7 +206,9 @@ int llg_measure_peak(int which, double* ops_per_s);
 
 /* Frees the two-pass test that llg_run keeps, with its tables, buffers and graphs, after a
  * single-exponent call (one per engine, for the next call on the same exponent, length and split
- * on the same device). Idle memory of up to ~30 bytes a digit is otherwise held until then. */
+ * on the same device). Idle memory of up to ~30 bytes a digit is otherwise held until then. Also gives
+ * back the streams and the device memory (up to 512 MiB a device) that calls keep for the next one;
+ * calls running in other threads go on. */
 void llg_release_cached(void);
 
 /* Bytes the library has copied from host to device since it was loaded, all threads together
