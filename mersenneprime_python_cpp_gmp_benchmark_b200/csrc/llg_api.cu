@@ -380,6 +380,9 @@ struct Group {
     std::vector<Item> items;
     cudaStream_t st = nullptr;
     cudaEvent_t done = nullptr;
+    // the uploaded bytes (jobs, word offsets): an asynchronous copy may read pageable memory as late as
+    // the stream gets to it, so they live as long as the group (release_group waits for the stream)
+    std::vector<unsigned char> up;
     void* d_mem = nullptr;  // one allocation: every buffer below, at 256-byte offsets
     void* d_jobs = nullptr;
     uint64_t* d_word_off = nullptr;
@@ -450,8 +453,7 @@ void destroy_batch(llg_batch* b) {
     delete b;
 }
 
-// Allocates one group's buffers and uploads its job list (the pageable copy has left the host buffer
-// when the call returns).
+// Allocates one group's buffers and enqueues the upload of its job list (g.up holds it meanwhile).
 int setup_group(Group& g, int dev, bool keep_words) {
     StreamPair sp;
     CK(take_stream(dev, sp));
@@ -469,9 +471,9 @@ int setup_group(Group& g, int dev, bool keep_words) {
     const bool words = keep_words && g.n != 0;
     const size_t o_jobs = place(cnt * sizeof(SmallJob)), o_off = place(words ? cnt * sizeof(uint64_t) : 0);
     const size_t up_bytes = o;
-    std::vector<unsigned char> up(up_bytes, 0);
-    SmallJob* jobs = reinterpret_cast<SmallJob*>(up.data() + o_jobs);
-    uint64_t* off = reinterpret_cast<uint64_t*>(up.data() + o_off);
+    g.up.assign(up_bytes, 0);
+    SmallJob* jobs = reinterpret_cast<SmallJob*>(g.up.data() + o_jobs);
+    uint64_t* off = reinterpret_cast<uint64_t*>(g.up.data() + o_off);
     g.pmax = 0;
     g.total_words = 0;
     for (size_t i = 0; i < cnt; ++i) {
@@ -498,7 +500,7 @@ int setup_group(Group& g, int dev, bool keep_words) {
         g.d_word_off = reinterpret_cast<uint64_t*>(base + o_off);
         g.d_words = reinterpret_cast<uint64_t*>(base + o_words);
     }
-    CK(cudaMemcpyAsync(base, up.data(), up_bytes, cudaMemcpyHostToDevice, g.st));
+    CK(cudaMemcpyAsync(base, g.up.data(), up_bytes, cudaMemcpyHostToDevice, g.st));
     count_h2d(up_bytes);
     return LLG_OK;
 }

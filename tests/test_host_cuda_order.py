@@ -1,0 +1,78 @@
+"""The library's host code against a CUDA runtime that is as late as the documentation allows
+(fake_cudart.cpp, linked with the library's own objects): copies read their source when the stream
+gets to them, legacy-stream work stays pending until something waits for it, two devices. No GPU."""
+import ctypes
+import glob
+import os
+import subprocess
+
+import pytest
+
+from conftest import PKG, ROOT
+
+FP64, NTT, KEEP_WORDS, ERRLOG = 0, 1, 1, 2
+
+
+@pytest.fixture(scope="module")
+def fake_lib(tmp_path_factory):
+    from mersenneprime_python_cpp_gmp_benchmark_b200 import llgpu
+    out = tmp_path_factory.mktemp("fake")
+    objs = ["_build/" + os.path.splitext(os.path.basename(f))[0] + ".o"
+            for f in sorted(glob.glob(os.path.join(PKG, "csrc", "llg_*.c*"))) if f.endswith((".cu", ".cpp"))]
+    subprocess.run(["make", "-s", "-j8", "-C", PKG, *objs], check=True)
+    so = str(out / "libfake.so")
+    subprocess.run(["g++", "-std=c++17", "-O1", "-fPIC", "-shared", "-Wl,-Bsymbolic", "-I/usr/local/cuda/include",
+                    os.path.join(ROOT, "tests", "fake_cudart.cpp"), *[os.path.join(PKG, o) for o in objs],
+                    "-lpthread", "-o", so], check=True)
+    L = ctypes.CDLL(so)
+    u64, u32, i, sz, vp, P = (ctypes.c_uint64, ctypes.c_uint32, ctypes.c_int, ctypes.c_size_t, ctypes.c_void_p,
+                              ctypes.POINTER)
+    L.llg_batch_create.argtypes = [P(u64), sz, u64, i, i, P(vp)]
+    L.llg_batch_launch.argtypes = [vp, vp]
+    L.llg_batch_results.argtypes = [vp, P(llgpu.LlgResult), P(u64), sz]
+    L.llg_batch_destroy.argtypes = [vp]
+    L.llg_run.argtypes = [u64, u64, i, u32, P(llgpu.LlgResult), P(u64), sz]
+    L.llg_test_create.argtypes = [u64, u32, i, P(vp)]
+    L.llg_test_start.argtypes = [vp, vp]
+    L.llg_test_iterate.argtypes = [vp, u64, vp]
+    L.llg_test_load.argtypes = [vp, P(u64), sz, u64, vp]
+    L.llg_test_destroy.argtypes = [vp]
+    L.llg_run_noalloc.argtypes = [u64, u64, u32, vp, P(ctypes.c_double), vp]
+    L.fake_violations.restype = ctypes.c_char_p
+    L.fake_in_use.restype = L.fake_host_news.restype = u64
+    L.fake_set_free.argtypes = [u64]
+    L.Result = llgpu.LlgResult
+    return L
+
+
+@pytest.fixture
+def fake(fake_lib):
+    fake_lib.fake_set_device(0)
+    fake_lib.fake_reset()
+    yield fake_lib
+    fake_lib.fake_set_device(0)
+
+
+def _batch(L, ps, iters=20, engine=FP64, flags=0):
+    b = ctypes.c_void_p()
+    assert L.llg_batch_create((ctypes.c_uint64 * len(ps))(*ps), len(ps), iters, engine, flags, ctypes.byref(b)) == 0
+    return b
+
+
+def _results(L, b, n):
+    out = (L.Result * n)()
+    assert L.llg_batch_results(b, out, None, 0) == 0
+    return out
+
+
+# one word test, whole tests of one and of several lengths, with the word offsets of kept residues
+@pytest.mark.parametrize("ps,flags", [([127], 0), ([2203], 0), ([127, 521, 2203, 9689, 44497], KEEP_WORDS)])
+@pytest.mark.parametrize("engine", [FP64, NTT])
+def test_job_lists_live_until_their_copy_ran(fake, ps, flags, engine):
+    b = _batch(fake, ps, engine=engine, flags=flags)
+    churn = [ctypes.create_string_buffer(256) for _ in range(64)]  # reuses what the call has freed
+    assert fake.llg_batch_launch(b, None) == 0
+    _results(fake, b, len(ps))
+    fake.llg_batch_destroy(b)
+    del churn
+    assert b"source of an asynchronous copy" not in fake.fake_violations()
