@@ -116,6 +116,21 @@ int device_ready(int* dev_out) {
     return LLG_OK;
 }
 
+// A device copy of a table. A blocking copy from pageable memory may return before the bytes are on the
+// device, and the groups' non-blocking streams are not ordered against it: wait for it, once a table.
+template <class T>
+int upload_table(const std::vector<T>& h, T** out) {
+    T* d = nullptr;
+    CK(cudaMalloc(&d, h.size() * sizeof(T)));
+    cudaError_t e = cudaMemcpy(d, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice);
+    if (!e) e = cudaStreamSynchronize(nullptr);
+    if (e) cudaFree(d);
+    CK(e);
+    count_h2d(h.size() * sizeof(T));
+    *out = d;
+    return LLG_OK;
+}
+
 // A twiddle table of the whole-test FP64 kernels, built and uploaded on its first use: key 64 log2 M
 // + log2 E (pass order), log2 M alone (spread quarter table), 4096 R0 + 64 log2 L + log2 E (mixed).
 int get_table(int dev, uint32_t key, const double2** out) {
@@ -125,9 +140,8 @@ int get_table(int dev, uint32_t key, const double2** out) {
         const std::vector<double2> h = key >= 4096 ? mixed_twiddle_table((int)(key >> 12), (int)((key >> 6) & 63), (int)(key & 63))
                                        : key >= 64 ? pass_twiddle_table((int)(key >> 6), (int)(key & 63))
                                                    : spread_quarter_table(1ull << key);
-        CK(cudaMalloc(&d, h.size() * sizeof(double2)));
-        CK(cudaMemcpy(d, h.data(), h.size() * sizeof(double2), cudaMemcpyHostToDevice));
-        count_h2d(h.size() * sizeof(double2));
+        const int rc = upload_table(h, &d);
+        if (rc) return rc;
     }
     *out = d;
     return LLG_OK;
@@ -140,11 +154,8 @@ int get_ntt(int dev, int log_n, const uint64_t** qtw, NttConst* K) {
         NttConst k;
         if (!ntt_constants(log_n, k)) return fail(LLG_E_UNSUPPORTED, "no N-th root of 2 for N=2^%d", log_n);
         const std::vector<uint64_t> h = ntt_pass_table(log_n, small_ntt_values(log_n));
-        uint64_t* d = nullptr;
-        CK(cudaMalloc(&d, h.size() * sizeof(uint64_t)));
-        CK(cudaMemcpy(d, h.data(), h.size() * sizeof(uint64_t), cudaMemcpyHostToDevice));
-        count_h2d(h.size() * sizeof(uint64_t));
-        T.nqtw[log_n] = d;
+        const int rc = upload_table(h, &T.nqtw[log_n]);
+        if (rc) return rc;
         T.nk[log_n] = k;
     }
     *qtw = T.nqtw[log_n];
@@ -962,7 +973,7 @@ int make_batch(const uint64_t* ps, size_t count, uint64_t max_iters, int engine,
         b->groups[0].items.size() == 1 && b->groups[0].n) {
         b->errlog_len = b->groups[0].items[0].iters;
         e = cudaMalloc(&b->d_errlog, b->errlog_len * sizeof(float));
-        if (e == cudaSuccess) e = cudaMemset(b->d_errlog, 0, b->errlog_len * sizeof(float));
+        if (e == cudaSuccess) e = cudaMemsetAsync(b->d_errlog, 0, b->errlog_len * sizeof(float), b->groups[0].st);
     }
     if (e != cudaSuccess) {
         destroy_batch(b);

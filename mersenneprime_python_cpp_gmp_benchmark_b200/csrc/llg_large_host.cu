@@ -247,7 +247,6 @@ cudaError_t LargeTest::init(uint64_t p_, uint64_t n, int log_c, int rows_) {
     if ((e = upload(&sB, hsB))) return e;
     if ((e = cudaMalloc(&kinds, large_kind_words(M, large_row_log_e(logC, rows)) * sizeof(uint32_t)))) return e;
     if ((e = launch_fill_kinds(kinds, sA, sB, (int)N, (int)(p % N), C, R, rows, large_row_log_e(logC, rows), nullptr))) return e;
-    if ((e = cudaStreamSynchronize(nullptr))) return e;  // before any other stream reads them
     // state
     if ((e = cudaMalloc(&V, M * sizeof(double2)))) return e;
     // carry slots: one per tile plus slot 0 for the wrap-around job
@@ -260,6 +259,9 @@ cudaError_t LargeTest::init(uint64_t p_, uint64_t n, int log_c, int rows_) {
     errlog_len = 1 << 16;
     if ((e = cudaMalloc(&errlog, errlog_len * sizeof(float)))) return e;
     if ((e = cudaMemset(errlog, 0, errlog_len * sizeof(float)))) return e;
+    // the uploads, the kinds and the clears above are the legacy stream's, which the streams the test runs
+    // in need not wait for
+    if ((e = cudaStreamSynchronize(nullptr))) return e;
 
     LargeArgs& A = args;
     std::memset(&A, 0, sizeof A);
@@ -586,7 +588,6 @@ cudaError_t NttLargeTest::init(uint64_t p_, int log_n) {
     void *dV, *dc1, *dc2, *dc3, *dctl, *dd, *dfl, *dk;
     if ((e = alloc(N / 8 * sizeof(uint32_t), &dk))) return e;
     if ((e = launch_fill_ntt_kinds(static_cast<uint32_t*>(dk), csA, csB, (int)N, (int)(p & (N - 1)), C, R, nullptr))) return e;
-    if ((e = cudaStreamSynchronize(nullptr))) return e;  // before any other stream reads them
     if ((e = alloc(N * sizeof(uint64_t), &dV)) || (e = alloc((size_t)(nblocks + 1) * C * sizeof(long long), &dc1)) ||
         (e = alloc((size_t)(nblocks + 1) * C * sizeof(int), &dc2)) ||
         (e = alloc((size_t)(nblocks + 1) * C * sizeof(int), &dc3)) ||
@@ -595,6 +596,7 @@ cudaError_t NttLargeTest::init(uint64_t p_, int log_n) {
         return e;
     if ((e = cudaMemset(dctl, 0, sizeof(LargeCtl)))) return e;
     if ((e = cudaMemset(dfl, 0, (size_t)(nblocks + 1) * sizeof(unsigned)))) return e;
+    if ((e = cudaStreamSynchronize(nullptr))) return e;  // as in LargeTest::init
     ctl = static_cast<LargeCtl*>(dctl);
     digits = static_cast<int*>(dd);
     A.V = static_cast<uint64_t*>(dV);

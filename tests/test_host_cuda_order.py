@@ -76,3 +76,21 @@ def test_job_lists_live_until_their_copy_ran(fake, ps, flags, engine):
     fake.llg_batch_destroy(b)
     del churn
     assert b"source of an asynchronous copy" not in fake.fake_violations()
+
+
+# tables built on first use by every kind of test, one-exponent batches with a round-off log, and the
+# objects of both two-pass engines (power-of-two and R0 x 2^k lengths)
+def test_no_kernel_starts_beside_pending_setup(fake):
+    for p in (127, 521, 2203, 9689, 44497, 80021):
+        for engine in (FP64, NTT):
+            b = _batch(fake, [p], engine=engine, flags=ERRLOG)
+            assert fake.llg_batch_launch(b, None) == 0
+            _results(fake, b, 1)
+            fake.llg_batch_destroy(b)
+    for p, n, engine in ((300007, 1 << 14, FP64), (300007, 1 << 14, NTT), (14000017, 3 << 18, FP64)):
+        t = ctypes.c_void_p()
+        assert fake.llg_test_create(p, n, engine, ctypes.byref(t)) == 0
+        assert fake.llg_test_start(t, None) == 0
+        assert fake.llg_test_iterate(t, 3, None) == 0
+        fake.llg_test_destroy(t)
+    assert b"legacy-stream work is pending" not in fake.fake_violations()
