@@ -149,7 +149,8 @@ int llg_test_errlog(llg_test* t, float* log, size_t cap, size_t* len);
 /* Sets the test's state to a residue s (ceil(p/64) little-endian limbs, s < 2^p) reached after
  * `iters_done` squarings and starts the next squaring, as llg_test_start does from s_0 = 4. The
  * digits are formed on the GPU at the test's own length, so a residue from any length (or from
- * another engine) resumes here; llg_test_read's words are such a residue. Replaces restarting
+ * another engine) resumes here; llg_test_read's words are such a residue. `words` has been read when
+ * the call returns (it waits for its copy in `stream`). Replaces restarting
  * lucas_lehmer_fft_raw() from s_0 (lucaslehmer.cpp:272-273) after a round-off abort
  * (lucaslehmer.cpp:296, 334): a test moved to a longer length goes on from its last residue. */
 int llg_test_load(llg_test* t, const uint64_t* words, size_t nwords, uint64_t iters_done, void* stream);

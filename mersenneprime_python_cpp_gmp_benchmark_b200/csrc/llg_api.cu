@@ -1522,6 +1522,11 @@ int llg_test_load(llg_test* t, const uint64_t* words, size_t nwords, uint64_t it
     CK(pool_malloc(reinterpret_cast<void**>(&dw), nw * sizeof(uint64_t), st));
     cudaError_t e = cudaMemcpyAsync(dw, words, nw * sizeof(uint64_t), cudaMemcpyHostToDevice, st);
     count_h2d(nw * sizeof(uint64_t));
+    // the words are the caller's again on return, so their copy is waited for (a copy that is being
+    // captured reads them when the graph runs)
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (e == cudaSuccess) e = cudaStreamIsCapturing(st, &cap);
+    if (e == cudaSuccess && cap == cudaStreamCaptureStatusNone) e = cudaStreamSynchronize(st);
     int* digits = t->f ? t->f->digits : t->n->digits;
     if (e == cudaSuccess) e = digits_from_words(p, t->len(), dw, digits, st);
     if (e == cudaSuccess) e = t->f ? t->f->start_device(st) : t->n->start_device(st);

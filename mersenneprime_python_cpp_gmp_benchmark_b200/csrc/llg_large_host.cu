@@ -378,6 +378,7 @@ cudaError_t LargeTest::diag_withhold_wrap(unsigned long long spin_limit, cudaStr
     const unsigned long long next = h.tickets + 1;
     count_h2d(sizeof next);
     if ((e = cudaMemcpyAsync(&ctl->tickets, &next, sizeof next, cudaMemcpyHostToDevice, st))) return e;
+    if ((e = cudaStreamSynchronize(st))) return e;  // `next` is read by then
     LargeArgs a = args;
     a.spin_limit = spin_limit;
     if ((e = launch_large_row(logC, rows, LARGE_ITER, a, st, nblocks))) return e;

@@ -321,6 +321,10 @@ FAKE cudaError_t cudaStreamEndCapture(cudaStream_t st, cudaGraph_t* g) {
     *g = nullptr;
     return cudaSuccess;
 }
+FAKE cudaError_t cudaStreamIsCapturing(cudaStream_t st, enum cudaStreamCaptureStatus* out) {
+    *out = get(st)->capturing ? cudaStreamCaptureStatusActive : cudaStreamCaptureStatusNone;
+    return cudaSuccess;
+}
 FAKE cudaError_t cudaGraphInstantiate(cudaGraphExec_t* e, cudaGraph_t, unsigned long long) {
     static int dummy;
     *e = reinterpret_cast<cudaGraphExec_t>(&dummy);

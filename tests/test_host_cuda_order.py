@@ -94,3 +94,17 @@ def test_no_kernel_starts_beside_pending_setup(fake):
         assert fake.llg_test_iterate(t, 3, None) == 0
         fake.llg_test_destroy(t)
     assert b"legacy-stream work is pending" not in fake.fake_violations()
+
+
+def test_loaded_residue_is_the_callers_again_on_return(fake):
+    p, n = 300007, 1 << 14
+    for engine in (FP64, NTT):
+        t = ctypes.c_void_p()
+        assert fake.llg_test_create(p, n, engine, ctypes.byref(t)) == 0
+        words = (ctypes.c_uint64 * ((p + 63) // 64))(*range(1, (p + 63) // 64 + 1))
+        words[-1] = 0
+        assert fake.llg_test_load(t, words, len(words), 5, None) == 0
+        words[0] = 99  # the call is over: the buffer may be reused
+        assert fake.llg_test_iterate(t, 2, None) == 0
+        fake.llg_test_destroy(t)  # waits
+    assert b"source of an asynchronous copy" not in fake.fake_violations()
