@@ -304,6 +304,7 @@ void destroy_pair(const StreamPair& sp) {
     if (sp.done) cudaEventDestroy(sp.done);
 }
 
+// A stream and an event of `dev`, which is the current device.
 cudaError_t take_stream(int dev, StreamPair& out) {
     {
         std::lock_guard<std::mutex> lk(g_res_mx);
@@ -999,9 +1000,24 @@ int launch_batch(llg_batch* b, cudaStream_t caller) {
     return LLG_OK;
 }
 
-// Collects every group; round-off aborts are rerun (synchronously) at longer lengths until done.
+// Makes `dev` the current device for a scope.
+struct OnDevice {
+    int old = -1;
+    explicit OnDevice(int dev) {
+        if (cudaGetDevice(&old) != cudaSuccess || old == dev || cudaSetDevice(dev) != cudaSuccess) old = -1;
+    }
+    ~OnDevice() {
+        if (old >= 0) cudaSetDevice(old);
+    }
+    OnDevice(const OnDevice&) = delete;
+    OnDevice& operator=(const OnDevice&) = delete;
+};
+
+// Collects every group, on the batch's device (the reading thread's current one may be another: the
+// reruns' streams, memory and tables belong to the batch's); round-off aborts are rerun (synchronously) at longer lengths until done.
 int collect_batch(llg_batch* b) {
     if (b->collected) return LLG_OK;
+    const OnDevice on(b->dev);
     b->word_bufs.clear();
     b->word_view.assign(b->keep_words ? b->count : 0, llg_batch::WordView{});
     std::vector<Item> retry;

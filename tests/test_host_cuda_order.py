@@ -108,3 +108,23 @@ def test_loaded_residue_is_the_callers_again_on_return(fake):
         assert fake.llg_test_iterate(t, 2, None) == 0
         fake.llg_test_destroy(t)  # waits
     assert b"source of an asynchronous copy" not in fake.fake_violations()
+
+
+def test_redone_tests_stay_on_the_batchs_device(fake):
+    """A batch collected by a thread whose current device is another one: its round-off redo runs on the
+    batch's device, and the stream it used is not handed to later calls of the wrong device."""
+    b = _batch(fake, [521])
+    assert fake.llg_batch_launch(b, None) == 0
+    fake.fake_script_status(1, 1)  # round-off above the limit: redone at the next length
+    fake.fake_set_device(1)
+    out = _results(fake, b, 1)
+    assert out[0].escalations == 1
+    fake.llg_batch_destroy(b)
+    ps = [127, 521, 2203, 9689]  # a group and a stream each
+    for dev in (0, 1, 0):
+        fake.fake_set_device(dev)
+        b = _batch(fake, ps)
+        assert fake.llg_batch_launch(b, None) == 0
+        _results(fake, b, len(ps))
+        fake.llg_batch_destroy(b)
+    assert b"device" not in fake.fake_violations()
