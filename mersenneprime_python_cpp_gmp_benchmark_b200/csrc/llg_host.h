@@ -28,7 +28,9 @@ std::vector<double2> padded_quarter_table(uint64_t L);
 double2 padded_quarter_slot(uint64_t L, uint64_t i);
 // The same quarter-wave table in the spread layout (entry r at qpad_s(r)).
 std::vector<double2> spread_quarter_table(uint64_t L);
-// The twiddles of an L-point FFT of 2^log_e values a thread, pass by pass (TW_PASS).
+// The twiddles of an L-point FFT of 2^log_e values a thread, pass by pass (TW_PASS); write_pass_twiddles
+// writes them to `out` (fewer than L values) and returns their number.
+size_t write_pass_twiddles(int log_l, int log_e, double2* out);
 std::vector<double2> pass_twiddle_table(int log_l, int log_e);
 // pass_twiddle_table(log_l, log_e), then w_M^{n k0} over n < L for k0 = 1 .. r0 - 1 (M = r0 L, L = 2^log_l).
 std::vector<double2> mixed_twiddle_table(int r0, int log_l, int log_e);

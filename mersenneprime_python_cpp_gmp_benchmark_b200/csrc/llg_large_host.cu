@@ -70,9 +70,9 @@ std::vector<double2> spread_quarter_table(uint64_t L) {
     return t;
 }
 
-std::vector<double2> pass_twiddle_table(int log_l, int log_e) {
+size_t write_pass_twiddles(int log_l, int log_e, double2* out) {
     const uint64_t L = 1ull << log_l, E = 1ull << log_e;
-    std::vector<double2> t;
+    size_t n = 0;
     const long double two_pi = 6.283185307179586476925286766559005768L;
     // pass s: groups of len values in R strides of st; w_len^(n2 k1) = w_L^(n2 k1 L / len)
     for (uint64_t len = L; len > E || (len > 1 && len == L); len /= E) {
@@ -81,9 +81,15 @@ std::vector<double2> pass_twiddle_table(int log_l, int log_e) {
         for (uint64_t k1 = 1; k1 < E; ++k1)
             for (uint64_t n2 = 0; n2 < st; ++n2) {
                 const long double ang = two_pi * (long double)((n2 * k1 * (L / len)) % L) / (long double)L;
-                t.push_back(make_double2((double)cosl(ang), -(double)sinl(ang)));
+                out[n++] = make_double2((double)cosl(ang), -(double)sinl(ang));
             }
     }
+    return n;
+}
+
+std::vector<double2> pass_twiddle_table(int log_l, int log_e) {
+    std::vector<double2> t(1ull << log_l);
+    t.resize(write_pass_twiddles(log_l, log_e, t.data()));
     return t;
 }
 

@@ -32,7 +32,6 @@
 #include <cstdio>
 #include <cstring>
 #include <mutex>
-#include <vector>
 
 #include "../../include/llgpu.h"
 #include "llg_device.cuh"
@@ -54,8 +53,9 @@ static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocScratch
 std::mutex g_noalloc_mx;
 unsigned char* g_scratch_addr[kMaxDevices] = {};
 
-// Host staging for the tables (no host allocation either): the largest table set is ~24 KiB. The
-// tables are laid out contiguously in the array (qtwC .. sB), so one copy moves all of them.
+// Host staging for the tables (no host allocation either): the largest table set is 31 KiB. The
+// tables are laid out contiguously in the array (qtwC .. sB), so one copy moves all of them; the digit
+// kinds after them are formed on the device from sA and sB.
 constexpr size_t kStageBytes = 64u * 1024u;
 alignas(256) unsigned char g_stage[kStageBytes];
 // (p, n) whose tables the array holds, per device: a repeated call skips the upload
@@ -186,10 +186,7 @@ extern "C" int llg_run_noalloc(uint64_t p, uint64_t iters, uint32_t n, int32_t* 
         const long double Nl = (long double)N;
         const size_t o = L.qtwC;
         std::memset(g_stage, 0, L.kinds - o);
-        {
-            const std::vector<double2> t = pass_twiddle_table(logC, large_row_log_e(logC, kTileRows));  // < C values
-            std::memcpy(g_stage + (L.qtwC - o), t.data(), t.size() * sizeof(double2));
-        }
+        write_pass_twiddles(logC, large_row_log_e(logC, kTileRows), reinterpret_cast<double2*>(g_stage + (L.qtwC - o)));
         {  // the column pass's quarter table in the spread layout: entry r at qpad_s(r)
             double2* q = reinterpret_cast<double2*>(g_stage + (L.qtwR - o));
             for (uint32_t r = 0; r < (uint32_t)R / 4; ++r) q[qpad_s(r)] = padded_quarter_slot(R, qpad(r));

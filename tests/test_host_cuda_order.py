@@ -128,3 +128,12 @@ def test_redone_tests_stay_on_the_batchs_device(fake):
         _results(fake, b, len(ps))
         fake.llg_batch_destroy(b)
     assert b"device" not in fake.fake_violations()
+
+
+def test_noalloc_allocates_no_host_memory_either(fake):
+    out = (ctypes.c_int32 * 65536)()  # the fake's device memory is host memory
+    err = ctypes.c_double()
+    for p, n in ((300007, 1 << 14), (600011, 1 << 15), (1257787, 1 << 16)):
+        before = fake.fake_host_news()
+        assert fake.llg_run_noalloc(p, 3, n, out, ctypes.byref(err), None) == 0
+        assert fake.fake_host_news() == before, n
