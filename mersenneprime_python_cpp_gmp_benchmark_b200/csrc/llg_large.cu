@@ -213,8 +213,7 @@ __global__ void __launch_bounds__(large_row_threads(LOG_C, G), large_row_min_blo
             const double vb = v[i].y * scale_up(ia1 * iwb, kind(i, 3));
             long long ia, ib;
             const double r0 = round_shift(va, ia), r1 = round_shift(vb, ib);
-            err.add(va - r0);
-            err.add(vb - r1);
+            err.add(va - r0, vb - r1);
             double c, c1, c2 = 0.0;
             double x0 = dsplit_k(r0, dq, kind(i, 0), c);
             double x1 = dsplit_k(r1 + c, dq, kind(i, 1), c1);
@@ -234,8 +233,8 @@ __global__ void __launch_bounds__(large_row_threads(LOG_C, G), large_row_min_blo
         }
         if (wrap_job) return;
         // the tile's round-off max: one shared atomic per warp
-        err.m = __reduce_max_sync(FULL, err.m);
-        if ((t & 31) == 0) atomicMax(&s_err, (unsigned long long)__double_as_longlong(err.value()));
+        const unsigned long long werr = warp_max(err.value());
+        if ((t & 31) == 0) atomicMax(&s_err, werr);
         __syncthreads();  // every thread has left the inverse FFT's exchange buffer
         if (t == 0) {
             const unsigned long long eb = s_err;

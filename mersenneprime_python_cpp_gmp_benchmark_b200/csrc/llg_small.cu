@@ -213,8 +213,7 @@ __global__ void __launch_bounds__(SmallGeo<LOG_M, LE>::T, small_min_blocks(Small
                 const double b = v[i].y * scale_up(iwA1 * iw, kind(i, 3));
                 long long la, lb;
                 const double ra = round_shift(a, la), rb = round_shift(b, lb);
-                err.add(a - ra);
-                err.add(b - rb);
+                err.add(a - ra, b - rb);
                 double cy;
                 x0[i] = dsplit_k(ra, dq, kind(i, 0), cy);
                 x1[i] = dsplit_k(rb + cy, dq, kind(i, 1), c[i]);
@@ -244,8 +243,7 @@ __global__ void __launch_bounds__(SmallGeo<LOG_M, LE>::T, small_min_blocks(Small
                 const double b = v[i].y * scale_up(iwA1 * iw, kind(i, 3));
                 long long la, lb;
                 const double ra = round_shift(a, la), rb = round_shift(b, lb);
-                err.add(a - ra);
-                err.add(b - rb);
+                err.add(a - ra, b - rb);
                 double c;
                 const double x0 = dsplit_k(ra, dq, kind(i, 0), c);
                 const double x1 = dsplit_k(rb + c, dq, kind(i, 1), c);

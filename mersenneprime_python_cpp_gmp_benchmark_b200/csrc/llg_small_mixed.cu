@@ -277,8 +277,7 @@ __global__ void __launch_bounds__(MixedGeom<R0, LOG_L, LE, MINB>::T, MINB)
                 const double b = z[r].y * scale_up(iwA1 * iw, kind(c, 3));
                 long long la, lb;
                 const double ra = round_shift(a, la), rb = round_shift(b, lb);
-                err.add(a - ra);
-                err.add(b - rb);
+                err.add(a - ra, b - rb);
                 double cy;
                 double x0 = dsplit_k(ra, dq, kind(c, 0), cy);
                 const double x1 = dsplit_k(rb + cy, dq, kind(c, 1), cy);
