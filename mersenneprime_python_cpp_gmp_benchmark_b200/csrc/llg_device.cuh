@@ -1,7 +1,7 @@
 // Device-side building blocks shared by the Lucas-Lehmer kernels (sm_100a):
 //   * complex FP64 arithmetic on double2 and fixed-radix in-register DFTs (2, 4, 8, 16 points);
 //   * twiddles from a quarter-wave table (one load and a rotation by a power of -i);
-//   * round-to-nearest with the 1.5*2^52 shifter, which also yields the integer in the low bits;
+//   * round-to-nearest with the 1.5*2^52 shifter;
 //   * the balanced-digit carry step of the irrational-base DWT.
 //
 // The arithmetic follows the IBDWT of the reference's FFT engine (lucaslehmer.cpp:257-311):
@@ -192,13 +192,10 @@ __device__ __forceinline__ double2 twiddle(const double2* __restrict__ q, uint32
     return inv ? conj2(r) : r;
 }
 
-// Round to nearest even with the 1.5*2^52 shifter (valid for |v| < 2^51): returns the rounded
-// double and the same integer as int64.
-__device__ __forceinline__ double round_shift(double v, long long& iv) {
+// Round to nearest even with the 1.5*2^52 shifter (valid for |v| < 2^51).
+__device__ __forceinline__ double round_shift(double v) {
     constexpr double SH = 6755399441055744.0;  // 1.5 * 2^52
-    const double t = __dadd_rn(v, SH);
-    iv = __double_as_longlong(t) - 0x4338000000000000LL;
-    return __dsub_rn(t, SH);
+    return __dsub_rn(__dadd_rn(v, SH), SH);
 }
 
 // Exact conversion of a small signed integer (|x| < 2^51) to double by the same shifter.

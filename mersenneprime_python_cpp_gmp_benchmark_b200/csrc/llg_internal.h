@@ -156,7 +156,8 @@ constexpr bool large_row_pass_table(int log_c, int g) { return large_row_log_e(l
 
 struct LargeCtl {
     unsigned long long tickets;      // FP64 row-pass tickets taken since the start
-    unsigned int epoch;              // squarings whose column pass has finished; +1 per column pass
+    unsigned int epoch;              // squarings whose column pass has finished; +1 per column pass. The
+                                     // NTT row pass reads it; an FP64 one counts by its tickets
     unsigned int ticket[2];          // NTT row-pass block tickets, alternating by epoch parity
     unsigned int timeout;            // set when a bounded wait gave up (the result is then invalid)
     unsigned long long err_max;      // bits of the max round-off over the run (double, >= 0)
@@ -217,7 +218,7 @@ struct LargeArgs {
     int pdl_late;             // where the passes let the next one launch: at their end, or at their start
     int tw_shift;
     int C, R, nblocks;
-    int q, rem;               // p / N, p % N
+    int q;                    // p / N
 };
 
 constexpr size_t large_kind_words(size_t rc, int log_e) { return rc >> (log_e < 3 ? log_e : 3); }
@@ -258,7 +259,7 @@ struct NttLargeArgs {
     int pdl_late;             // as LargeArgs::pdl_late
     int tw_shift;
     int C, R, nblocks;
-    int q, rem;
+    int q;
     int logN;
 };
 

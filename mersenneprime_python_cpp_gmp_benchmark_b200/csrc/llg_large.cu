@@ -211,8 +211,7 @@ __global__ void __launch_bounds__(large_row_threads(LOG_C, G), large_row_min_blo
             const double iwb = siwB[b];
             const double va = v[i].x * scale_up(ia0 * iwb, kind(i, 2));
             const double vb = v[i].y * scale_up(ia1 * iwb, kind(i, 3));
-            long long ia, ib;
-            const double r0 = round_shift(va, ia), r1 = round_shift(vb, ib);
+            const double r0 = round_shift(va), r1 = round_shift(vb);
             err.add(va - r0, vb - r1);
             double c, c1, c2 = 0.0;
             double x0 = dsplit_k(r0, dq, kind(i, 0), c);
@@ -661,11 +660,6 @@ static cudaError_t col_attr_le() {
 }
 template <int LOG_R>
 static cudaError_t col_attr() {
-#ifdef LLG_PROBE_LE
-    if constexpr (LOG_R <= 10) { col_attr_le<LOG_R, 2>(); }
-    col_attr_le<LOG_R, 3>();
-    return col_attr_le<LOG_R, 4>();
-#endif
     return col_attr_le<LOG_R, large_col_log_e(LOG_R)>();
 }
 
@@ -727,13 +721,6 @@ static cudaError_t col_le(const LargeArgs& a, cudaStream_t st) {
 }
 template <int LOG_R>
 static cudaError_t col_t(const LargeArgs& a, cudaStream_t st) {
-#ifdef LLG_PROBE_LE
-    const char* ev = getenv("LLG_CLE");
-    const int le = ev ? atoi(ev) : 4;
-    if constexpr (LOG_R <= 10) if (le == 2) return col_le<LOG_R, 2>(a, st);
-    if (le == 3) return col_le<LOG_R, 3>(a, st);
-    return col_le<LOG_R, 4>(a, st);
-#endif
     return col_le<LOG_R, large_col_log_e(LOG_R)>(a, st);
 }
 

@@ -297,7 +297,6 @@ cudaError_t LargeTest::init(uint64_t p_, uint64_t n, int log_c, int rows_) {
     A.R = R;
     A.nblocks = nblocks;
     A.q = (int)(p / N);
-    A.rem = (int)(p % N);
     return cudaSuccess;
 }
 
@@ -630,7 +629,6 @@ cudaError_t NttLargeTest::init(uint64_t p_, int log_n) {
     A.R = R;
     A.nblocks = nblocks;
     A.q = (int)(p >> logN);
-    A.rem = (int)(p & (N - 1));
     A.logN = logN;
     return cudaSuccess;
 }

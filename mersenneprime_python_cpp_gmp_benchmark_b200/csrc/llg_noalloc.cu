@@ -245,7 +245,6 @@ extern "C" int llg_run_noalloc(uint64_t p, uint64_t iters, uint32_t n, int32_t* 
     A.nblocks = R / kTileRows;
     A.pdl_late = large_pdl_late(N);
     A.q = (int)(p >> logN);
-    A.rem = (int)(p & (N - 1));
 
     // s_0 = 4 as digits (the output buffer doubles as the INIT input), control block cleared.
     // From the first enqueue on, a failure waits for the stream before returning.

@@ -48,9 +48,6 @@ __device__ __forceinline__ uint64_t sub(uint64_t a, uint64_t b) {
 // a + b for any a and canonical b: a - (q - b); canonical when a is.
 __device__ __forceinline__ uint64_t add(uint64_t a, uint64_t b) { return sub(a, Q - b); }
 
-// The canonical form of any a.
-__device__ __forceinline__ uint64_t canon(uint64_t a) { return sub(a, Q); }
-
 // Montgomery product a b 2^-64 mod q; canonical when a or b is (then xh <= q - 1, so xh + r1 does
 // not overflow), any otherwise excluded: one operand must be canonical.
 __device__ __forceinline__ uint64_t mul(uint64_t a, uint64_t b) {

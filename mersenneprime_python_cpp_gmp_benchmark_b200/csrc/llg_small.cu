@@ -211,8 +211,7 @@ __global__ void __launch_bounds__(SmallGeo<LOG_M, LE>::T, small_min_blocks(Small
                 const double iw = iwB[i];
                 const double a = v[i].x * scale_up(iwA0 * iw, kind(i, 2));
                 const double b = v[i].y * scale_up(iwA1 * iw, kind(i, 3));
-                long long la, lb;
-                const double ra = round_shift(a, la), rb = round_shift(b, lb);
+                const double ra = round_shift(a), rb = round_shift(b);
                 err.add(a - ra, b - rb);
                 double cy;
                 x0[i] = dsplit_k(ra, dq, kind(i, 0), cy);
@@ -241,8 +240,7 @@ __global__ void __launch_bounds__(SmallGeo<LOG_M, LE>::T, small_min_blocks(Small
                 const double iw = iwB[i];
                 const double a = v[i].x * scale_up(iwA0 * iw, kind(i, 2));
                 const double b = v[i].y * scale_up(iwA1 * iw, kind(i, 3));
-                long long la, lb;
-                const double ra = round_shift(a, la), rb = round_shift(b, lb);
+                const double ra = round_shift(a), rb = round_shift(b);
                 err.add(a - ra, b - rb);
                 double c;
                 const double x0 = dsplit_k(ra, dq, kind(i, 0), c);

@@ -207,7 +207,7 @@ __global__ void __launch_bounds__(MixedGeom<R0, LOG_L, LE, MINB>::T, MINB)
 #pragma unroll
                 for (int r = 0; r < R0; ++r) {
                     const int c = i + NPT * r;
-                        const double w = wB[c];
+                    const double w = wB[c];
                     z[r] = make_double2(i2d_shift(x0s[c]) * scale_down(wA0 * w, kind(c, 2)),
                                         i2d_shift(x1s[c]) * scale_down(wA1 * w, kind(c, 3)));
                 }
@@ -271,26 +271,25 @@ __global__ void __launch_bounds__(MixedGeom<R0, LOG_L, LE, MINB>::T, MINB)
                 dft_r0<R0, true>(z);
 #pragma unroll
                 for (int r = 0; r < R0; ++r) {
-                const int c = i + NPT * r;
-                const double iw = iwB[c];
-                const double a = z[r].x * scale_up(iwA0 * iw, kind(c, 2));
-                const double b = z[r].y * scale_up(iwA1 * iw, kind(c, 3));
-                long long la, lb;
-                const double ra = round_shift(a, la), rb = round_shift(b, lb);
-                err.add(a - ra, b - rb);
-                double cy;
-                double x0 = dsplit_k(ra, dq, kind(c, 0), cy);
-                const double x1 = dsplit_k(rb + cy, dq, kind(c, 1), cy);
-                const double cout = cy;
-                if (lane == 31) cbuf[warp * CA + c] = cout;
-                const double cin = __shfl_up_sync(0xffffffffu, cout, 1);
-                if (lane != 0) {
-                    x0 = dsplit_k(x0 + cin, dq, kind(c, 0), cy);
-                    x1s[c] = d2i_exact(x1 + cy);
-                } else {
-                    x1s[c] = d2i_exact(x1);
-                }
-                x0s[c] = d2i_exact(x0);
+                    const int c = i + NPT * r;
+                    const double iw = iwB[c];
+                    const double a = z[r].x * scale_up(iwA0 * iw, kind(c, 2));
+                    const double b = z[r].y * scale_up(iwA1 * iw, kind(c, 3));
+                    const double ra = round_shift(a), rb = round_shift(b);
+                    err.add(a - ra, b - rb);
+                    double cy;
+                    double x0 = dsplit_k(ra, dq, kind(c, 0), cy);
+                    const double x1 = dsplit_k(rb + cy, dq, kind(c, 1), cy);
+                    const double cout = cy;
+                    if (lane == 31) cbuf[warp * CA + c] = cout;
+                    const double cin = __shfl_up_sync(0xffffffffu, cout, 1);
+                    if (lane != 0) {
+                        x0 = dsplit_k(x0 + cin, dq, kind(c, 0), cy);
+                        x1s[c] = d2i_exact(x1 + cy);
+                    } else {
+                        x1s[c] = d2i_exact(x1);
+                    }
+                    x0s[c] = d2i_exact(x0);
                 }
             }
         }
