@@ -204,7 +204,7 @@ __global__ void __launch_bounds__(large_row_threads(LOG_C, G), large_row_min_blo
         if (wrap_job && t == 0) *reinterpret_cast<volatile unsigned*>(A.wrap_read) = ep + 1u;  // its rows are read
         LargeCarry* pub = A.carry + (size_t)(job + 1) * C;
         const double ia0 = __ldg(A.iwA + 2 * a), ia1 = __ldg(A.iwA + 2 * a + 1);
-        ErrMax err;
+        ErrMax<1> err;
 #pragma unroll
         for (int i = 0; i < E; ++i) {
             const int b = tr + TR * i;

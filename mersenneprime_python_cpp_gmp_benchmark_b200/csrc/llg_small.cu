@@ -199,7 +199,7 @@ __global__ void __launch_bounds__(SmallGeo<LOG_M, LE>::T, small_min_blocks(Small
 
         // unweight, round, error, local carry (even -> odd digit); the carry-out of column i goes
         // to thread t+1 (lane shuffle) or, at a warp boundary, through cbuf after the barrier
-        ErrMax err;
+        ErrMax<2> err;
         double lerr;
         int bad;
         refresh_kinds();

@@ -259,7 +259,7 @@ __global__ void __launch_bounds__(MixedGeom<R0, LOG_L, LE, MINB>::T, MINB)
 
         // ---- inverse radix-R0 DFT back to the thread's columns, then unweight, round and carry
         //      each column (the columns' carries are independent until the exchange below) ----
-        ErrMax err;
+        ErrMax<2> err;
         refresh_kinds();
         if (holds) {
 #pragma unroll

@@ -18,7 +18,7 @@ SOURCE = r"""
 #include <vector>
 #include "llg_device.cuh"
 __global__ void k(const double* x, int n, unsigned long long* out) {
-    llg::ErrMax e;
+    llg::ErrMax<COUNT> e;
     for (int i = 0; i < n; ++i) e.add(x[2 * (32 * i + threadIdx.x)], x[2 * (32 * i + threadIdx.x) + 1]);
     const unsigned long long w = llg::warp_max(e.value());
     if (threadIdx.x == 0) *out = w;
@@ -47,9 +47,10 @@ def _bits(x):
     return struct.unpack("<Q", struct.pack("<d", x))[0]
 
 
-def test_warp_maximum_is_exact(gpu, tmp_path):
+@pytest.mark.parametrize("chains", [1, 2])
+def test_warp_maximum_is_exact(gpu, tmp_path, chains):
     src, exe = tmp_path / "m.cu", tmp_path / "m"
-    src.write_text(SOURCE)
+    src.write_text(SOURCE.replace("COUNT", str(chains)))
     subprocess.run(["nvcc", "-std=c++17", "-O3", "-gencode", "arch=compute_100a,code=sm_100a", "-I",
                     os.path.join(PKG, "csrc"), str(src), "-o", str(exe)], check=True)
     rng = random.Random(5)
@@ -74,6 +75,6 @@ def test_warp_maximum_is_exact(gpu, tmp_path):
     out = subprocess.run([str(exe)], input=text, capture_output=True, text=True, check=True).stdout.split()
     assert [int(x, 16) for x in out] == [_bits(max(abs(x) for x in v)) for v in cases]
     # not a number (it spreads to a whole transform's outputs) exceeds every bound
-    nan = f"1 " + " ".join(f"{_bits(math.nan):x}" for _ in range(64))
+    nan = "1 " + " ".join(f"{_bits(math.nan):x}" for _ in range(64))
     out = subprocess.run([str(exe)], input=nan, capture_output=True, text=True, check=True).stdout.split()
     assert int(out[0], 16) == _bits(math.inf)
