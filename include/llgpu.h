@@ -208,7 +208,8 @@ int llg_measure_peak(int which, double* ops_per_s);
 /* Frees the two-pass test that llg_run keeps, with its tables, buffers and graphs, after a
  * single-exponent call (one per engine, for the next call on the same exponent, length and split
  * on the same device). Idle memory of up to ~30 bytes a digit is otherwise held until then. Also gives
- * back the streams and the device memory (up to 512 MiB a device) that calls keep for the next one;
+ * back the streams and the device memory (up to 512 MiB a device) that calls keep for the next one
+ * (cudaMalloc in the same process takes that memory when the device is full; other processes do not);
  * calls running in other threads go on. */
 void llg_release_cached(void);
 

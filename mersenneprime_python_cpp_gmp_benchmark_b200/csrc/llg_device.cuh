@@ -261,13 +261,13 @@ __device__ __forceinline__ double dsplit_k(double v, const DigitBase& B, uint32_
 
 // Largest |d| of a run of differences, to the last bit: it is compared with the round-off bound, reported
 // and logged. The whole-test kernels keep two maxima side by side, for the even and the odd digits: one
-// chain of compares and selects was slower there (1184 tests at N = 1024 12.42 us a squaring against 12.33,
-// at 2048 20.4 against 20.3) and faster in the row kernels of 16 values a thread, which are short of
-// registers (2^23 137.9 against 139.6; the others within .6% either way). A maximum of high words alone takes .6 to 2.7% less with
-// many tests an SM (N = 1024 12.26, 2048 20.13, 592 tests at 4096 14.01 against 14.37, at 6144 27.9 against
-// 28.4) and up to 1% less in the row kernels (2^23 137.7, 2^22 64.6 against 65.3), but holds 20 bits of
-// mantissa and rounds down. Not-a-number counts as infinite when it ends a run; a transform spreads one
-// such value to all of its outputs.
+// chain of compares and selects was slower there (1184 tests at N = 1024 12.42 us a squaring against
+// 12.33, at 2048 20.4 against 20.3) and faster in the row kernels of 16 values a thread, which are short
+// of registers (2^23 137.9 against 139.6; the others within .6% either way). A maximum of high words
+// alone takes .6 to 2.7% less with many tests an SM (N = 1024 12.26, 2048 20.13, 592 tests at 4096 14.01
+// against 14.37, at 6144 27.9 against 28.4) and up to 1% less in the row kernels (2^23 137.7, 2^22 64.6
+// against 65.3), but holds 20 bits of mantissa and rounds down. Not-a-number counts as infinite when it
+// ends a run; a transform spreads one such value to all of its outputs.
 template <int CHAINS>
 struct ErrMax {
     double m[CHAINS] = {};

@@ -154,8 +154,8 @@ bool large_mixed_length_supported(uint64_t n, int* r0, int* log_c) {
 
 // Row length (2^log_c complex values) and rows per tile of the two-pass FP64 engine at N = 2^log_n by
 // default: the fastest of the supported shapes on a B200. us a squaring, this shape / the default
-// before: 2^14 6.2 / 9.8, 2^15 6.4 / 12.3, 2^16 7.0 / 13.1, 2^17 7.9 / 13.7, 2^18 8.9 / 26.3, 2^19 12.1 / 29.9, 2^20
-// 18.3 / 34.5, 2^21 32.3 / 41.2, 2^22 64.7 / 76.5, 2^23 138 / 156.
+// before: 2^14 6.2 / 9.8, 2^15 6.3 / 12.3, 2^16 7.0 / 13.1, 2^17 7.9 / 13.7, 2^18 8.8 / 26.3, 2^19 12.5 / 29.9, 2^20
+// 18.4 / 34.5, 2^21 32.4 / 41.2, 2^22 65.4 / 76.5, 2^23 138 / 156.
 int large_default_log_c(int log_n) {
     return log_n <= 15 ? 6 : log_n <= 17 ? 7 : log_n == 19 ? 9 : log_n <= 21 ? 8 : log_n == 22 ? 9 : 10;
 }

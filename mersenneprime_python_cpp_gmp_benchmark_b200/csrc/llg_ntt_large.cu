@@ -23,7 +23,7 @@
 //
 // Both passes are bound by the integer ALU (the arithmetic of llg_ntt.cuh). Measured, us a squaring
 // replayed from graphs, against radix-16 passes of one row per warp group with the 128-bit
-// reduction: N = 2^16 55.5 -> 17.5, 2^18 67.3 -> 23.2, 2^21 176.8 -> 106.9, 2^23 654 -> 432. At 2^21 the
+// reduction: N = 2^16 55.5 -> 17.7, 2^18 67.3 -> 23.2, 2^21 176.8 -> 106.9, 2^23 654 -> 431. At 2^21 the
 // row pass issued 37.2 M warp instructions (47.3 M before) at 57% of the ALU's rate (39%), the
 // column pass 31.1 M at 67% (58%); neither waits for instruction fetch any more (5.5 cycles per
 // issued instruction before). Kinds from a table and pass-ordered twiddles then took the row pass at
@@ -323,7 +323,7 @@ static size_t ntt_col_smem() {
     return sizeof(uint64_t) * (GR::PAD + gl::table_len<GR>() + 4 * GR::E);
 }
 
-// Programmatic stream serialisation, as the FP64 passes at power-of-two lengths.
+// Programmatic stream serialisation, as the FP64 passes.
 template <class... KArgs>
 static cudaError_t launch_pdl(void (*kernel)(KArgs...), int grid, int block, size_t smem, cudaStream_t st,
                               const NttLargeArgs& a) {

@@ -49,6 +49,8 @@ __host__ __device__ constexpr int small_tw_layout(int le) { return le >= 4 ? TW_
 //   1184 tests    N = 32 2.5 (4 values); 64 2.1; 128 2.7; 256 2.9 (8); 512 6.4 (8); 1024 14.9 (8);
 //                 2048 25.7 (8); 592 tests: 4096 17.0 (16), 17.4 (8)
 //        before   15.8, 11.2, 7.4, 10.1, 9.4, 16.9, 34.6, 17.0
+// With the digits as doubles and the kinds in the exponent field, the chosen forms now: one test .54, .64,
+// .73, 1.02, 1.25, 1.90, 2.65, 4.58, 8.3; 1184 tests 2.1, 1.8, 2.5, 3.1, 5.9, 14.1, 23.0, 592 at 4096 14.6.
 // Above one test per SM (small_fp64_log_e) the batch form runs.
 __host__ __device__ constexpr int small_log_e_alone(int log_m) {
     return log_m <= 5 ? 1 : log_m <= 8 ? 2 : log_m <= 11 ? 3 : 4;
@@ -72,7 +74,7 @@ __global__ void __launch_bounds__(SmallGeo<LOG_M, LE>::T, small_min_blocks(Small
     constexpr int PAD = M + M / E;  // exchange slots: one of padding per E
     extern __shared__ __align__(16) unsigned char smem_raw[];
     double2* buf = reinterpret_cast<double2*>(smem_raw);          // exchange buffer
-    double2* qtw = buf + PAD;                                   // padded quarter-wave table
+    double2* qtw = buf + PAD;                                   // twiddles (small_tw_layout)
     constexpr int QL = (int)twiddle_table_len<G>();
     double* wB = reinterpret_cast<double*>(qtw + QL);
     double* iwB = wB + E;

@@ -24,10 +24,10 @@
 //
 // Twiddles are read where they are used: the passes' in pass order (TW_PASS), w_M^{n k0} as a table
 // of R0 - 1 rows over n, the radix-R0 constants as immediates. Against quarter-wave tables with a fold
-// and factored products, us a squaring: N = 3072 5.65 -> 4.27 for one test, 28.9 -> 25.7 for 1184; 5120
-// 7.2 -> 5.9, 50.3 -> 43.9; 6144 10.2 -> 7.8, 32.1 -> 28.7 (592 tests); 10240 and 12288, which had read R0
-// values from shared memory for every output of a radix-R0 step, 16.5 -> 12.3 and 17.4 -> 15.0, 33.3
-// -> 24.9 and 35.1 -> 30.6 (296 tests). Fewer FP64 instructions and no integer fold; barriers and the
+// and factored products, us a squaring: N = 3072 5.65 -> 4.2 for one test, 28.9 -> 26.3 for 1184; 5120
+// 7.2 -> 6.0, 50.3 -> 43.9; 6144 10.2 -> 7.7, 32.1 -> 29.2 (592 tests); 10240 and 12288, which had read R0
+// values from shared memory for every output of a radix-R0 step, 16.5 -> 12.5 and 17.4 -> 15.3, 33.3
+// -> 25.3 and 35.1 -> 31.1 (296 tests). Fewer FP64 instructions and no integer fold; barriers and the
 // latency of the shared-memory exchanges bound it now.
 
 #include <cuda_runtime.h>
@@ -381,6 +381,7 @@ bool mixed_length_supported(uint32_t n, int* r0, int* log_l) {
 // values), 5120 5.94 (6.20 for two, 8.5), 6144 7.79 (9.8, 9.8); more tests than SMs: N = 3072 13.1 (8
 // values, four blocks; 592 tests; 17.5 with 16), 5120 22.1 (two blocks; 25.1), 6144 28.7 (16 values, two
 // blocks; 32.5 with 8). One block fits an SM at 10240 and 12288: 16 values, 12.3 and 15.0 (8: 13.1, 17.2).
+// (All with the round-off maximum in 20 bits; in full, 1 to 2% more with several tests an SM.)
 int small_fp64_mixed_log_e(uint32_t n, int njobs) {
     int r0 = 0, l = 0;
     if (!mixed_length_supported(n, &r0, &l)) return 0;

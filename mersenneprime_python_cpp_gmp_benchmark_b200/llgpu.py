@@ -134,7 +134,8 @@ def h2d_bytes():
 
 
 def release_cached():
-    """Frees the two-pass test llg_run keeps for a repeated call on the same exponent."""
+    """Frees the two-pass test llg_run keeps for a repeated call on the same exponent, and gives back
+    the streams and device memory that calls keep for the next one."""
     lib().llg_release_cached()
 
 
